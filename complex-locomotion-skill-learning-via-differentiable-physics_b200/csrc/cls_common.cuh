@@ -104,6 +104,13 @@ template <typename R> __device__ __forceinline__ R sqrt_s(R x);
 template <> __device__ __forceinline__ float sqrt_s<float>(float x) { return x * rsqrtf(x); }
 template <> __device__ __forceinline__ double sqrt_s<double>(double x) { return sqrt(x); }
 
+// a product that is rounded by itself: where a sum of two products would let the
+// compiler choose which of them to fuse, and kernels that must agree bit for
+// bit (or on a branch) could be given different choices
+template <typename R> __device__ __forceinline__ R mul_rn(R x, R y);
+template <> __device__ __forceinline__ float mul_rn<float>(float x, float y) { return __fmul_rn(x, y); }
+template <> __device__ __forceinline__ double mul_rn<double>(double x, double y) { return __dmul_rn(x, y); }
+
 template <typename R> __device__ __forceinline__ R dsin(R x);
 template <> __device__ __forceinline__ float dsin<float>(float x) { return sinf(x); }
 template <> __device__ __forceinline__ double dsin<double>(double x) { return sin(x); }

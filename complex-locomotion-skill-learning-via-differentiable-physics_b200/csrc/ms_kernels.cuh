@@ -368,22 +368,23 @@ __host__ __device__ inline size_t rev_smem_bytes(int nmax, int amax, int omax, i
 
 // Hooke + dashpot impulse of one spring seen from one of its endpoints
 // (solver_mass_spring.py:89-103).  xa/xb/va/vb are the spring's a/b endpoints.
+// Every kernel rounds it alike (mul_rn in its sums of products).
 template <typename R>
 __device__ __forceinline__ void spring_impulse(const V4<R>& xa, const V4<R>& xb, const V4<R>& va,
                                                const V4<R>& vb, R l0, R k, R coef, R act, R dt,
                                                R dashpot, R imp[3]) {
   R d0 = xa.x - xb.x, d1 = xa.y - xb.y, d2 = xa.z - xb.z;
-  R n2 = d0 * d0 + d1 * d1 + d2 * d2;
+  R n2 = d0 * d0 + mul_rn<R>(d1, d1) + d2 * d2;
   R length = sqrt_s<R>(n2 + R(1e-8)) + R(1e-4);        // norm(1e-8) + 1e-4
   R target = l0 * (R(1) + coef * act);
   R sc = dt * (length - target) * k * rcp_s<R>(length);
   R invlen = rsqrt_s<R>(n2);                           // normalized(): 1 / norm()
   R n0 = d0 * invlen, n1 = d1 * invlen, nz = d2 * invlen;
-  R vrel = (va.x - vb.x) * n0 + (va.y - vb.y) * n1 + (va.z - vb.z) * nz;
+  R vrel = (va.x - vb.x) * n0 + mul_rn<R>(va.y - vb.y, n1) + (va.z - vb.z) * nz;
   R c = dashpot * vrel;
-  imp[0] = sc * d0 + c * n0;
-  imp[1] = sc * d1 + c * n1;
-  imp[2] = sc * d2 + c * nz;
+  imp[0] = sc * d0 + mul_rn<R>(c, n0);
+  imp[1] = sc * d1 + mul_rn<R>(c, n1);
+  imp[2] = sc * d2 + mul_rn<R>(c, nz);
 }
 
 // One spring incidence: the other endpoint, which side this vertex is on, the
@@ -424,19 +425,28 @@ __device__ __forceinline__ Inc<double> load_inc<double>(const MsArgs<double>& a,
 }
 
 template <typename R>
+__device__ __forceinline__ V4<R> pick(bool first, const V4<R>& p, const V4<R>& q) {
+  V4<R> r;
+  r.x = first ? p.x : q.x; r.y = first ? p.y : q.y; r.z = first ? p.z : q.z; r.w = 0;
+  return r;
+}
+
+template <typename R>
 __device__ __forceinline__ void accumulate_incidence(const MsArgs<R>& a, const Inc<R>& in, const V4<R>& xi,
                                                      const V4<R>& vi, const V4<R>* xs, const V4<R>* vs,
                                                      const R* out, R& s0, R& s1, R& s2) {
-  const int o = in.other;
+  // the spring's endpoints by selection, not by branches: the two sides of a
+  // warp's springs share one evaluation
+  const bool at_a = in.side == 0;
+  const V4<R> xo = xs[in.other], vo = vs[in.other];
   const R act = in.out >= 0 ? out[in.out] : R(0);
   R imp[3];
-  if (in.side == 0) {  // this vertex is endpoint a: -impulse
-    spring_impulse<R>(xi, xs[o], vi, vs[o], in.l0, in.k, in.coef, act, a.dt, a.dashpot, imp);
-    s0 -= imp[0]; s1 -= imp[1]; s2 -= imp[2];
-  } else {             // endpoint b: +impulse
-    spring_impulse<R>(xs[o], xi, vs[o], vi, in.l0, in.k, in.coef, act, a.dt, a.dashpot, imp);
-    s0 += imp[0]; s1 += imp[1]; s2 += imp[2];
-  }
+  spring_impulse<R>(pick(at_a, xi, xo), pick(at_a, xo, xi), pick(at_a, vi, vo), pick(at_a, vo, vi), in.l0, in.k,
+                    in.coef, act, a.dt, a.dashpot, imp);
+  // endpoint a: -impulse, endpoint b: +impulse
+  s0 += at_a ? -imp[0] : imp[0];
+  s1 += at_a ? -imp[1] : imp[1];
+  s2 += at_a ? -imp[2] : imp[2];
 }
 
 // v_inc of all vertices, half-warp per vertex: the 16 lanes of a half-warp
@@ -606,7 +616,7 @@ __device__ __forceinline__ void gather_vinc_table(const MsArgs<R>& a, const Robo
 template <typename R>
 __device__ __forceinline__ void advance_vertex(const MsArgs<R>& a, V4<R>& x, V4<R>& v, const V4<R>& vi) {
   R ov0 = a.drag_s * v.x + vi.x;
-  R ov1 = a.drag_s * v.y + a.dt * a.gravity + vi.y;
+  R ov1 = a.drag_s * v.y + mul_rn<R>(a.dt, a.gravity) + vi.y;
   R ov2 = a.drag_s * v.z + vi.z;
   R nv0 = ov0, nv1 = ov1, nv2 = ov2, toi = 0;
   R nx1 = x.y + a.dt * ov1;
