@@ -14,6 +14,7 @@
 
 #include "../../include/cls_b200.h"
 #include "cls_profile.cuh"
+#include "ms_cluster_host.h"
 #include "ms_dense_host.h"
 #include "ms_env_host.h"
 #include "ms_sched.h"
@@ -450,6 +451,9 @@ class SimImpl final : public SimBase {
     };
     std::stable_sort(order_host_.begin(), order_host_.end(),
                      [&](int a, int b) { return cost(a) > cost(b); });
+    cost_.resize(E);
+    for (int ie = 0; ie < E; ++ie) cost_[ie] = (std::is_same<R, double>::value ? 4 : 1) * cost(ie);
+    inc_ptr_h_ = inc_ptr;
     // launch shape
     smem_p0max_ = p0max;
     smem_dmax_ = dmax;
@@ -673,10 +677,110 @@ class SimImpl final : public SimBase {
       rev_smem_ = rev0 + (on ? ctrl : 0);
       resident_ = on ? r_on : r_off;
       wsh_on_ = on;
+      plan_clusters(optin);
     } catch (...) {
       threads_ = keep;
       throw;
     }
+  }
+
+  // Shared-memory plans of the cluster-per-env kernels for clusters of 2, 4 and
+  // 8 CTAs of the current block size (invalid where a robot's share does not
+  // fit), and how many clusters can be resident.
+  struct ClusterPlan {
+    int size = 0, resident = 0;
+    ClusterCaps cap{};
+    size_t fwd_smem = 0, rev_smem = 0;
+  };
+  void plan_clusters(int optin) {
+    plans_.clear();
+    batch_plan_ = -1;
+    if (threads_ > ClusterLaunch<R>::max_threads()) return;
+    size_t fwd_max = 0, rev_max = 0;
+    CLS_CUDA(ClusterLaunch<R>::setup(optin, &fwd_max, &rev_max));
+    for (int C : {2, 4, 8}) {
+      ClusterPlan p;
+      p.size = C;
+      ClusterCaps& c = p.cap;
+      while ((1 << c.log2c) < C) ++c.log2c;
+      c.n = nmax_;
+      c.p0 = smem_p0max_;
+      c.o = smem_omax_;
+      c.oslice = round4((smem_omax_ + C - 1) / C + 1);
+      c.h = 4;
+      for (const HostRobot& h : hr_)
+        for (int l = 1; l < h.n_layers; ++l) c.h = std::max(c.h, round4(h.width[l]));
+      for (const RobotDesc& d : rd_host_)
+        for (int r = 0; r < C; ++r) {
+          const int v0 = cluster_cut(d.n_v, kVertexUnit, r, c.log2c);
+          const int v1 = cluster_cut(d.n_v, kVertexUnit, r + 1, c.log2c);
+          c.own = std::max(c.own, v1 - v0);
+          c.inc = std::max(c.inc, inc_ptr_h_[d.ptr_off + v1] - inc_ptr_h_[d.ptr_off + v0]);
+        }
+      auto sizes = [&] {
+        p.fwd_smem = ClusterLaunch<R>::fwd_bytes(c);
+        p.rev_smem = ClusterLaunch<R>::rev_bytes(c, C, threads_);
+        return p.fwd_smem <= fwd_max && p.rev_smem <= rev_max;
+      };
+      if (!sizes()) {
+        c.inc = 0;  // incidence records from global memory
+        if (!sizes()) continue;
+      }
+      CLS_CUDA(ClusterLaunch<R>::resident(C, threads_, p.fwd_smem, p.rev_smem, &p.resident));
+      if (p.resident > 0) plans_.push_back(p);
+    }
+    const ClusterPlan* all = cluster_plan(order_host_.data(), E_);
+    batch_plan_ = all ? (int)(all - plans_.data()) : -1;
+  }
+
+  // Cluster size for a launch over envs `ies` (heaviest first): the one with
+  // the shortest makespan when the envs are taken in order by the resident
+  // clusters (or single CTAs) and an env's substep costs kFixed plus its cost
+  // over the cluster's size.  Fitted to forward + reverse times per substep of
+  // 1-200 envs (quadruped, spider and random lattices, B200; one unit of cost
+  // is 0.105 ns, four in FP64): one CTA 20 / 44 / 88 / 195 us for robots of cost 47 k / 334 k
+  // / 601 k / 1.7 M, clusters of 8 17 / 25 / 34 / 51 us.  A cluster's share of
+  // an env costs 1.35 times its part: exchanges, and phases that every CTA
+  // repeats.  nullptr: one CTA per env.
+  const ClusterPlan* cluster_plan(const int* ies, int n) const {
+#ifdef CLS_CLUSTER_SIZE
+    for (const ClusterPlan& p : plans_)
+      if (p.size == CLS_CLUSTER_SIZE) return &p;
+    return nullptr;
+#endif
+    if (plans_.empty() || n > 2 * n_sm_) return nullptr;
+    std::vector<double> busy;
+    auto makespan = [&](double fixed, double per_cost, int slots) {
+      busy.assign((size_t)std::max(1, std::min(slots, n)), 0.0);
+      for (int k = 0; k < n; ++k)
+        *std::min_element(busy.begin(), busy.end()) += fixed + per_cost * cost_[ies[k]];
+      return *std::max_element(busy.begin(), busy.end());
+    };
+    const ClusterPlan* best = nullptr;
+    double t = makespan(1.45e5, 1.0, n_sm_);
+    for (const ClusterPlan& p : plans_) {
+      const double tp = makespan(1.64e5, 1.35 / p.size, p.resident);
+      if (tp < t) {
+        t = tp;
+        best = &p;
+      }
+    }
+    return best;
+  }
+
+  // forward / reverse launches of the fused path over a.n_items envs: one
+  // cluster each with a plan, else one CTA each from the work queue
+  void launch_fwd(const MsArgs<R>& a, const ClusterPlan* p, int grid, int t0, int t1, int mode, int src) {
+    if (p) CLS_CUDA(ClusterLaunch<R>::forward(a, p->cap, p->size, threads_, p->fwd_smem, stream, t0, t1, mode, src));
+    else fwd_fn()<<<grid, threads_, fwd_smem_, stream>>>(a, t0, t1, mode, src);
+  }
+  void launch_rev(const MsArgs<R>& a, const ClusterPlan* p, int grid, int t0, int t1, int last) {
+    if (p) CLS_CUDA(ClusterLaunch<R>::reverse(a, p->cap, p->size, threads_, p->rev_smem, stream, t0, t1, last));
+    else rev_fn()<<<grid, threads_, rev_smem_, stream>>>(a, t0, t1, last);
+  }
+  // of the whole batch (per-env launches keep the single-CTA kernels)
+  const ClusterPlan* batch_plan(bool per_env) const {
+    return per_env || batch_plan_ < 0 ? nullptr : &plans_[batch_plan_];
   }
 
   // Per-spring tables in shared memory (forward impulses, reverse adjoint
@@ -1029,8 +1133,9 @@ class SimImpl final : public SimBase {
     if (dense_ && !per_env) {
       dense_pass(a, 0, t_end, mode, 0, true, PK_FWD);
     } else {
+      const ClusterPlan* plan = batch_plan(per_env);
       each_launch(per_env, a, qslot_, [&](const MsArgs<R>& b, int grid) {
-        timed(PK_FWD, [&] { fwd_fn()<<<grid, threads_, fwd_smem_, stream>>>(b, 0, t_end, mode, 0); });
+        timed(PK_FWD, [&] { launch_fwd(b, plan, grid, 0, t_end, mode, 0); });
       });
     }
     CLS_CUDA(cudaGetLastError());
@@ -1312,16 +1417,13 @@ class SimImpl final : public SimBase {
         // the first pass recorded every substep's controller in this layout:
         // replay its outputs
         const int rmode = FWD_RECORD | (tail && episode ? FWD_REPLAY : 0);
+        const ClusterPlan* plan = batch_plan(per_env);
         if (recompute)
           each_launch(per_env, a, qslot, [&](const MsArgs<R>& b, int grid) {
-            timed(PK_RECOMP, [&] {
-              fwd_fn()<<<grid, threads_, fwd_smem_, stream>>>(b, t0, t1, rmode, s);
-            });
+            timed(PK_RECOMP, [&] { launch_fwd(b, plan, grid, t0, t1, rmode, s); });
           });
         each_launch(per_env, a, qslot, [&](const MsArgs<R>& b, int grid) {
-          timed(PK_REV, [&] {
-            rev_fn()<<<grid, threads_, rev_smem_, stream>>>(b, t0, t1, s == n_seg - 1 ? 1 : 0);
-          });
+          timed(PK_REV, [&] { launch_rev(b, plan, grid, t0, t1, s == n_seg - 1 ? 1 : 0); });
         });
       }
       if (episode) continue;
@@ -1864,9 +1966,8 @@ class SimImpl final : public SimBase {
     CLS_CUDA(cudaMemsetAsync(d_squeue_.p, 0, sizeof(int) * 2, stream));
     MsArgs<R> a = serve_args(n);
     a.queue = d_squeue_.p;
-    timed(PK_FWD, [&] {
-      fwd_fn()<<<grid_for(n), threads_, fwd_smem_, stream>>>(a, 0, 0, FWD_CKPT | FWD_OBS | FWD_CKEND, 0);
-    });
+    const ClusterPlan* plan = cluster_plan(serve_order_h_.data(), n);
+    timed(PK_FWD, [&] { launch_fwd(a, plan, grid_for(n), 0, 0, FWD_CKPT | FWD_OBS | FWD_CKEND, 0); });
     CLS_CUDA(cudaGetLastError());
   }
 
@@ -1894,9 +1995,10 @@ class SimImpl final : public SimBase {
     CLS_CUDA(cudaMemsetAsync(d_squeue_.p, 0, sizeof(int) * 2, stream));
     MsArgs<R> a = serve_args(n);
     a.queue = d_squeue_.p;
-    timed(PK_RECOMP, [&] { fwd_fn()<<<grid_for(n), threads_, fwd_smem_, stream>>>(a, 0, 0, FWD_RECORD, 0); });
+    const ClusterPlan* plan = cluster_plan(serve_order_h_.data(), n);
+    timed(PK_RECOMP, [&] { launch_fwd(a, plan, grid_for(n), 0, 0, FWD_RECORD, 0); });
     a.queue = d_squeue_.p + 1;
-    timed(PK_REV, [&] { rev_fn()<<<grid_for(n), threads_, rev_smem_, stream>>>(a, 0, 0, 0); });
+    timed(PK_REV, [&] { launch_rev(a, plan, grid_for(n), 0, 0, 0); });
     if (!tiles.empty()) {
       unsigned char *h, *d;
       int slot;
@@ -2092,6 +2194,10 @@ class SimImpl final : public SimBase {
   bool wsh_on_ = false;
   size_t fwd_base_ = 0;
   size_t fwd_smem_ = 0, rev_smem_ = 0, n_queue_ = 0;
+  std::vector<double> cost_;       // per env: cost of a substep (processing order, cluster sizes)
+  std::vector<int> inc_ptr_h_;     // incidence row starts of the robot types
+  std::vector<ClusterPlan> plans_;
+  int batch_plan_ = -1;            // plans_ index for launches over the whole batch
   std::vector<int> perm_, user_voff_, env_robot_, order_host_;
   bool identity_perm_ = true;
   std::vector<EnvDesc> ed_host_;

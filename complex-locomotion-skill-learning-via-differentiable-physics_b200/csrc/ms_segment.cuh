@@ -513,8 +513,48 @@ __device__ __forceinline__ void apply_center_velocity(const CenterVelocitySeed<R
   }
 }
 
-// d loss / d x[t, i] and d loss / d center[t] from the rotation loss
-// (taichi_env.py:235-252) and pose loss (:224-233).  Adds to gxi and gc.
+// The rotation loss's term (taichi_env.py:235-252) of the pair (t - run_period,
+// t), at its later end: d loss / d x1 with x0 at the earlier end, and at its
+// earlier end: d loss / d x0.  c1, c0: the centres; ca, sn: the goal's rotation;
+// k: the term's scale.  Both add to gxi and to the centre's adjoint gc.
+template <typename R>
+__device__ __forceinline__ void rotation_seed_late(const V4<R>& x1, const V4<R>& c1, const V4<R>& x0, const V4<R>& c0,
+                                                   R ca, R sn, R k, R gxi[3], R gc[3]) {
+  const R t0x = x1.x - c1.x, t0y = x1.y - c1.y, t0z = x1.z - c1.z;
+  const R t1x = x0.x - c0.x, t1y = x0.y - c0.y, t1z = x0.z - c0.z;
+  const R gx = (t0x - (ca * t1x - sn * t1z)) * k;
+  const R gy = (t0y - t1y) * k;
+  const R gz = (t0z - (sn * t1x + ca * t1z)) * k;
+  gxi[0] += gx; gxi[1] += gy; gxi[2] += gz;
+  gc[0] -= gx; gc[1] -= gy; gc[2] -= gz;
+}
+template <typename R>
+__device__ __forceinline__ void rotation_seed_early(const V4<R>& x1, const V4<R>& c1, const V4<R>& x0, const V4<R>& c0,
+                                                    R ca, R sn, R k, R gxi[3], R gc[3]) {
+  const R t0x = x1.x - c1.x, t0y = x1.y - c1.y, t0z = x1.z - c1.z;
+  const R t1x = x0.x - c0.x, t1y = x0.y - c0.y, t1z = x0.z - c0.z;
+  const R g2x = -(t0x - (ca * t1x - sn * t1z)) * k;
+  const R g2y = -(t0y - t1y) * k;
+  const R g2z = -(t0z - (sn * t1x + ca * t1z)) * k;
+  const R g1x = ca * g2x + sn * g2z, g1y = g2y, g1z = -sn * g2x + ca * g2z;
+  gxi[0] += g1x; gxi[1] += g1y; gxi[2] += g1z;
+  gc[0] -= g1x; gc[1] -= g1y; gc[2] -= g1z;
+}
+// pose loss (taichi_env.py:224-233)
+template <typename R>
+__device__ __forceinline__ void pose_seed(const MsArgs<R>& a, const EnvDesc& ed, int t, int e, int i, const V4<R>& xi,
+                                          R Br, R gxi[3]) {
+  if (!(a.loss_mask & LOSS_POSE)) return;
+  const int jp = a.jump_period, st = steps_of(a, e);
+  if (t >= 1 && t % jp == 0 && t <= st && t < a.T) {
+    const V4<R> p = a.init_obj[ed.v_off + i];
+    const R k = R(2) / R(st / jp) / Br;
+    gxi[0] += (xi.x - p.x) * k; gxi[1] += (xi.y - p.y) * k; gxi[2] += (xi.z - p.z) * k;
+  }
+}
+
+// d loss / d x[t, i] and d loss / d center[t] from the rotation and pose losses.
+// Adds to gxi and gc.
 template <typename R>
 __device__ __forceinline__ void seed_x_rotation_pose(const MsArgs<R>& a, const RobotDesc& rb,
                                                      const EnvDesc& ed, int t, int e, int i,
@@ -523,42 +563,18 @@ __device__ __forceinline__ void seed_x_rotation_pose(const MsArgs<R>& a, const R
   if (a.loss_mask & LOSS_ROTATION) {
     const R k = R(2) / R(40) / R(st);
     if (t >= 1 && t % tp > rp && t <= st && t < a.T) {
-      const V4<R> c1 = obs_c(a, t, e), c0 = obs_c(a, t - rp, e);
-      const V4<R> x0 = a.x_full[(size_t)(t - rp) * a.v_total + ed.v_off + i];
       const R ang = a.th[(size_t)(t - rp) * a.n_envs + e] * R(72.) / R(180.) * R(3.1415926535);
-      const R ca = dcos<R>(ang), sn = dsin<R>(ang);
-      const R t0x = xi.x - c1.x, t0y = xi.y - c1.y, t0z = xi.z - c1.z;
-      const R t1x = x0.x - c0.x, t1y = x0.y - c0.y, t1z = x0.z - c0.z;
-      const R gx = (t0x - (ca * t1x - sn * t1z)) * k;
-      const R gy = (t0y - t1y) * k;
-      const R gz = (t0z - (sn * t1x + ca * t1z)) * k;
-      gxi[0] += gx; gxi[1] += gy; gxi[2] += gz;
-      gc[0] -= gx; gc[1] -= gy; gc[2] -= gz;
+      rotation_seed_late<R>(xi, obs_c(a, t, e), a.x_full[(size_t)(t - rp) * a.v_total + ed.v_off + i],
+                            obs_c(a, t - rp, e), dcos<R>(ang), dsin<R>(ang), k, gxi, gc);
     }
     const int u = t + rp;
     if (u <= st && u < a.T && u % tp > rp) {
-      const V4<R> c1 = obs_c(a, u, e), c0 = obs_c(a, t, e);
-      const V4<R> x1 = a.x_full[(size_t)u * a.v_total + ed.v_off + i];
       const R ang = a.th[(size_t)t * a.n_envs + e] * R(72.) / R(180.) * R(3.1415926535);
-      const R ca = dcos<R>(ang), sn = dsin<R>(ang);
-      const R t0x = x1.x - c1.x, t0y = x1.y - c1.y, t0z = x1.z - c1.z;
-      const R t1x = xi.x - c0.x, t1y = xi.y - c0.y, t1z = xi.z - c0.z;
-      const R g2x = -(t0x - (ca * t1x - sn * t1z)) * k;
-      const R g2y = -(t0y - t1y) * k;
-      const R g2z = -(t0z - (sn * t1x + ca * t1z)) * k;
-      const R g1x = ca * g2x + sn * g2z, g1y = g2y, g1z = -sn * g2x + ca * g2z;
-      gxi[0] += g1x; gxi[1] += g1y; gxi[2] += g1z;
-      gc[0] -= g1x; gc[1] -= g1y; gc[2] -= g1z;
+      rotation_seed_early<R>(a.x_full[(size_t)u * a.v_total + ed.v_off + i], obs_c(a, u, e), xi, obs_c(a, t, e),
+                             dcos<R>(ang), dsin<R>(ang), k, gxi, gc);
     }
   }
-  if (a.loss_mask & LOSS_POSE) {
-    const int jp = a.jump_period;
-    if (t >= 1 && t % jp == 0 && t <= st && t < a.T) {
-      const V4<R> p = a.init_obj[ed.v_off + i];
-      const R k = R(2) / R(st / jp) / Br;
-      gxi[0] += (xi.x - p.x) * k; gxi[1] += (xi.y - p.y) * k; gxi[2] += (xi.z - p.z) * k;
-    }
-  }
+  pose_seed<R>(a, ed, t, e, i, xi, Br, gxi);
 }
 
 template <typename R>
@@ -802,6 +818,48 @@ __device__ __forceinline__ void spring_adjoint_gather(const MsArgs<R>& a, const 
 // The two halves of the adjoint of substep t around the controller, shared
 // by the fused segment kernel and the batched-controller step kernels.
 
+// Adjoint of advance_toi for one vertex: x, v, v_inc of t and the adjoint (gx1,
+// gv1) of the state it produced give the adjoint of x and v (gx0, gv0) and of
+// v_inc (gvi).
+template <typename R>
+__device__ __forceinline__ void advance_adjoint(const MsArgs<R>& a, const V4<R>& x, const V4<R>& v, const V4<R>& vi,
+                                                const V4<R>& gx1, const V4<R>& gv1, V4<R>& gx0, V4<R>& gv0,
+                                                V4<R>& gvi) {
+  R ov0 = a.drag_s * v.x + vi.x;
+  R ov1 = a.drag_s * v.y + mul_rn<R>(a.dt, a.gravity) + vi.y;
+  R ov2 = a.drag_s * v.z + vi.z;
+  R nv0 = ov0, nv1 = ov1, nv2 = ov2, toi = 0, f = 0;
+  const R nx1 = x.y + a.dt * ov1;
+  const bool hit = (nx1 < a.ground && ov1 < R(-1e-4));
+  if (hit) {
+    toi = -(x.y - a.ground) / ov1;
+    f = a.friction * (-ov1);
+    nv1 = 0;
+    nv0 = (ov0 < 0) ? fmin(R(0), ov0 + f) : fmax(R(0), ov0 - f);
+    nv2 = (ov2 < 0) ? fmin(R(0), ov2 + f) : fmax(R(0), ov2 - f);
+  }
+  R gox0 = gx1.x, gox1 = gx1.y, gox2 = gx1.z;
+  R gov0 = toi * gx1.x, gov1 = toi * gx1.y, gov2 = toi * gx1.z;
+  const R dtt = a.dt - toi;
+  const R gnv0 = dtt * gx1.x + gv1.x, gnv1 = dtt * gx1.y + gv1.y, gnv2 = dtt * gx1.z + gv1.z;
+  const R gtoi = gx1.x * ov0 - gx1.x * nv0 + gx1.y * ov1 - gx1.y * nv1 + gx1.z * ov2 - gx1.z * nv2;
+  if (hit) {
+    R gf = 0;
+    if (ov0 < 0) { if (!(R(0) < ov0 + f)) { gov0 += gnv0; gf += gnv0; } }
+    else { if (!(ov0 - f < R(0))) { gov0 += gnv0; gf -= gnv0; } }
+    if (ov2 < 0) { if (!(R(0) < ov2 + f)) { gov2 += gnv2; gf += gnv2; } }
+    else { if (!(ov2 - f < R(0))) { gov2 += gnv2; gf -= gnv2; } }
+    gov1 += -a.friction * gf;
+    gox1 += -gtoi / ov1;
+    gov1 += gtoi * (x.y - a.ground) / (ov1 * ov1);
+  } else {
+    gov0 += gnv0; gov1 += gnv1; gov2 += gnv2;
+  }
+  gx0.x = gox0; gx0.y = gox1; gx0.z = gox2; gx0.w = 0;
+  gv0.x = a.drag_s * gov0; gv0.y = a.drag_s * gov1; gv0.z = a.drag_s * gov2; gv0.w = 0;
+  gvi.x = gov0; gvi.y = gov1; gvi.z = gov2; gvi.w = 0;
+}
+
 // Adjoint of substep t up to the controller outputs: x(t), v(t) from the
 // records (slot kslot), advance_toi adjoint, spring-force adjoint, then
 // dz of the output layer (recorded, and left in s.dz).
@@ -828,43 +886,10 @@ __device__ __forceinline__ void rev_pre(const MsArgs<R>& a, const RobotDesc& rb,
   __syncthreads();
   // adjoint of advance_toi(t + 1)
   for (int i = tid; i < N; i += nt) {
-    V4<R> x, v, gx1, gv1;
+    V4<R> x, v, gx1, gv1, gx0, gv0, gvi;
     s.xv.get(i, x, v);
     s.g.get(i, gx1, gv1);
-    const V4<R> vi = s.gvinc[i];
-    R ov0 = a.drag_s * v.x + vi.x;
-    R ov1 = a.drag_s * v.y + a.dt * a.gravity + vi.y;
-    R ov2 = a.drag_s * v.z + vi.z;
-    R nv0 = ov0, nv1 = ov1, nv2 = ov2, toi = 0, f = 0;
-    const R nx1 = x.y + a.dt * ov1;
-    const bool hit = (nx1 < a.ground && ov1 < R(-1e-4));
-    if (hit) {
-      toi = -(x.y - a.ground) / ov1;
-      f = a.friction * (-ov1);
-      nv1 = 0;
-      nv0 = (ov0 < 0) ? fmin(R(0), ov0 + f) : fmax(R(0), ov0 - f);
-      nv2 = (ov2 < 0) ? fmin(R(0), ov2 + f) : fmax(R(0), ov2 - f);
-    }
-    R gox0 = gx1.x, gox1 = gx1.y, gox2 = gx1.z;
-    R gov0 = toi * gx1.x, gov1 = toi * gx1.y, gov2 = toi * gx1.z;
-    const R dtt = a.dt - toi;
-    const R gnv0 = dtt * gx1.x + gv1.x, gnv1 = dtt * gx1.y + gv1.y, gnv2 = dtt * gx1.z + gv1.z;
-    const R gtoi = gx1.x * ov0 - gx1.x * nv0 + gx1.y * ov1 - gx1.y * nv1 + gx1.z * ov2 - gx1.z * nv2;
-    if (hit) {
-      R gf = 0;
-      if (ov0 < 0) { if (!(R(0) < ov0 + f)) { gov0 += gnv0; gf += gnv0; } }
-      else { if (!(ov0 - f < R(0))) { gov0 += gnv0; gf -= gnv0; } }
-      if (ov2 < 0) { if (!(R(0) < ov2 + f)) { gov2 += gnv2; gf += gnv2; } }
-      else { if (!(ov2 - f < R(0))) { gov2 += gnv2; gf -= gnv2; } }
-      gov1 += -a.friction * gf;
-      gox1 += -gtoi / ov1;
-      gov1 += gtoi * (x.y - a.ground) / (ov1 * ov1);
-    } else {
-      gov0 += gnv0; gov1 += gnv1; gov2 += gnv2;
-    }
-    V4<R> gx0; gx0.x = gox0; gx0.y = gox1; gx0.z = gox2; gx0.w = 0;
-    V4<R> gv0; gv0.x = a.drag_s * gov0; gv0.y = a.drag_s * gov1; gv0.z = a.drag_s * gov2; gv0.w = 0;
-    V4<R> gvi; gvi.x = gov0; gvi.y = gov1; gvi.z = gov2; gvi.w = 0;
+    advance_adjoint<R>(a, x, v, s.gvinc[i], gx1, gv1, gx0, gv0, gvi);
     s.g.set(i, gx0, gv0);
     s.gvinc[i] = gvi;
   }
