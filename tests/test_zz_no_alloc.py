@@ -107,3 +107,74 @@ def test_noalloc_rejects_sizes_beyond_its_scratch():
                        1e-3, -9.8, 0.0, 0.0, 0.1, 0.4, ctypes.cast(msg, ctypes.c_char_p), 256)
     assert fn(ctypes.byref(a), None) == -1
     assert b"exceeds the fixed scratch" in msg.value
+
+
+def _advance64(x, v, springs, act, n, dt, gravity, ground, drag_s, dashpot, friction):
+    """FP64 restatement of one env's substeps (solver_mass_spring.py:86-148)."""
+    a, b = springs[:, 0].astype(int), springs[:, 1].astype(int)
+    ok = (a >= 0) & (a < len(x)) & (b >= 0) & (b < len(x))
+    a, b, l0, k, coef, act = a[ok], b[ok], springs[ok, 2], springs[ok, 3], springs[ok, 4], act[ok]
+    for _ in range(n):
+        d, dv = x[a] - x[b], v[a] - v[b]
+        n2 = (d * d).sum(1)
+        length = np.sqrt(n2 + 1e-8) + 1e-4
+        nrm = d / np.sqrt(n2)[:, None]
+        imp = (dt * (length - l0 * (1 + coef * act)) * k / length)[:, None] * d
+        imp += (dashpot * (dv * nrm).sum(1))[:, None] * nrm
+        vinc = np.zeros_like(v)
+        np.add.at(vinc, a, -imp)
+        np.add.at(vinc, b, imp)
+        ov = drag_s * v + vinc
+        ov[:, 1] += dt * gravity
+        hit = (x[:, 1] + dt * ov[:, 1] < ground) & (ov[:, 1] < -1e-4)
+        toi = np.where(hit, -(x[:, 1] - ground) / np.where(hit, ov[:, 1], -1.0), 0.0)
+        f = np.where(hit, -friction * ov[:, 1], 0.0)
+        nv = ov.copy()
+        nv[hit, 1] = 0.0
+        for c in (0, 2):
+            nv[:, c] = np.where(ov[:, c] < 0, np.minimum(0.0, ov[:, c] + f), np.maximum(0.0, ov[:, c] - f))
+        x = x + toi[:, None] * ov + (dt - toi)[:, None] * nv
+        v = nv
+    return x, v
+
+
+@pytest.mark.parametrize("n_v, n_s, n_sub, envs", [
+    (1, 0, 3, 2),            # no springs
+    (2, 1, 1, 1), (33, 31, 5, 3), (300, 257, 4, 2), (257, 1025, 7, 2),
+    (900, 4600, 3, 2),       # near the largest table that fits one CTA
+    (900, 6500, 3, 2),       # beyond it: a launch per phase
+    (40, 90, 0, 1),          # nothing to do
+])
+def test_noalloc_advance_sizes(n_v, n_s, n_sub, envs):
+    """One launch per call (springs in shared memory) and one per phase, against
+    the FP64 restatement; some springs name vertices that do not exist and are
+    skipped.  The file's tolerances."""
+    import torch
+    fn = _lib()
+    rng = np.random.default_rng(n_v + n_s)
+    x0 = rng.uniform(0.0, 1.0, (envs, n_v, 3))
+    v0 = rng.uniform(-0.5, 0.5, (envs, n_v, 3))
+    springs = np.zeros((n_s, 5))
+    if n_s:
+        a = rng.integers(0, n_v, n_s)
+        springs[:, 0], springs[:, 1] = a, (a + 1 + rng.integers(0, max(1, n_v - 1), n_s)) % n_v
+        springs[:, 2], springs[:, 3], springs[:, 4] = rng.uniform(0.2, 0.5, n_s), rng.uniform(1, 20, n_s), 0.2
+        springs[::7, rng.integers(0, 2)] = n_v + 3
+        springs[3::11, 0] = -1
+    act = rng.uniform(-1, 1, (envs, n_s))
+    ph = dict(dt=2e-3, gravity=-9.8, ground=0.0, drag=2.0, dashpot=0.1, friction=0.5)
+    f32 = dict(dtype=torch.float32, device="cuda:0")
+    i32 = dict(dtype=torch.int32, device="cuda:0")
+    sa, sb = (torch.tensor(springs[:, c].astype(np.int32), **i32) for c in (0, 1))
+    rest, stiff, coef = (torch.tensor(springs[:, c].copy(), **f32) for c in (2, 3, 4))
+    ta, x, v = torch.tensor(act, **f32), torch.tensor(x0, **f32), torch.tensor(v0, **f32)
+    args = NoallocAdvance(envs, n_v, n_s, n_sub, sa.data_ptr(), sb.data_ptr(), rest.data_ptr(), stiff.data_ptr(),
+                          coef.data_ptr(), ta.data_ptr(), x.data_ptr(), v.data_ptr(), ph["dt"], ph["gravity"],
+                          ph["ground"], ph["drag"], ph["dashpot"], ph["friction"], None, 0)
+    assert fn(ctypes.byref(args), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    gx, gv = x.cpu().numpy(), v.cpu().numpy()
+    for e in range(envs):
+        rx, rv = _advance64(x0[e], v0[e], springs, act[e], n_sub, ph["dt"], ph["gravity"], ph["ground"],
+                            np.exp(-ph["dt"] * ph["drag"]), ph["dashpot"], ph["friction"])
+        assert max_rel(gx[e], rx) < 1e-5
+        assert max_rel(gv[e], rv) < 1e-4
