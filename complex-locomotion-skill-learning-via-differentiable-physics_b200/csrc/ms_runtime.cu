@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -768,6 +769,28 @@ class SimImpl final : public SimBase {
     return best;
   }
 
+  // Weight-gradient tiles over kseg record slots, a cluster of CTAs per tile
+  // where the tiles alone leave SMs idle: the largest size that keeps at most
+  // four CTAs per SM and at least 64 rows (four stages) in each.
+  void launch_wgrad(const MsArgs<R>& a, const GemmTile* tiles, int n, int kseg) {
+    long long rows = LLONG_MAX;
+    for (const RobotDesc& d : rd_host_)
+      if (d.n_env > 0) rows = std::min(rows, (long long)kseg * d.n_env);
+    int C = 8;
+    while (C > 1 && ((long long)n * C > 4LL * n_sm_ || rows / C < 64)) C >>= 1;
+    cudaLaunchConfig_t c{};
+    cudaLaunchAttribute at{};
+    c.gridDim = dim3((unsigned)(n * C));
+    c.blockDim = dim3(256);
+    c.stream = stream;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)C;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    c.attrs = &at;
+    c.numAttrs = C > 1 ? 1 : 0;
+    CLS_CUDA(cudaLaunchKernelEx(&c, ms_wgrad_kernel<R>, a, tiles, kseg, d_gw_.p, d_gb_.p));
+  }
+
   // forward / reverse launches of the fused path over a.n_items envs: one
   // cluster each with a plan, else one CTA each from the work queue
   void launch_fwd(const MsArgs<R>& a, const ClusterPlan* p, int grid, int t0, int t1, int mode, int src) {
@@ -1439,15 +1462,13 @@ class SimImpl final : public SimBase {
         }
       } else if (!tiles_host_.empty()) {
         timed(PK_WGRAD, [&] {
-          ms_wgrad_kernel<R><<<(int)tiles_host_.size(), 256, 0, stream>>>(a, d_tiles_.p, t1 - t0,
-                                                                           d_gw_.p, d_gb_.p);
+          launch_wgrad(a, d_tiles_.p, (int)tiles_host_.size(), t1 - t0);
         });
       }
     }
     if (episode)
       timed(PK_WGRAD, [&] {
-        ms_wgrad_kernel<R><<<(int)tiles_ep_.size(), 256, 0, stream>>>(a0, d_tiles_ep_.p, t_last, d_gw_.p,
-                                                                        d_gb_.p);
+        launch_wgrad(a0, d_tiles_ep_.p, (int)tiles_ep_.size(), t_last);
       });
     CLS_CUDA(cudaGetLastError());
     bwd_done_ = true;
