@@ -101,7 +101,7 @@ struct FwdArgs {
   const R* act;           // [E][M] of step g
   V4<R>* acc;             // (momentum, mass) accumulator of step g
   int* bbox;              // [E][2 D] box of the base cells of step g (min, max)
-  R* csum;                // [E][D] pw-weighted position sums of the positions produced (or read)
+  double* csum;           // [E][D] pw-weighted position sums of the positions produced (or read)
 };
 
 // Reverse particle kernel: P2G^T of step f plus the loss seed of step f
@@ -119,7 +119,7 @@ struct AdjArgs {
   R* gact;                 // d actuation [E][M] of step f (accumulated)
   // loss seed of the state whose x-adjoint is completed here
   R seed_w;                // w_t (0: none)
-  const R* csum;           // [E][D] pw-weighted position sums of that step
+  const double* csum;      // [E][D] pw-weighted position sums of that step
   const R* target;         // [E][D]
   R pw_sum;
   // outputs of the last reverse step (no G2P^T follows)
@@ -545,20 +545,28 @@ __device__ __forceinline__ void tile_add(R* p, R v, bool atomic) {
   else *p += v;
 }
 
-// warp sum of D values, added to out[0..D) by lane 0
+// warp sum of D values, added to out[0..D) by lane 0 (64-bit sums: a thousand
+// warps add to one centre)
 template <typename R, int D>
-__device__ __forceinline__ void warp_sum_add(const R v[D], R* out) {
+__device__ __forceinline__ void warp_sum_add(const R v[D], double* out) {
 #pragma unroll
   for (int d = 0; d < D; ++d) {
     R s = v[d];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(out + d, s);
+    if ((threadIdx.x & 31) == 0) atomicAdd(out + d, (double)s);
   }
 }
 
 template <typename R>
 __device__ __forceinline__ R ld(const R* p) { return __ldg(p); }
+
+// distance of a centre (sum of weighted positions over the weights' sum) from
+// its target
+template <typename R>
+__device__ __forceinline__ R center_error(double csum, R pw_sum, R target) {
+  return (R)(csum / (double)pw_sum - (double)target);
+}
 
 // ------------------------------------------------------------------ forward
 // G2P of step f (solver_mpm.py:146-165) fused with P2G of step f + 1
@@ -1041,7 +1049,7 @@ __global__ void __launch_bounds__(kChunk, CLS_MPM_ADJ_MIN_BLOCKS) mpm_adj_kernel
     for (int d = 0; d < D; ++d) {
       R s = 0;
       if (a.seed_w != R(0) && valid)
-        s = R(2) * a.seed_w * (ld(a.csum + (long long)e * D + d) / a.pw_sum - ld(a.target + (long long)e * D + d)) *
+        s = R(2) * a.seed_w * center_error<R>(ld(a.csum + (long long)e * D + d), a.pw_sum, ld(a.target + (long long)e * D + d)) *
             ld(c.pw + p) / a.pw_sum;
       ax[d] = (valid ? ld(a.ax_in + d * EP + q) : R(0)) + gfx[d] * c.inv_dx + s;
     }
@@ -1078,7 +1086,7 @@ __global__ void __launch_bounds__(kChunk, CLS_MPM_ADJ_MIN_BLOCKS) mpm_adj_kernel
       ax[d] = 0;
       av[d] = 0;
       if (a.seed_w != R(0) && valid)
-        ax[d] = R(2) * a.seed_w * (ld(a.csum + (long long)e * D + d) / a.pw_sum - ld(a.target + (long long)e * D + d)) *
+        ax[d] = R(2) * a.seed_w * center_error<R>(ld(a.csum + (long long)e * D + d), a.pw_sum, ld(a.target + (long long)e * D + d)) *
                 ld(c.pw + p) / a.pw_sum;
     }
 #pragma unroll

@@ -20,6 +20,7 @@
 #include "../../include/cls_b200.h"
 #include "cls_profile.cuh"
 #include "mpm_kernels.cuh"
+#include "mpm_small_host.h"
 
 namespace cls {
 namespace mpm {
@@ -110,6 +111,20 @@ class MpmImpl final : public MpmBase {
     MPM_REQUIRE((long long)E_ * nblk_ < (1LL << 31), "grid too large");
     slots_ = std::max(K_, 2);
     n_ckpt_ = (T_ + K_ - 1) / K_ + 1;
+    // Record slots for every step of the longest rollout, written by the first
+    // pass, so that the reverse pass recomputes nothing (27 % of an 8-env
+    // legged-body iteration): when that takes no more slots than two segment
+    // records, or at most a sixteenth of the free device memory.
+    {
+      const double per_slot = sizeof(R) * ((double)E_ * P_ * 2 * (D + D * D) + 4.0 * E_ * nblk_ * Blk<D>::NODES);
+      size_t free_b = 0, total_b = 0;
+      MPM_CUDA(cudaMemGetInfo(&free_b, &total_b));
+      whole_ = T_ <= 2 * slots_ || T_ * per_slot <= free_b / 16.0;
+      if (whole_) {
+        slots_ = std::max(T_, 2);
+        n_ckpt_ = 1;
+      }
+    }
     build_order(b);
     n_chunks_ = (int)chunk_start_h_.size();
     MPM_REQUIRE((long long)E_ * n_chunks_ < (1LL << 31), "too many particle chunks");
@@ -119,9 +134,11 @@ class MpmImpl final : public MpmBase {
     ck_x_.alloc(n_ckpt_ * VX); ck_v_.alloc(n_ckpt_ * VX);
     ck_C_.alloc(n_ckpt_ * VM); ck_F_.alloc(n_ckpt_ * VM);
     for (int s = 0; s < 2; ++s) {
-      X_[s].alloc(VX); Fw_[s].alloc(VM);
-      RX_[s].alloc(K_ * VX); RV_[s].alloc(K_ * VX); RC_[s].alloc(K_ * VM); RF_[s].alloc(K_ * VM);
       AX_[s].alloc(VX); AF_[s].alloc(VM);
+      if (whole_ && s == 1) break;  // one record holds the rollout
+      const size_t rs = whole_ ? T_ : K_;
+      if (!whole_) { X_[s].alloc(VX); Fw_[s].alloc(VM); }
+      RX_[s].alloc(rs * VX); RV_[s].alloc(rs * VX); RC_[s].alloc(rs * VM); RF_[s].alloc(rs * VM);
       gv_[s].alloc(slots_ * nodes);
     }
     bboxes_.alloc((size_t)2 * slots_ * E_ * 2 * D);
@@ -140,7 +157,7 @@ class MpmImpl final : public MpmBase {
     MPM_CUDA(cudaMemset(acc_.p, 0, sizeof(V) * nodes));
     MPM_CUDA(cudaMemset(gacc_.p, 0, sizeof(V) * nodes));
     MPM_CUDA(cudaMemset(ga_.p, 0, sizeof(V) * nodes));
-    for (int s = 0; s < 2; ++s) MPM_CUDA(cudaMemset(gv_[s].p, 0, sizeof(V) * slots_ * nodes));
+    for (int s = 0; s < (whole_ ? 1 : 2); ++s) MPM_CUDA(cudaMemset(gv_[s].p, 0, sizeof(V) * slots_ * nodes));
 
     std::vector<int> mus(P_, -1);
     for (int i = 0; i < P_; ++i) {
@@ -158,12 +175,17 @@ class MpmImpl final : public MpmBase {
     pw_sum_ = P_;
     MPM_CUDA(cudaMemcpy(pw_.p, pw.data(), sizeof(R) * P_, cudaMemcpyHostToDevice));
     loss_w_.assign(T_ + 1, 0.0);
+    seed_w_.alloc(T_ + 1);
+    MPM_CUDA(cudaMemset(seed_w_.p, 0, sizeof(R) * (T_ + 1)));
     MPM_CUDA(cudaMemset(act_.p, 0, sizeof(R) * act_.n));
     MPM_CUDA(cudaMemset(target_.p, 0, sizeof(R) * target_.n));
     // shared-memory opt-in for the tile
     fwd_smem_ = tile_cap_ > 0 ? (size_t)kWarps * kFwdPlanes * tile_cap_ * sizeof(R) : 0;
     adj_smem_ = tile_cap_ > 0 ? (size_t)kWarps * kAdjPlanes * tile_cap_ * sizeof(R) : 0;
     set_smem_attrs<kStageGather | kScatterTile>();
+    // bodies whose grid fits in one CTA's shared memory (default order, no tiles):
+    // one CTA per env for the whole rollout
+    if (whole_ && runs_ && tile_cap_ == 0) MPM_CUDA((SmallLaunch<R, D>::plan(E_, P_, n_grid_, &small_, &small_cap_[0], &small_cap_[1])));
     // initial state: body positions in every env, v = C = 0, F = I
     std::vector<double> x0(EP * D), v0(EP * D, 0.0);
     for (int e = 0; e < E_; ++e)
@@ -269,14 +291,24 @@ class MpmImpl final : public MpmBase {
   R* ckF(int s) { return ck_F_.p + (size_t)s * VM(); }
   V* gv(int r, int k) { return gv_[r].p + (size_t)k * NODES(); }
   int* bbox(int r, int k) { return bboxes_.p + ((size_t)r * slots_ + k) * E_ * 2 * D; }
-  // state of step t0(s) + k of segment s (slot 0 is the checkpoint)
-  R* rx(int s, int k) { return k == 0 ? ckx(s) : RX_[s % 2].p + (size_t)k * VX(); }
-  R* rv(int s, int k) { return k == 0 ? ckv(s) : RV_[s % 2].p + (size_t)k * VX(); }
-  R* rC(int s, int k) { return k == 0 ? ckC(s) : RC_[s % 2].p + (size_t)k * VM(); }
-  R* rF(int s, int k) { return k == 0 ? ckF(s) : RF_[s % 2].p + (size_t)k * VM(); }
-  // first pass: x and F of step g (checkpoint steps live in the checkpoints)
-  R* fx(int g) { return g % K_ == 0 ? ckx(g / K_) : X_[g % 2].p; }
-  R* fF(int g) { return g % K_ == 0 ? ckF(g / K_) : Fw_[g % 2].p; }
+  // state of step t0(s) + k of segment s (slot 0 is the checkpoint); with the
+  // whole rollout recorded, of step t0(s) + k at its own slot
+  R* rec(Buf<R>* rb, R* first, int s, int k, size_t n) {
+    if (whole_) return s * K_ + k == 0 ? first : rb[0].p + (size_t)(s * K_ + k) * n;
+    return k == 0 ? first : rb[s % 2].p + (size_t)k * n;
+  }
+  R* rx(int s, int k) { return rec(RX_, whole_ ? ckx(0) : ckx(s), s, k, VX()); }
+  R* rv(int s, int k) { return rec(RV_, whole_ ? ckv(0) : ckv(s), s, k, VX()); }
+  R* rC(int s, int k) { return rec(RC_, whole_ ? ckC(0) : ckC(s), s, k, VM()); }
+  R* rF(int s, int k) { return rec(RF_, whole_ ? ckF(0) : ckF(s), s, k, VM()); }
+  // grid and boxes of step t0(s) + k in the reverse pass
+  V* rg(int s, int k) { return whole_ ? gv(0, s * K_ + k) : gv(s % 2, k); }
+  int* rbox(int s, int k) { return whole_ ? bbox(0, s * K_ + k) : bbox(s % 2, k); }
+  // first pass: x, F and the grid slot of step g (checkpoint steps live in the
+  // checkpoints)
+  R* fx(int g) { return whole_ ? rx(0, g) : (g % K_ == 0 ? ckx(g / K_) : X_[g % 2].p); }
+  R* fF(int g) { return whole_ ? rF(0, g) : (g % K_ == 0 ? ckF(g / K_) : Fw_[g % 2].p); }
+  int fg(int g) const { return whole_ ? g : g % 2; }
   const R* act(int g) const { return act_.p + (size_t)g * E_ * M_; }
 
   int particle_grid() const { return E_ * n_chunks_; }
@@ -345,7 +377,24 @@ class MpmImpl final : public MpmBase {
     MPM_REQUIRE(steps >= 1 && steps <= T_, "steps must be in [1, max_steps]");
     steps_ = steps;
     const size_t cslab = (size_t)E_ * D;
-    timed(MK_OTHER, [&] { cudaMemsetAsync(csum_.p, 0, sizeof(R) * (steps + 1) * cslab, stream); });
+    timed(MK_OTHER, [&] { cudaMemsetAsync(csum_.p, 0, sizeof(double) * (steps + 1) * cslab, stream); });
+    if (small_) {
+      SmallFwdArgs<R> a;
+      std::memset(&a, 0, sizeof(a));
+      a.c = phys();
+      a.cap = small_cap_[0];
+      a.steps = steps;
+      a.x0 = ckx(0); a.v0 = ckv(0); a.C0 = ckC(0); a.F0 = ckF(0);
+      a.rec_x = RX_[0].p; a.rec_v = RV_[0].p; a.rec_C = RC_[0].p; a.rec_F = RF_[0].p;
+      a.fin_x = fin_x_.p; a.fin_v = fin_v_.p; a.fin_C = fin_C_.p; a.fin_F = fin_F_.p;
+      a.grid = gv_[0].p;
+      a.act = act_.p;
+      a.csum = csum_.p;
+      timed(MK_PFWD, [&] { MPM_CUDA((SmallLaunch<R, D>::forward(a, stream))); });
+      fwd_done_ = true;
+      bwd_done_ = false;
+      return;
+    }
     reset_bbox(0, 0);
     {  // P2G of step 0
       FwdArgs<R> a = fwd_args();
@@ -361,21 +410,22 @@ class MpmImpl final : public MpmBase {
       const int g = f + 1;
       FwdArgs<R> a = fwd_args();
       a.x_in = fx(f);
-      a.gv = gv(0, f % 2);
+      a.gv = gv(0, fg(f));
       a.x_out = fx(g);
-      if (g % K_ == 0) { a.v_out = ckv(g / K_); a.C_out = ckC(g / K_); }
+      if (whole_) { a.v_out = rv(0, g); a.C_out = rC(0, g); }
+      else if (g % K_ == 0) { a.v_out = ckv(g / K_); a.C_out = ckC(g / K_); }
       a.F_in = fF(g);
       a.F_out = g + 1 <= steps - 1 ? fF(g + 1) : fin_F_.p;
       a.act = act(g);
-      a.bbox = bbox(0, g % 2);
+      a.bbox = bbox(0, fg(g));
       a.csum = csum_.p + (size_t)g * cslab;
       launch_fwd(3, a, MK_PFWD);
-      launch_grid(gv(0, g % 2), 0, g % 2, g + 1 <= steps - 1 ? bbox(0, f % 2) : nullptr);
+      launch_grid(gv(0, fg(g)), 0, fg(g), g + 1 <= steps - 1 ? bbox(0, fg(g + 1)) : nullptr);
     }
     {  // G2P of the last step
       FwdArgs<R> a = fwd_args();
       a.x_in = fx(steps - 1);
-      a.gv = gv(0, (steps - 1) % 2);
+      a.gv = gv(0, fg(steps - 1));
       a.x_out = fin_x_.p; a.v_out = fin_v_.p; a.C_out = fin_C_.p;
       a.csum = csum_.p + (size_t)steps * cslab;
       launch_fwd(1, a, MK_PFWD);
@@ -414,15 +464,16 @@ class MpmImpl final : public MpmBase {
 
   double loss() override {
     MPM_REQUIRE(fwd_done_, "cls_mpm_loss before a forward rollout");
-    std::vector<R> c((size_t)(steps_ + 1) * E_ * D), tg((size_t)(steps_ + 1) * E_ * D);
-    MPM_CUDA(cudaMemcpyAsync(c.data(), csum_.p, sizeof(R) * c.size(), cudaMemcpyDeviceToHost, stream));
+    std::vector<double> c((size_t)(steps_ + 1) * E_ * D);
+    std::vector<R> tg((size_t)(steps_ + 1) * E_ * D);
+    MPM_CUDA(cudaMemcpyAsync(c.data(), csum_.p, sizeof(double) * c.size(), cudaMemcpyDeviceToHost, stream));
     MPM_CUDA(cudaMemcpyAsync(tg.data(), target_.p, sizeof(R) * tg.size(), cudaMemcpyDeviceToHost, stream));
     MPM_CUDA(cudaStreamSynchronize(stream));
     double L = 0;
     for (int t = 0; t <= steps_; ++t) {
       if (loss_w_[t] == 0.0) continue;
       for (size_t q = 0; q < (size_t)E_ * D; ++q) {
-        const double e = (double)(c[(size_t)t * E_ * D + q] / (R)pw_sum_) - (double)tg[(size_t)t * E_ * D + q];
+        const double e = c[(size_t)t * E_ * D + q] / pw_sum_ - (double)tg[(size_t)t * E_ * D + q];
         L += loss_w_[t] * e * e;
       }
     }
@@ -444,11 +495,31 @@ class MpmImpl final : public MpmBase {
     auto g2pT = [&](AdjArgs<R>& a, int h) {
       const int sh = h / K_, kh = h - sh * K_;
       a.x_h = rx(sh, kh);
-      a.gv_h = gv(sh % 2, kh);
+      a.gv_h = rg(sh, kh);
       a.gacc = gacc_.p;
     };
     timed(MK_OTHER, [&] { cudaMemsetAsync(gact_.p, 0, sizeof(R) * gact_.n, stream); });
-    recompute(n_seg - 1);
+    if (small_) {
+      SmallAdjArgs<R> a;
+      std::memset(&a, 0, sizeof(a));
+      a.c = c;
+      a.cap = small_cap_[1];
+      a.steps = steps;
+      a.x0 = ckx(0); a.v0 = ckv(0); a.C0 = ckC(0); a.F0 = ckF(0);
+      a.rec_x = RX_[0].p; a.rec_v = RV_[0].p; a.rec_C = RC_[0].p; a.rec_F = RF_[0].p;
+      a.grid = gv_[0].p;
+      a.act = act_.p;
+      a.gact = gact_.p;
+      a.seed_w = seed_w_.p;
+      a.csum = csum_.p;
+      a.target = target_.p;
+      a.pw_sum = (R)pw_sum_;
+      a.out_ax = out_ax_.p; a.out_av = out_av_.p; a.out_aC = out_aC_.p; a.out_aF = out_aF_.p;
+      timed(MK_PADJ, [&] { MPM_CUDA((SmallLaunch<R, D>::reverse(a, stream))); });
+      bwd_done_ = true;
+      return;
+    }
+    if (!whole_) recompute(n_seg - 1);
     int cur = 0;
     {  // G2P^T of the last step, seeded by the loss at step `steps`
       AdjArgs<R> a;
@@ -461,10 +532,10 @@ class MpmImpl final : public MpmBase {
     }
     for (int f = steps - 1; f >= 0; --f) {
       const int s = f / K_, k = f - s * K_;
-      if (f >= 1 && k == 0) recompute(s - 1);
+      if (!whole_ && f >= 1 && k == 0) recompute(s - 1);
       timed(MK_GADJ, [&] {
-        mpm_grid_adj_kernel<R, D><<<grid_dims(), 256, 0, stream>>>(c, gacc_.p, gv(s % 2, k), ga_.p,
-                                                                   bbox(s % 2, k));
+        mpm_grid_adj_kernel<R, D><<<grid_dims(), 256, 0, stream>>>(c, gacc_.p, rg(s, k), ga_.p,
+                                                                   rbox(s, k));
       });
       AdjArgs<R> a;
       std::memset(&a, 0, sizeof(a));
@@ -567,7 +638,10 @@ class MpmImpl final : public MpmBase {
   void set_actuation(const double* act_h) override { up(act_h, act_.p, (size_t)T_ * E_ * M_); }
 
   void set_loss(const double* w, const double* target, const double* pw) override {
-    if (w) loss_w_.assign(w, w + T_ + 1);
+    if (w) {
+      loss_w_.assign(w, w + T_ + 1);
+      up(w, seed_w_.p, T_ + 1);
+    }
     if (target) up(target, target_.p, (size_t)(T_ + 1) * E_ * D);
     if (pw) {
       std::vector<double> pi(P_);
@@ -599,7 +673,8 @@ class MpmImpl final : public MpmBase {
   }
 
   void centers(double* c) override {
-    down(csum_.p, c, (size_t)(T_ + 1) * E_ * D);
+    MPM_CUDA(cudaMemcpyAsync(c, csum_.p, sizeof(double) * (T_ + 1) * E_ * D, cudaMemcpyDeviceToHost, stream));
+    MPM_CUDA(cudaStreamSynchronize(stream));
     for (size_t i = 0; i < (size_t)(T_ + 1) * E_ * D; ++i) c[i] /= pw_sum_;
   }
 
@@ -623,13 +698,17 @@ class MpmImpl final : public MpmBase {
   std::vector<int> perm_;  // internal particle -> user particle
   std::vector<int> chunk_start_h_, chunk_len_h_;
   bool runs_ = false;  // CLS_MPM_ORDER_BASE_RUNS
+  bool whole_ = false;  // every step recorded by the first pass
+  bool small_ = false;  // one CTA per env (mpm_small.cuh)
+  int small_cap_[2] = {0, 0};  // its scatter tables' sizes
   bool fwd_done_ = false, bwd_done_ = false;
   Buf<R> ck_x_, ck_v_, ck_C_, ck_F_;
   Buf<R> X_[2], Fw_[2], RX_[2], RV_[2], RC_[2], RF_[2], AX_[2], AF_[2];
   Buf<V> gv_[2], acc_, gacc_, ga_;
   Buf<int> bboxes_, muscle_, chunk_start_, chunk_len_;
   Buf<R> fin_x_, fin_v_, fin_C_, fin_F_, out_ax_, out_av_, out_aC_, out_aF_;
-  Buf<R> act_, gact_, csum_, target_, fibre_, pw_;
+  Buf<R> act_, gact_, target_, fibre_, pw_, seed_w_;
+  Buf<double> csum_;  // centre sums in 64 bits: many warps' contributions each
   EventProfile<MK_COUNT> prof_;
   cudaGraph_t graph_ = nullptr;
   cudaGraphExec_t gexec_ = nullptr;

@@ -506,8 +506,12 @@ int cls_mpm_set_loss(cls_mpm* sim, const double* w, const double* target, const 
 /* steps x advance_core (clear_grid, p2g, grid_op, g2p; solver_mpm.py:175-180). */
 int cls_mpm_forward(cls_mpm* sim, int32_t steps);
 int cls_mpm_loss(cls_mpm* sim, double* loss);
-/* Reverse pass (advance_core_grad, solver_mpm.py:182-190, over checkpointed
- * segments). */
+/* Reverse pass (advance_core_grad, solver_mpm.py:182-190): over segments
+ * recomputed from their checkpoints, or, where every step of max_steps can be
+ * recorded in no more slots than two segments take or in a sixteenth of the
+ * device memory that is free at creation, over what cls_mpm_forward recorded.
+ * Bodies whose grid and particles fit in one CTA's shared memory run whole
+ * rollouts in one launch per direction (base-cell order, no tiles). */
 int cls_mpm_backward(cls_mpm* sim);
 int cls_mpm_get_final_state(cls_mpm* sim, double* x, double* v, double* C, double* F);
 /* d loss / d actuation [T][n_envs][n_muscles] and / d initial x, v, C, F. */
