@@ -95,15 +95,19 @@ template <typename R>
 cudaError_t EnvLaunch<R>::step(const MsArgs<R>& a, size_t smem, cudaStream_t s, int t, int from_ckpt,
                                const R* outs, int out_pitch, R* obs, int obs_pitch, R* aux) {
   auto fn = ms_env_step_kernel<R>;
-  int dev = 0, optin = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  cudaFuncAttributes fa{};
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fn);
-  if (e != cudaSuccess) return e;
-  if (smem + fa.sharedSizeBytes > (size_t)optin) return cudaErrorInvalidConfiguration;
-  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
+  // above the default limit the attribute is set on every call (it is per kernel
+  // and process, and handles differ); the queries cost more than the launch
+  if (smem > 40 * 1024) {
+    int dev = 0, optin = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    cudaFuncAttributes fa{};
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fn);
+    if (e != cudaSuccess) return e;
+    if (smem + fa.sharedSizeBytes > (size_t)optin) return cudaErrorInvalidConfiguration;
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
   fn<<<a.n_envs, kEnvThreads, smem, s>>>(a, t, from_ckpt, outs, out_pitch, obs, obs_pitch, aux);
   return cudaGetLastError();
 }
