@@ -6,11 +6,6 @@
 #include "ms_dense.cuh"
 #include "ms_dense_host.h"
 
-// threads of the step kernels (one CTA per env)
-#ifndef CLS_STEP_THREADS
-#define CLS_STEP_THREADS 128
-#endif
-
 namespace cls {
 
 template <typename R>
@@ -23,19 +18,20 @@ long long DenseLaunch<R>::split_floats(int rows, int tile_rows, int k) {
 }
 
 template <typename R>
-cudaError_t DenseLaunch<R>::setup(int threads, size_t* fwd_static, size_t* rev_static, int optin) {
-  if (threads != CLS_STEP_THREADS) return cudaErrorInvalidValue;
-  auto fwd = ms_step_fwd_kernel<R, CLS_STEP_THREADS>;
-  auto rev = ms_step_rev_kernel<R, CLS_STEP_THREADS>;
-  cudaFuncAttributes fa{}, ra{};
-  cudaError_t e = cudaFuncGetAttributes(&fa, fwd);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&ra, rev);
-  if (e != cudaSuccess) return e;
-  *fwd_static = fa.sharedSizeBytes;
-  *rev_static = ra.sharedSizeBytes;
-  e = cudaFuncSetAttribute(fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((size_t)optin - fa.sharedSizeBytes));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(rev, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((size_t)optin - ra.sharedSizeBytes));
+cudaError_t DenseLaunch<R>::setup(size_t* fwd_static, size_t* rev_static, int optin) {
+  *fwd_static = *rev_static = 0;
+  cudaError_t e = cudaSuccess;
+  auto prepare = [&](auto fn, size_t* st) {
+    cudaFuncAttributes fa{};
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fn);
+    if (e != cudaSuccess) return;
+    *st = std::max(*st, fa.sharedSizeBytes);
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((size_t)optin - fa.sharedSizeBytes));
+  };
+  prepare(ms_step_fwd_kernel<R, kStepThreads, false>, fwd_static);
+  prepare(ms_step_fwd_kernel<R, kStepThreads, true>, fwd_static);
+  prepare(ms_step_rev_kernel<R, kStepThreads, false>, rev_static);
+  prepare(ms_step_rev_kernel<R, kStepThreads, true>, rev_static);
   if constexpr (std::is_same<R, float>::value) {
     const int sm = (int)umma::BulkShape<kDenseTN, kBulkStages>::kSmemBytes;
     if (e == cudaSuccess) e = cudaFuncSetAttribute(ms_ctrl_gemm_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
@@ -48,15 +44,15 @@ cudaError_t DenseLaunch<R>::setup(int threads, size_t* fwd_static, size_t* rev_s
 template <typename R>
 void DenseLaunch<R>::step_fwd(const MsArgs<R>& a, int grid, int threads, size_t smem, cudaStream_t s, int t,
                               int t_first, int t_end, int mode, int src_slot, int k_prev, int k_cur) {
-  ms_step_fwd_kernel<R, CLS_STEP_THREADS><<<grid, threads, smem, s>>>(a, t, t_first, t_end, mode, src_slot,
-                                                                       k_prev, k_cur);
+  auto fn = a.imp_cap ? ms_step_fwd_kernel<R, kStepThreads, true> : ms_step_fwd_kernel<R, kStepThreads, false>;
+  fn<<<grid, threads, smem, s>>>(a, t, t_first, t_end, mode, src_slot, k_prev, k_cur);
 }
 
 template <typename R>
 void DenseLaunch<R>::step_rev(const MsArgs<R>& a, int grid, int threads, size_t smem, cudaStream_t s, int t_post,
                               int t_pre, int t_begin, int t_end, int last_seg) {
-  ms_step_rev_kernel<R, CLS_STEP_THREADS><<<grid, threads, smem, s>>>(a, t_post, t_pre, t_begin, t_end,
-                                                                       last_seg);
+  auto fn = a.adj_cap ? ms_step_rev_kernel<R, kStepThreads, true> : ms_step_rev_kernel<R, kStepThreads, false>;
+  fn<<<grid, threads, smem, s>>>(a, t_post, t_pre, t_begin, t_end, last_seg);
 }
 
 template <typename R>

@@ -31,6 +31,11 @@ namespace cls {
 __host__ __device__ __forceinline__ int pad4(int x) { return (x + 3) & ~3; }
 
 // ------------------------------------------------------------ step kernels
+// Registers for four CTAs of 256 threads per SM, which is also what the spider's
+// spring tables leave room for (54 KB per CTA).  4096 spiders, 80 substeps, forward
+// / reverse step kernels: 128 threads 15.3 / 19.5 ms, 128 x 8 CTAs 11.1 / 15.9, 256 x
+// 3 12.6 / 14.8, 256 x 4 10.8 / 12.8; 300 spiders differ by 10 %.
+constexpr int kStepCtas = 4;
 // One CTA per env; the substep halves with the env's state in the CTA's
 // shared memory (the fused kernels' carve with the controller buffers sized
 // for the output layer only).  One warp per env
@@ -45,8 +50,8 @@ __host__ __device__ __forceinline__ int pad4(int x) { return (x + 3) & ~3; }
 //   t == t_end:  the range's end (checkpoint, final state).
 // The state comes from checkpoint slot src_slot at t == t_first, else from
 // live_x/v.
-template <typename R, int MAXT>
-__global__ void __launch_bounds__(MAXT)
+template <typename R, int MAXT, bool TAB>
+__global__ void __launch_bounds__(MAXT, sizeof(R) == 4 ? kStepCtas : 1)
 ms_step_fwd_kernel(MsArgs<R> a, int t, int t_first, int t_end, int mode, int src_slot, int k_prev,
                    int k_cur) {
   extern __shared__ __align__(256) char smem_raw[];
@@ -73,7 +78,7 @@ ms_step_fwd_kernel(MsArgs<R> a, int t, int t_first, int t_end, int mode, int src
     for (int o = tid; o < rb.n_out; o += nt) s.buf0[o] = act_f<R>(a.act_out, zl[o] + bo[o]);
     __syncthreads();
     CLS_PHASE(a, 20);
-    fwd_post<R>(a, rb, ed, s, t - 1, mode, k_prev, s.buf0);
+    fwd_post<R, TAB>(a, rb, ed, s, t - 1, mode, k_prev, s.buf0);
     CLS_PHASE(a, 21);
   }
   if (t < t_end) {
@@ -108,8 +113,8 @@ ms_step_fwd_kernel(MsArgs<R> a, int t, int t_first, int t_end, int mode, int src
 // The adjoint state is carried in adj_x/v/h between launches; the first
 // launch of the segment (t_pre = t_end - 1) seeds it (last segment) or takes
 // the carry of the later segment.
-template <typename R, int MAXT>
-__global__ void __launch_bounds__(MAXT)
+template <typename R, int MAXT, bool TAB>
+__global__ void __launch_bounds__(MAXT, sizeof(R) == 4 ? kStepCtas : 1)
 ms_step_rev_kernel(MsArgs<R> a, int t_post, int t_pre, int t_begin, int t_end, int last_seg) {
   extern __shared__ __align__(256) char smem_raw[];
   __shared__ RobotDesc rb;
@@ -136,7 +141,7 @@ ms_step_rev_kernel(MsArgs<R> a, int t_post, int t_pre, int t_begin, int t_end, i
     CLS_PHASE(a, 26);
   }
   if (t_pre >= 0) {
-    rev_pre<R>(a, rb, ed, s, e, t_pre, t_pre - t_begin);
+    rev_pre<R, TAB>(a, rb, ed, s, e, t_pre, t_pre - t_begin);
     CLS_PHASE(a, 27);
     if constexpr (std::is_same<R, float>::value) {
       // dZ of the output layer as the adjoint GEMM's pre-split A operand

@@ -10,6 +10,10 @@
 
 namespace cls {
 
+// threads of the step kernels (one CTA per env): one per vertex of the largest
+// robot up to this many
+constexpr int kStepThreads = 256;
+
 template <typename R>
 struct DenseLaunch {
   // GEMM tile of one job (envs x outputs): tensor-core tile for FP32, SIMT for FP64
@@ -19,7 +23,7 @@ struct DenseLaunch {
   static long long split_floats(int rows, int tile_rows, int k);
   // shared-memory attributes of the step and GEMM kernels; the step kernels'
   // static shared bytes are returned for the capacity check
-  static cudaError_t setup(int threads, size_t* fwd_static, size_t* rev_static, int optin);
+  static cudaError_t setup(size_t* fwd_static, size_t* rev_static, int optin);
   static void step_fwd(const MsArgs<R>& a, int grid, int threads, size_t smem, cudaStream_t s, int t, int t_first,
                        int t_end, int mode, int src_slot, int k_prev, int k_cur);
   static void step_rev(const MsArgs<R>& a, int grid, int threads, size_t smem, cudaStream_t s, int t_post,

@@ -42,6 +42,8 @@ struct RobotDesc {
                                      // one shard of a controller's envs: cls_set_loss_envs)
   int env_first;                     // envs are sorted by type
   int rot_idx[4];                    // heading vertices for robot 100
+  int ell_off, ell_rows;             // per-vertex spring lists for the tables: start (in groups of 8
+                                     // entries), entries per vertex (largest degree)
 };
 
 // Batched-controller offsets of one robot type, kept out of RobotDesc (which
@@ -142,11 +144,13 @@ struct MsArgs {
   const V4<R>* inc_f;                // {rest length, stiffness, actuation coef, 0}
   const int4* inc_p;                 // FP32 only: packed 16-byte incidence records
   const int* spring_out;             // per spring: MLP output index or -1
+  const uint4* inc_ell;              // [vertex][ceil(rows / 8)] groups of 8 incidences, 2 spring + side
+                                     // (0: a, 1: b) in 16 bits, 2 n_s where a vertex has fewer (robots
+                                     // with spring tables)
   const int4* spr_ab;                // per spring {a, b, MLP output or -1, 0} (spr_off)
   const V4<R>* spr_p;                // per spring {rest length, stiffness, actuation coef, 0}
-  int imp_cap;                       // springs of the shared impulse table (0: none)
-  int adj_cap;                       // springs of the shared adjoint table (0: none; the
-                                     // batched step kernels keep their occupancy instead)
+  int imp_cap;                       // entries of the shared impulse table, springs + 1 (0: none)
+  int adj_cap;                       // entries of the shared adjoint table, springs + 1 (0: none)
   const R* w;                        // compact weights
   const R* bias;
   const R* sin_table;                // [T + 1][n_sin], sin(omega (t) dt + 2 pi j / n_sin)
@@ -207,8 +211,8 @@ struct MsArgs {
 
 // ------------------------------------------------------------ shared memory
 // reduction scratch: 8 values x 32 warps, then 32 ints for arg-reductions;
-// the forward pass's fused observable reduction (11 sums and two extrema with
-// their indices per warp) takes kRedFwd.  The reverse pass keeps kRed: with
+// the forward pass's fused observable reduction (11 sums and two extrema per
+// warp, rows of 33) takes kRedFwd.  The reverse pass keeps kRed: with
 // its packed vertex rows its shared memory (155 KB for the largest
 // benchmark robot) sits under the 164 KB carveout step.
 constexpr int kRed = 320;
@@ -313,7 +317,7 @@ struct RevSmem {
   R* dz;           // union region, MLP phase
   V4<R>* part;     // union region, MLP phase: blockDim partials
   R* red;
-  V4<R>* adj;      // per-spring adjoint terms (2 per spring) when MsArgs::adj_cap > 0
+  PairRows<R> adj; // per-spring adjoint terms (d x, d v) when MsArgs::adj_cap > 0
   R* w; R* b;      // the env's controller when MsArgs::w_smem > 0, else null
 };
 
@@ -349,7 +353,8 @@ __device__ __forceinline__ RevSmem<R> carve_rev(char* base, const MsArgs<R>& a) 
   s.gvinc = (V4<R>*)u;
   s.dz = (R*)u;
   s.part = (V4<R>*)(u + ((sizeof(R) * a.smem_dmax + 255) & ~size_t(255)));
-  s.adj = a.adj_cap ? (V4<R>*)take(2 * sizeof(V4<R>) * a.adj_cap) : nullptr;
+  s.adj.lo = a.adj_cap ? (V4<R>*)take(sizeof(V4<R>) * a.adj_cap) : nullptr;
+  s.adj.hi = a.adj_cap ? (V2<R>*)take(sizeof(V2<R>) * a.adj_cap) : nullptr;
   s.w = a.w_smem ? (R*)take(sizeof(R) * a.w_smem) : nullptr;
   s.b = a.w_smem ? (R*)take(sizeof(R) * a.b_smem) : nullptr;
   return s;
@@ -361,7 +366,7 @@ __host__ __device__ inline size_t rev_smem_bytes(int nmax, int amax, int omax, i
   auto rb = [](size_t b) { return (b + 255) & ~size_t(255); };
   return 2 * (rb(sizeof(V4<R>) * nmax) + rb(sizeof(V2<R>) * nmax)) + rb(sizeof(R) * rev_io_values(amax, omax)) +
          rb(sizeof(R) * kRed) + rev_union_bytes<R>(nmax, dmax, threads) +
-         (adj_cap ? rb(2 * sizeof(V4<R>) * adj_cap) : 0);
+         (adj_cap ? rb(sizeof(V4<R>) * adj_cap) + rb(sizeof(V2<R>) * adj_cap) : 0);
 }
 
 // ------------------------------------------------------------- primitives
@@ -509,25 +514,91 @@ __device__ __forceinline__ void gather_vinc_all(const MsArgs<R>& a, const RobotD
   }
 }
 
-// The same v_inc with each spring's impulse computed once: phase A evaluates
-// every spring (spring-parallel, a -> b order as both of its incidences do) into
-// imp[], phase B is gather_vinc_all's half-warp gather with the impulses read
-// from imp[] instead of recomputed, in the same lanes and the same order.  For
-// robots whose impulse table fits in shared memory (MsArgs::imp_cap).
-// spring-parallel table phase: the next spring's records in flight while one
-// is evaluated (spider step kernel, 4096 envs: forward 11.65 -> 11.41 ms per
-// 61 substeps)
-#ifndef CLS_TABLE_PREFETCH
-#define CLS_TABLE_PREFETCH 1
-#endif
+// advance_toi for one vertex (solver_mass_spring.py:119-148); in place
 template <typename R>
-__device__ __forceinline__ void gather_vinc_table(const MsArgs<R>& a, const RobotDesc& rb, int N,
-                                                  const V4<R>* xs, const V4<R>* vs, const R* out,
-                                                  V4<R>* imp, V4<R>* vinc, V4<R>* rec) {
-  constexpr int U = 4;
+__device__ __forceinline__ void advance_vertex(const MsArgs<R>& a, V4<R>& x, V4<R>& v, const V4<R>& vi) {
+  R ov0 = a.drag_s * v.x + vi.x;
+  R ov1 = a.drag_s * v.y + mul_rn<R>(a.dt, a.gravity) + vi.y;
+  R ov2 = a.drag_s * v.z + vi.z;
+  R nv0 = ov0, nv1 = ov1, nv2 = ov2, toi = 0;
+  R nx1 = x.y + a.dt * ov1;
+  if (nx1 < a.ground && ov1 < R(-1e-4)) {
+    toi = -(x.y - a.ground) / ov1;
+    R f = a.friction * (-ov1);
+    nv1 = 0;
+    nv0 = (ov0 < 0) ? fmin(R(0), ov0 + f) : fmax(R(0), ov0 - f);
+    nv2 = (ov2 < 0) ? fmin(R(0), ov2 + f) : fmax(R(0), ov2 - f);
+  }
+  R dtt = a.dt - toi;
+  x.x = x.x + toi * ov0 + dtt * nv0;
+  x.y = x.y + toi * ov1 + dtt * nv1;
+  x.z = x.z + toi * ov2 + dtt * nv2;
+  v.x = nv0; v.y = nv1; v.z = nv2;
+}
+
+// A vertex's list of incidences: the first 24 in registers (loaded together, ahead
+// of the barrier before their use), the rest read as they are needed.
+struct EllRow {
+  static constexpr int kHeld = 3;
+  uint4 w[kHeld];
+  const uint4* rest;
+  __device__ __forceinline__ void load(const uint4* row, int groups) {
+    rest = row;
+#pragma unroll
+    for (int g = 0; g < kHeld; ++g) w[g] = g < groups ? __ldg(row + g) : make_uint4(0, 0, 0, 0);
+  }
+  __device__ __forceinline__ static unsigned at(const uint4& v, int k) {  // k: 0 .. 7
+    const unsigned u = k < 2 ? v.x : (k < 4 ? v.y : (k < 6 ? v.z : v.w));
+    return (k & 1) ? u >> 16 : u & 0xffffu;
+  }
+  template <int K>
+  __device__ __forceinline__ unsigned held() const { return at(w[K / 8], K % 8); }
+  __device__ __forceinline__ unsigned far(int k) const {
+    return reinterpret_cast<const unsigned short*>(rest)[k];
+  }
+};
+
+// Sum of a vertex's incident terms in the order of gather_vinc_all's half-warp:
+// leaf l holds the entries l, l + 16, ... in turn, the leaves are added by the xor
+// tree 8, 4, 2, 1 -- here by one thread, so a warp sums 32 vertices with 32 busy
+// lanes and no shuffles.  add(c, u): adds the term of incidence c to u.
+template <typename R, int M, int L, typename Add>
+__device__ __forceinline__ void ell_leaf(const EllRow& e, int rows, Add add, R (&u)[M]) {
+#pragma unroll
+  for (int m = 0; m < M; ++m) u[m] = 0;
+  if (L < rows) add(e.template held<L>(), u);
+  if constexpr (L + 16 < 8 * EllRow::kHeld) {
+    if (L + 16 < rows) add(e.template held<L + 16>(), u);
+    for (int r = L + 32; r < rows; r += 16) add(e.far(r), u);
+  } else {
+    for (int r = L + 16; r < rows; r += 16) add(e.far(r), u);
+  }
+}
+template <typename R, int M, int L, int STEP, typename Add>
+__device__ __forceinline__ void ell_tree(const EllRow& e, int rows, Add add, R (&u)[M]) {
+  if constexpr (STEP == 16) {
+    ell_leaf<R, M, L>(e, rows, add, u);
+  } else {
+    R w[M];
+    ell_tree<R, M, L, 2 * STEP>(e, rows, add, u);
+    ell_tree<R, M, L + STEP, 2 * STEP>(e, rows, add, w);
+#pragma unroll
+    for (int m = 0; m < M; ++m) u[m] += w[m];
+  }
+}
+
+// apply_spring_force and advance_toi with each spring's impulse computed once:
+// phase A evaluates every spring (spring-parallel, a -> b order as both of its
+// incidences do) into imp[], phase B sums each vertex's impulses in
+// gather_vinc_all's order and advances it, one thread per vertex.  For robots
+// whose impulse table fits in shared memory (MsArgs::imp_cap).  The batched step
+// kernel (4096 spiders: 236 vertices, 1378 springs) is bound by its instructions;
+// the half-warp gather took 7 k of its warp instructions per env, this one 1.5 k.
+template <typename R>
+__device__ __forceinline__ void springs_table(const MsArgs<R>& a, const RobotDesc& rb, int N, V4<R>* xs, V4<R>* vs,
+                                              const R* out, V4<R>* imp, V4<R>* rec) {
   const unsigned long long pol = policy_evict_last();
   const int tid = threadIdx.x, nt = blockDim.x;
-#if CLS_TABLE_PREFETCH
   // the next spring's records are loaded before this one is evaluated, so
   // one pair of L2 loads per thread is always in flight (same arithmetic)
   int4 ab = make_int4(0, 0, -1, 0);
@@ -553,85 +624,29 @@ __device__ __forceinline__ void gather_vinc_table(const MsArgs<R>& a, const Robo
     ab = ab_n;
     f = f_n;
   }
-#else
-  for (int sp = tid; sp < rb.n_s; sp += nt) {
-    const int4 ab = ldg_i4_hint(a.spr_ab + rb.spr_off + sp, pol);
-    const V4<R> f = ldg4_hint<R>(a.spr_p + rb.spr_off + sp, pol);
-    const R act = ab.z >= 0 ? out[ab.z] : R(0);
-    R im[3];
-    spring_impulse<R>(xs[ab.x], xs[ab.y], vs[ab.x], vs[ab.y], f.x, f.y, f.z, act, a.dt, a.dashpot, im);
-    V4<R> r; r.x = im[0]; r.y = im[1]; r.z = im[2]; r.w = 0;
-    imp[sp] = r;
+  if (tid == 0) {
+    V4<R> z; z.x = z.y = z.z = z.w = 0;
+    imp[rb.n_s] = z;  // the entry of absent incidences
   }
-#endif
+  const int rows = rb.ell_rows, groups = (rows + 7) >> 3;
+  const uint4* ell = a.inc_ell + rb.ell_off;
+  EllRow er;
+  if (tid < N) er.load(ell + tid * groups, groups);
   __syncthreads();
-  const int lane = threadIdx.x & 31, wid = (threadIdx.x >> 5), nw = (blockDim.x >> 5);
-  const int l16 = lane & 15, half = lane >> 4;
-  const int* ptr = a.inc_ptr + rb.ptr_off;
-  const int stride = nw * 2;
-  for (int vb0 = wid * 2; vb0 < N; vb0 += stride * U) {
-    const int vb = vb0 + half;
-    int beg[U], end[U];
-    int4 first[U];
-#pragma unroll
-    for (int k = 0; k < U; ++k) {
-      const int v = vb + k * stride;
-      beg[k] = 0;
-      end[k] = 0;
-      if (v < N) { beg[k] = ptr[v]; end[k] = ptr[v + 1]; }
-      const int q = beg[k] + l16;
-      first[k] = make_int4(0, 0, 0, 0);
-      if (q < end[k]) first[k] = ldg_i4_hint(a.inc_i + rb.inc_off + q, pol);
-    }
-#pragma unroll
-    for (int k = 0; k < U; ++k) {
-      const int v = vb + k * stride;
-      R s0 = 0, s1 = 0, s2 = 0;
-      if (v < N) {
-        int q = beg[k] + l16;
-        for (int4 in = first[k]; q < end[k];) {
-          const V4<R> im = imp[in.z];
-          if (in.y == 0) { s0 -= im.x; s1 -= im.y; s2 -= im.z; }
-          else { s0 += im.x; s1 += im.y; s2 += im.z; }
-          q += 16;
-          if (q < end[k]) in = ldg_i4_hint(a.inc_i + rb.inc_off + q, pol);
-        }
-      }
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) {
-        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-        s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-      }
-      if (l16 == 0 && v < N) {
-        V4<R> r; r.x = s0; r.y = s1; r.z = s2; r.w = 0;
-        vinc[v] = r;
-        if (rec) rec[v] = r;
-      }
-    }
+  for (int v = tid; v < N; v += nt) {
+    if (v != tid) er.load(ell + v * groups, groups);
+    R s[3];
+    ell_tree<R, 3, 0, 1>(er, rows, [&](unsigned c, R (&u)[3]) {
+      const V4<R> im = imp[c >> 1];
+      const bool plus = c & 1;
+      u[0] += plus ? im.x : -im.x;
+      u[1] += plus ? im.y : -im.y;
+      u[2] += plus ? im.z : -im.z;
+    }, s);
+    V4<R> vi; vi.x = s[0]; vi.y = s[1]; vi.z = s[2]; vi.w = 0;
+    if (rec) rec[v] = vi;
+    advance_vertex<R>(a, xs[v], vs[v], vi);
   }
-}
-
-// advance_toi for one vertex (solver_mass_spring.py:119-148); in place
-template <typename R>
-__device__ __forceinline__ void advance_vertex(const MsArgs<R>& a, V4<R>& x, V4<R>& v, const V4<R>& vi) {
-  R ov0 = a.drag_s * v.x + vi.x;
-  R ov1 = a.drag_s * v.y + mul_rn<R>(a.dt, a.gravity) + vi.y;
-  R ov2 = a.drag_s * v.z + vi.z;
-  R nv0 = ov0, nv1 = ov1, nv2 = ov2, toi = 0;
-  R nx1 = x.y + a.dt * ov1;
-  if (nx1 < a.ground && ov1 < R(-1e-4)) {
-    toi = -(x.y - a.ground) / ov1;
-    R f = a.friction * (-ov1);
-    nv1 = 0;
-    nv0 = (ov0 < 0) ? fmin(R(0), ov0 + f) : fmax(R(0), ov0 - f);
-    nv2 = (ov2 < 0) ? fmin(R(0), ov2 + f) : fmax(R(0), ov2 - f);
-  }
-  R dtt = a.dt - toi;
-  x.x = x.x + toi * ov0 + dtt * nv0;
-  x.y = x.y + toi * ov1 + dtt * nv1;
-  x.z = x.z + toi * ov2 + dtt * nv2;
-  v.x = nv0; v.y = nv1; v.z = nv2;
 }
 
 // One 4-wide group of controller weights: from the shared-memory copy (SH) or

@@ -21,11 +21,6 @@
 #include "ms_sched.h"
 #include "ms_segment.cuh"
 
-// threads of the batched controller's step kernels (one CTA per env)
-#ifndef CLS_STEP_THREADS
-#define CLS_STEP_THREADS 128
-#endif
-
 namespace cls {
 
 static thread_local std::string g_create_error;
@@ -265,6 +260,7 @@ class SimImpl final : public SimBase {
     std::vector<int4> inc_i, inc_p;
     std::vector<V4<R>> inc_f;
     std::vector<int> spring_out;
+    std::vector<unsigned short> inc_ell;  // see MsArgs::inc_ell
     std::vector<int4> spr_ab;  // per spring {a, b, MLP output or -1, 0}
     std::vector<V4<R>> spr_p;  // per spring {rest length, stiffness, actuation coef, 0}
     int smax = 0;
@@ -354,6 +350,18 @@ class SimImpl final : public SimBase {
         }
       }
       inc_ptr.push_back(run);
+      // the springs per vertex as rows for the tables' sums (robots whose table fits)
+      d.ell_off = (int)(inc_ell.size() / 8);
+      if ((size_t)(h.n_s + 1) * sizeof(V4<R>) <= kImpSmemMax) {
+        for (const std::vector<int>& p : per) d.ell_rows = std::max(d.ell_rows, (int)p.size());
+        const size_t width = ((size_t)d.ell_rows + 7) / 8 * 8;
+        const size_t at = inc_ell.size();
+        CLS_REQUIRE(at / 8 + width * h.n_v / 8 < (1LL << 31), "too many incidences");
+        inc_ell.resize(at + width * h.n_v, (unsigned short)(2 * h.n_s));
+        for (int i = 0; i < h.n_v; ++i)
+          for (size_t p = 0; p < per[i].size(); ++p) inc_ell[at + i * width + p] = (unsigned short)per[i][p];
+        ell_rows_max_ = std::max(ell_rows_max_, d.ell_rows);
+      }
       for (int s = 0; s < h.n_s; ++s) {
         spring_out.push_back(h.out[s]);
         spr_ab.push_back(make_int4(h.sa[s], h.sb[s], h.out[s], 0));
@@ -492,7 +500,7 @@ class SimImpl final : public SimBase {
     // spring impulses computed once per spring into shared memory when the
     // largest robot's table is small (the forward gathers then read them)
     smax_ = smax;
-    imp_cap_ = (size_t)smax * sizeof(V4<R>) <= kImpSmemMax ? smax : 0;
+    imp_cap_ = table_fits() && ell_rows_max_ <= kEllRowsAuto ? smax + 1 : 0;
     fwd_base_ = fwd_smem_bytes<R>(nmax_, dmax, p0max, imp_cap_);
     int dev = 0;
     CLS_CUDA(cudaGetDevice(&dev));
@@ -525,6 +533,9 @@ class SimImpl final : public SimBase {
     d_inc_p_.alloc(std::max<size_t>(1, inc_p.size()));
     d_spring_out_.alloc(std::max<size_t>(1, spring_out.size()));
     d_spr_ab_.alloc(std::max<size_t>(1, spr_ab.size()));
+    d_inc_ell_.alloc(std::max<size_t>(1, inc_ell.size()));
+    if (!inc_ell.empty())
+      CLS_CUDA(cudaMemcpy(d_inc_ell_.p, inc_ell.data(), sizeof(unsigned short) * inc_ell.size(), cudaMemcpyHostToDevice));
     d_spr_p_.alloc(std::max<size_t>(1, spr_p.size()));
     d_w_.alloc(woff);
     d_gw_.alloc(woff);
@@ -647,14 +658,26 @@ class SimImpl final : public SimBase {
   // kernel instances by block size (the register budget follows MAXT)
   using FwdFn = void (*)(MsArgs<R>, int, int, int, int);
   using RevFn = void (*)(MsArgs<R>, int, int, int);
-  FwdFn fwd_fn() const {
-    return threads_ <= 256 ? ms_forward_kernel<R, 256>
-                           : (threads_ <= 512 ? ms_forward_kernel<R, 512> : ms_forward_kernel<R, 1024>);
+  template <bool TAB>
+  FwdFn fwd_of() const {
+    return threads_ <= 256 ? ms_forward_kernel<R, 256, TAB>
+                           : (threads_ <= 512 ? ms_forward_kernel<R, 512, TAB> : ms_forward_kernel<R, 1024, TAB>);
   }
-  RevFn rev_fn() const {
-    return threads_ <= 256 ? ms_reverse_kernel<R, 256>
-                           : (threads_ <= 512 ? ms_reverse_kernel<R, 512> : ms_reverse_kernel<R, 1024>);
+  template <bool TAB>
+  RevFn rev_of() const {
+    return threads_ <= 256 ? ms_reverse_kernel<R, 256, TAB>
+                           : (threads_ <= 512 ? ms_reverse_kernel<R, 512, TAB> : ms_reverse_kernel<R, 1024, TAB>);
   }
+  FwdFn fwd_fn() const { return imp_cap_ ? fwd_of<true>() : fwd_of<false>(); }
+  RevFn rev_fn() const { return adj_entries(threads_) ? rev_of<true>() : rev_of<false>(); }
+  // entries of the fused reverse kernel's adjoint table: none for robots so small
+  // that the direct gather's half-warps take their vertices in two rounds (160
+  // robots of 44 vertices, 512 threads: reverse 1.29 ms with the table, 1.22 without)
+  size_t adj_entries(int threads) const { return 8 * nmax_ > threads ? imp_cap_ : 0; }
+  // the batched step kernels' tables: FP32 only (300 FP64 robots of 44 vertices:
+  // forward + reverse 3.8 ms with tables, 2.7 without)
+  size_t dense_entries() const { return std::is_same<R, float>::value ? imp_cap_ : 0; }
+
 
   // Launch shape of the fused kernels: threads per CTA select the kernel
   // instance; its dynamic shared-memory limit is raised, the largest robot
@@ -672,7 +695,7 @@ class SimImpl final : public SimBase {
     const int keep = threads_;
     threads_ = threads;
     try {
-      const size_t rev0 = rev_smem_bytes<R>(nmax_, smem_amax_, smem_omax_, smem_dmax_, threads, imp_cap_);
+      const size_t rev0 = rev_smem_bytes<R>(nmax_, smem_amax_, smem_omax_, smem_dmax_, threads, adj_entries(threads));
       const size_t ctrl = ctrl_smem_bytes<R>(wspan_max_, bspan_max_);
       int dev = 0, optin = 0;
       CLS_CUDA(cudaGetDevice(&dev));
@@ -842,7 +865,7 @@ class SimImpl final : public SimBase {
   void set_spring_tables(int mode) override {
     CLS_REQUIRE(!capturing_, "the spring tables cannot change during graph capture");
     CLS_REQUIRE(mode >= -1 && mode <= 1, "spring_tables must be -1 (automatic), 0 or 1");
-    const size_t fit = (size_t)smax_ * sizeof(V4<R>) <= kImpSmemMax ? (size_t)smax_ : 0;
+    const size_t fit = table_fits() ? (size_t)smax_ + 1 : 0;
     CLS_REQUIRE(mode != 1 || fit, "the spring tables do not fit in shared memory");
     const size_t keep = imp_cap_;
     auto apply = [&](size_t cap) {
@@ -850,18 +873,19 @@ class SimImpl final : public SimBase {
       fwd_base_ = fwd_smem_bytes<R>(nmax_, smem_dmax_, smem_p0max_, imp_cap_);
       use_shape(threads_, wsh_on_ ? 1 : 0);
       if (d_wt_.p) {  // the batched step kernels carve with the same table
-        dfwd_smem_ = fwd_smem_bytes<R>(nmax_, smem_omax_, smem_p0max_, imp_cap_);
+        dfwd_smem_ = fwd_smem_bytes<R>(nmax_, smem_omax_, smem_p0max_, dense_entries());
+        drev_smem_ = rev_smem_bytes<R>(nmax_, smem_amax_, smem_omax_, smem_omax_, dense_threads_, dense_entries());
         int dev = 0, optin = 0;
         CLS_CUDA(cudaGetDevice(&dev));
         CLS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
         size_t fwd_static = 0, rev_static = 0;
-        CLS_CUDA(DenseLaunch<R>::setup(dense_threads_, &fwd_static, &rev_static, optin));
+        CLS_CUDA(DenseLaunch<R>::setup(&fwd_static, &rev_static, optin));
         CLS_REQUIRE(dfwd_smem_ + fwd_static <= (size_t)optin,
                     "robot too large for the batched controller's step kernels");
       }
     };
     try {
-      apply(mode == 0 ? 0 : fit);
+      apply(mode == 0 || (mode < 0 && ell_rows_max_ > kEllRowsAuto) ? 0 : fit);
     } catch (...) {
       try {
         apply(keep);
@@ -872,6 +896,10 @@ class SimImpl final : public SimBase {
     fwd_done_ = bwd_done_ = false;
   }
   bool spring_tables() const override { return imp_cap_ > 0; }
+  bool table_fits() const { return (size_t)(smax_ + 1) * sizeof(V4<R>) <= kImpSmemMax; }
+  // a thread walks as many rows as the robot's largest degree: tables by default
+  // only up to twice the cube lattices' (24)
+  static constexpr int kEllRowsAuto = 48;
 
   void set_launch_shape(int threads, int ctas, int wsh) override {
     CLS_REQUIRE(!capturing_, "the launch shape cannot change during graph capture");
@@ -1033,10 +1061,11 @@ class SimImpl final : public SimBase {
     a.inc_f = d_inc_f_.p;
     a.inc_p = d_inc_p_.p;
     a.spring_out = d_spring_out_.p;
+    a.inc_ell = reinterpret_cast<const uint4*>(d_inc_ell_.p);
     a.spr_ab = d_spr_ab_.p;
     a.spr_p = d_spr_p_.p;
     a.imp_cap = (int)imp_cap_;
-    a.adj_cap = (int)imp_cap_;
+    a.adj_cap = (int)adj_entries(threads_);
     a.w = d_w_.p;
     a.bias = d_bias_.p;
     a.sin_table = d_sin_.p;
@@ -1329,18 +1358,18 @@ class SimImpl final : public SimBase {
     }
     d_dense_.alloc(std::max<size_t>(1, dd_host_.size()));
     CLS_CUDA(cudaMemcpy(d_dense_.p, dd_host_.data(), sizeof(DenseDesc) * dd_host_.size(), cudaMemcpyHostToDevice));
-    // step kernels: one CTA of CLS_STEP_THREADS threads per env (64 and 128
-    // measured the same on the 4096-env spider); per CTA the fused kernels'
-    // shared-memory carve with the controller buffers sized for the output
-    // layer only (step_args)
-    dense_threads_ = CLS_STEP_THREADS;
-    dfwd_smem_ = fwd_smem_bytes<R>(nmax_, smem_omax_, smem_p0max_, imp_cap_);
-    drev_smem_ = rev_smem_bytes<R>(nmax_, smem_amax_, smem_omax_, smem_omax_, dense_threads_, 0);
+    // step kernels: one CTA per env, a thread per vertex up to kStepThreads (FP64:
+    // 128, its 180 registers leave no second CTA of 256); per
+    // CTA the fused kernels' shared-memory carve with the controller buffers
+    // sized for the output layer only (step_args)
+    dense_threads_ = std::min(f32 ? kStepThreads : 128, std::max(128, (nmax_ + 31) / 32 * 32));
+    dfwd_smem_ = fwd_smem_bytes<R>(nmax_, smem_omax_, smem_p0max_, dense_entries());
+    drev_smem_ = rev_smem_bytes<R>(nmax_, smem_amax_, smem_omax_, smem_omax_, dense_threads_, dense_entries());
     int dev = 0, optin = 0;
     CLS_CUDA(cudaGetDevice(&dev));
     CLS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     size_t fwd_static = 0, rev_static = 0;
-    CLS_CUDA(DenseLaunch<R>::setup(dense_threads_, &fwd_static, &rev_static, optin));
+    CLS_CUDA(DenseLaunch<R>::setup(&fwd_static, &rev_static, optin));
     CLS_REQUIRE(dfwd_smem_ + fwd_static <= (size_t)optin && drev_smem_ + rev_static <= (size_t)optin,
                 "robot too large for the batched controller's step kernels");
     transpose_weights();
@@ -1353,7 +1382,7 @@ class SimImpl final : public SimBase {
     MsArgs<R> b = a;
     b.smem_dmax = smem_omax_;
     b.w_smem = b.b_smem = 0;  // the step kernels read the controller from its GEMM tiles
-    b.adj_cap = 0;            // and keep their residency: the spring adjoint gathers directly
+    b.imp_cap = b.adj_cap = (int)dense_entries();
     b.n_items = E_;
     return b;
   }
@@ -2351,7 +2380,9 @@ class SimImpl final : public SimBase {
   DevBuf<V4<R>> d_spr_p_;
   size_t imp_cap_ = 0;
   int smax_ = 0;
-  static constexpr size_t kImpSmemMax = 48 * 1024;
+  static constexpr size_t kImpSmemMax = 48 * 1024 + 32;  // 3072 springs in FP32 and the zero entry
+  int ell_rows_max_ = 0;
+  DevBuf<unsigned short> d_inc_ell_;
   DevBuf<V4<R>> d_inc_f_, d_ckx_, d_ckv_, d_finx_, d_finv_, d_recx_, d_recv_, d_recvinc_, d_obsc_, d_xfull_,
       d_tv_, d_init_, d_adjx_, d_adjv_;
   DevBuf<R> d_w_, d_gw_, d_bias_, d_gb_, d_bm_, d_bv_, d_wm_, d_wmm_, d_wmv_, d_sin_, d_recin_,

@@ -89,16 +89,18 @@ __device__ __forceinline__ void load_descs(const MsArgs<R>& a, int e, RobotDesc&
 
 // goal columns of the compact input: (vx, vz) / max_speed if duplicate_v > 0,
 // target height if duplicate_h > 0, crawl target if duplicate_c > 0
-// The observables' reductions of one substep in one pass: sums v[0..10]
-// (centre, then the heading sides' coordinate sums and counts) in block_sum's
-// order, and the min / max of the height with block_argext's order -- the same
-// bits as block_sum<R, 3> + 2 x block_argext + block_sum<R, 8>, with two
-// barriers instead of ten.  red: kRedFwd entries (sums at [m * 32 + warp], the
-// extrema at [352 + warp] and [384 + warp], their indices as ints from 416).
+// The observables' reductions of one substep in one pass: sums v[0..10] (centre,
+// then the heading sides' coordinate sums and counts) in block_sum's order, and
+// the min / max of the height -- the same bits as block_sum<R, 3> + extrema +
+// block_sum<R, 8>, with two barriers instead of ten.  Only what is needed where:
+// every thread gets the centre (v[0..2], each warp adds the warps' sums itself, lane
+// m those of component m), the first warp the rest.  (With every thread adding all
+// 11 + 2 values over the warps, the batched step kernel spent a tenth of its
+// instructions here.)  red: kRedFwd entries, sums at [m * 33 + warp], extrema at
+// [363 + warp] and [396 + warp].
 template <typename R>
-__device__ __forceinline__ void block_obs(R (&v)[11], R& lo, int& li, R& hi, int& hidx, R* red) {
+__device__ __forceinline__ void block_obs(R (&v)[11], R& lo, R& hi, R* red) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  int* redi = reinterpret_cast<int*>(red + 416);
 #pragma unroll
   for (int m = 0; m < 11; ++m) {
 #pragma unroll
@@ -106,37 +108,37 @@ __device__ __forceinline__ void block_obs(R (&v)[11], R& lo, int& li, R& hi, int
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
-    const R l2 = __shfl_xor_sync(0xffffffffu, lo, o);
-    const int li2 = __shfl_xor_sync(0xffffffffu, li, o);
-    if ((l2 < lo) || (l2 == lo && li2 > li)) { lo = l2; li = li2; }
-    const R h2 = __shfl_xor_sync(0xffffffffu, hi, o);
-    const int hi2 = __shfl_xor_sync(0xffffffffu, hidx, o);
-    if ((h2 > hi) || (h2 == hi && hi2 > hidx)) { hi = h2; hidx = hi2; }
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
   }
   __syncthreads();
   if (lane == 0) {
 #pragma unroll
-    for (int m = 0; m < 11; ++m) red[m * 32 + wid] = v[m];
-    red[352 + wid] = lo;
-    red[384 + wid] = hi;
-    redi[wid] = li;
-    redi[32 + wid] = hidx;
+    for (int m = 0; m < 11; ++m) red[m * 33 + wid] = v[m];
+    red[363 + wid] = lo;
+    red[396 + wid] = hi;
   }
   __syncthreads();
+  const int rows = wid == 0 ? 13 : 3;
+  R s = 0;
+  if (lane < rows) {
+    if (lane < 11) {
+      for (int w = 0; w < nw; ++w) s += red[lane * 33 + w];
+    } else {
+      const R* x = red + 33 * lane;
+      s = x[0];
+      for (int w = 1; w < nw; ++w) s = lane == 11 ? fmin(s, x[w]) : fmax(s, x[w]);
+    }
+  }
 #pragma unroll
-  for (int m = 0; m < 11; ++m) {
-    R sm = 0;
-    for (int w = 0; w < nw; ++w) sm += red[m * 32 + w];
-    v[m] = sm;
+  for (int m = 0; m < 3; ++m) v[m] = __shfl_sync(0xffffffffu, s, m);
+  if (wid == 0) {
+#pragma unroll
+    for (int m = 3; m < 11; ++m) v[m] = __shfl_sync(0xffffffffu, s, m);
+    hi = __shfl_sync(0xffffffffu, s, 12);
   }
-  lo = red[352]; li = redi[0];
-  hi = red[384]; hidx = redi[32];
-  for (int w = 1; w < nw; ++w) {
-    const R l2 = red[352 + w], h2 = red[384 + w];
-    const int li2 = redi[w], hi2 = redi[32 + w];
-    if ((l2 < lo) || (l2 == lo && li2 > li)) { lo = l2; li = li2; }
-    if ((h2 > hi) || (h2 == hi && hi2 > hidx)) { hi = h2; hidx = hi2; }
-  }
+  lo = red[363];
+  for (int w = 1; w < nw; ++w) lo = fmin(lo, red[363 + w]);
 }
 
 // Heading sides of the env's vertices (set at t = 0 by the first pass) into
@@ -226,7 +228,6 @@ __device__ __forceinline__ void fwd_pre(const MsArgs<R>& a, const RobotDesc& rb,
     const bool heading = rb.robot_id != 100;
     R v[11] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     R lo = R(10), hi = R(-10);
-    int li = 0, hiidx = 0;
     for (int i = tid; i < N; i += nt) {
       const V4<R> p = s.xs[i];
       v[0] += p.x * invN; v[1] += p.y * invN; v[2] += p.z * invN;
@@ -236,32 +237,27 @@ __device__ __forceinline__ void fwd_pre(const MsArgs<R>& a, const RobotDesc& rb,
         else { v[7] += p.x; v[8] += p.y; v[9] += p.z; v[10] += R(1); }
       }
     }
-    block_obs<R>(v, lo, li, hi, hiidx, s.red);
+    block_obs<R>(v, lo, hi, s.red);
     c[0] = v[0]; c[1] = v[1]; c[2] = v[2];
-    R rot;
-    if (heading) {
-      const R d0 = -v[3] * v[10] + v[7] * v[6];
-      const R d2 = -v[5] * v[10] + v[9] * v[6];
-      rot = datan2<R>(d2, d0);
-    } else {
-      R d0 = 0, d2 = 0;
-      if (tid == 0) {
+    // every thread holds the same lo and hprev: no broadcast
+    const R h = (t % a.jump_period == 0) ? lo : fmax(hprev, lo);
+    if (tid == 0) {
+      R d0, d2;
+      if (heading) {
+        d0 = -v[3] * v[10] + v[7] * v[6];
+        d2 = -v[5] * v[10] + v[9] * v[6];
+      } else {
         const V4<R> p = s.xs[rb.rot_idx[0]], q = s.xs[rb.rot_idx[1]];
         const V4<R> u = s.xs[rb.rot_idx[2]], w = s.xs[rb.rot_idx[3]];
         d0 = p.x + q.x - u.x - w.x;
         d2 = p.z + q.z - u.z - w.z;
       }
-      rot = datan2<R>(d2, d0);
-    }
-    // every thread holds the same lo and hprev: no broadcast
-    const R h = (t % a.jump_period == 0) ? lo : fmax(hprev, lo);
-    if (tid == 0) {
       const size_t o = (size_t)t * a.n_envs + e;
       V4<R> cc; cc.x = c[0]; cc.y = c[1]; cc.z = c[2]; cc.w = 0;
       a.obs_center[o] = cc;
       a.obs_height[o] = h;
       a.obs_upper[o] = hi;
-      a.obs_rot[o] = rot;
+      a.obs_rot[o] = datan2<R>(d2, d0);
     }
     hprev = h;
   } else {
@@ -334,8 +330,11 @@ __device__ __forceinline__ void fwd_pre(const MsArgs<R>& a, const RobotDesc& rb,
 }
 
 // Substep t after the controller: actuation record, apply_spring_force
-// (gather form) with the controller outputs `out`, advance_toi.
-template <typename R>
+// (gather form) with the controller outputs `out`, advance_toi.  TAB: spring
+// tables (MsArgs::imp_cap > 0) or not -- kernel instances of their own, because
+// either form's registers cost the other's products their loads in flight (the
+// uneven batch's first pass 18.9 -> 25.4 ms with both in one kernel).
+template <typename R, bool TAB>
 __device__ __forceinline__ void fwd_post(const MsArgs<R>& a, const RobotDesc& rb, const EnvDesc& ed,
                                          const FwdSmem<R>& s, int t, int mode, int kslot, const R* out) {
   const int tid = threadIdx.x, nt = blockDim.x;
@@ -345,12 +344,13 @@ __device__ __forceinline__ void fwd_post(const MsArgs<R>& a, const RobotDesc& rb
     for (int o = tid; o < rb.n_out; o += nt) af[o] = out[o];
   }
   V4<R>* rec = (mode & FWD_RECORD) ? a.rec_vinc + (size_t)kslot * a.v_total + ed.v_off : nullptr;
-  if (s.imp)
-    gather_vinc_table<R>(a, rb, N, s.xs, s.vs, out, s.imp, s.vinc, rec);
-  else
+  if constexpr (TAB) {
+    springs_table<R>(a, rb, N, s.xs, s.vs, out, s.imp, rec);
+  } else {
     gather_vinc_all<R>(a, rb, N, s.xs, s.vs, out, s.vinc, rec);
-  __syncthreads();
-  for (int i = tid; i < N; i += nt) advance_vertex<R>(a, s.xs[i], s.vs[i], s.vinc[i]);
+    __syncthreads();
+    for (int i = tid; i < N; i += nt) advance_vertex<R>(a, s.xs[i], s.vs[i], s.vinc[i]);
+  }
   __syncthreads();
 }
 
@@ -379,7 +379,7 @@ __device__ __forceinline__ void fwd_finish(const MsArgs<R>& a, const RobotDesc& 
 
 // Advances every env from t_begin (state in checkpoint slot src_slot) through
 // t_end (exclusive), i.e. runs pre_advance/nn_input/forward/advance for each t.
-template <typename R, int MAXT>
+template <typename R, int MAXT, bool TAB>
 __global__ void __launch_bounds__(MAXT, 1)
 ms_forward_kernel(MsArgs<R> a, int t_begin0, int t_end0, int mode, int src_slot0) {
   extern __shared__ __align__(256) char smem_raw[];
@@ -430,7 +430,7 @@ ms_forward_kernel(MsArgs<R> a, int t_begin0, int t_end0, int mode, int src_slot0
         R* y = (lo & 1) ? s.buf1 : s.buf0;
         for (int o = tid; o < ((nout + 3) & ~3); o += nt) y[o] = o < nout ? act_f<R>(a.act_out, zr[o] + bo[o]) : R(0);
         __syncthreads();
-        fwd_post<R>(a, rb, ed, s, t, mode_t, kk, y);
+        fwd_post<R, TAB>(a, rb, ed, s, t, mode_t, kk, y);
         continue;
       }
       // controller records: at slot t over the whole episode (FWD_RECCTRL),
@@ -460,7 +460,7 @@ ms_forward_kernel(MsArgs<R> a, int t_begin0, int t_end0, int mode, int src_slot0
         out = y;
       }
       CLS_PHASE(a, 13);
-      fwd_post<R>(a, rb, ed, s, t, mode_t, kk, out);
+      fwd_post<R, TAB>(a, rb, ed, s, t, mode_t, kk, out);
       CLS_PHASE(a, 16);
     }
     fwd_finish<R>(a, rb, ed, s, t_begin, t_end, mode);
@@ -683,19 +683,34 @@ __device__ __forceinline__ void spring_adjoint_one(const MsArgs<R>& a, const Inc
 }
 
 // The same with each spring's adjoint evaluated once: phase A (spring-
-// parallel) stores gd and h per spring in adj[2 s], adj[2 s + 1] and adds the
-// actuation gradient, phase B is spring_adjoint_gather's half-warp gather over
-// the table (same lanes, same order).  For robots whose table fits in shared
-// memory, in the fused reverse kernel (MsArgs::adj_cap).
+// parallel) stores gd and h per spring in adj and adds the actuation gradient,
+// phase B sums each vertex's terms in spring_adjoint_gather's order, one thread
+// per vertex (ell_tree).  For robots whose table fits in shared memory
+// (MsArgs::adj_cap).  4096 spiders' reverse step, 2756 incidences per env: the
+// direct gather issues 43.8 k warp instructions per env, this form half of them.
 template <typename R>
 __device__ __forceinline__ void spring_adjoint_table(const MsArgs<R>& a, const RobotDesc& rb,
                                                      const PairRows<R>& xv, const V4<R>* gvinc, const R* outv,
-                                                     R* gout, V4<R>* adj, const PairRows<R>& gs,
+                                                     R* gout, const PairRows<R>& adj, const PairRows<R>& gs,
                                                      R act_seed_scale, R act_lim, bool act_seed) {
   const unsigned long long pol = policy_evict_last();
-  for (int sp = threadIdx.x; sp < rb.n_s; sp += blockDim.x) {
-    const int4 ab = ldg_i4_hint(a.spr_ab + rb.spr_off + sp, pol);
-    const V4<R> f = ldg4_hint<R>(a.spr_p + rb.spr_off + sp, pol);
+  const int tid = threadIdx.x, nt = blockDim.x;
+  // one spring's records ahead, as springs_table does
+  int4 ab = make_int4(0, 0, -1, 0);
+  V4<R> f;
+  f.x = f.y = f.z = f.w = R(0);
+  if (tid < rb.n_s) {
+    ab = ldg_i4_hint(a.spr_ab + rb.spr_off + tid, pol);
+    f = ldg4_hint<R>(a.spr_p + rb.spr_off + tid, pol);
+  }
+  for (int sp = tid; sp < rb.n_s; sp += nt) {
+    const int nx = sp + nt;
+    int4 ab_n = ab;
+    V4<R> f_n = f;
+    if (nx < rb.n_s) {
+      ab_n = ldg_i4_hint(a.spr_ab + rb.spr_off + nx, pol);
+      f_n = ldg4_hint<R>(a.spr_p + rb.spr_off + nx, pol);
+    }
     const R act = ab.z >= 0 ? outv[ab.z] : R(0);
     V4<R> xa, va, xb, vb;
     xv.get(ab.x, xa, va);
@@ -704,47 +719,39 @@ __device__ __forceinline__ void spring_adjoint_table(const MsArgs<R>& a, const R
                                                    f.z);
     V4<R> g; g.x = t.gd0; g.y = t.gd1; g.z = t.gd2; g.w = 0;
     V4<R> h; h.x = t.h0; h.y = t.h1; h.z = t.h2; h.w = 0;
-    adj[2 * sp] = g;
-    adj[2 * sp + 1] = h;
+    adj.set(sp, g, h);
     if (ab.z >= 0) atomicAdd(gout + ab.z, spring_gact<R>(t.gact, act, act_seed_scale, act_lim, act_seed));
+    ab = ab_n;
+    f = f_n;
   }
+  if (tid == 0) {
+    V4<R> z; z.x = z.y = z.z = z.w = 0;
+    adj.set(rb.n_s, z, z);  // the entry of absent incidences
+  }
+  const int N = rb.n_v, rows = rb.ell_rows, groups = (rows + 7) >> 3;
+  const uint4* ell = a.inc_ell + rb.ell_off;
+  EllRow er;
+  if (tid < N) er.load(ell + tid * groups, groups);
   __syncthreads();
-  const int lane = threadIdx.x & 31, wid = (threadIdx.x >> 5), nw = (blockDim.x >> 5);
-  const int l16 = lane & 15, half = lane >> 4;
-  const int* ptr = a.inc_ptr + rb.ptr_off;
-  const int N = rb.n_v, stride = nw * 2;
-  for (int vb0 = wid * 2; vb0 < N; vb0 += stride) {
-    const int v = vb0 + half;
-    R gxs[3] = {0, 0, 0}, gvs[3] = {0, 0, 0};
-    if (v < N) {
-      const int beg = ptr[v], end = ptr[v + 1];
-      for (int q = beg + l16; q < end; q += 16) {
-        const int4 in = ldg_i4_hint(a.inc_i + rb.inc_off + q, pol);
-        const V4<R> g = adj[2 * in.z], h = adj[2 * in.z + 1];
-        if (in.y == 0) {
-          gxs[0] += g.x; gxs[1] += g.y; gxs[2] += g.z;
-          gvs[0] += h.x; gvs[1] += h.y; gvs[2] += h.z;
-        } else {
-          gxs[0] -= g.x; gxs[1] -= g.y; gxs[2] -= g.z;
-          gvs[0] -= h.x; gvs[1] -= h.y; gvs[2] -= h.z;
-        }
-      }
-    }
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        gxs[c] += __shfl_xor_sync(0xffffffffu, gxs[c], o);
-        gvs[c] += __shfl_xor_sync(0xffffffffu, gvs[c], o);
-      }
-    }
-    if (l16 == 0 && v < N) {
-      V4<R> x, w;
-      gs.get(v, x, w);
-      x.x += gxs[0]; x.y += gxs[1]; x.z += gxs[2];
-      w.x += gvs[0]; w.y += gvs[1]; w.z += gvs[2];
-      gs.set(v, x, w);
-    }
+  for (int v = tid; v < N; v += nt) {
+    if (v != tid) er.load(ell + v * groups, groups);
+    R s[6];
+    ell_tree<R, 6, 0, 1>(er, rows, [&](unsigned c, R (&u)[6]) {
+      V4<R> g, h;
+      adj.get(c >> 1, g, h);
+      const bool minus = c & 1;
+      u[0] += minus ? -g.x : g.x;
+      u[1] += minus ? -g.y : g.y;
+      u[2] += minus ? -g.z : g.z;
+      u[3] += minus ? -h.x : h.x;
+      u[4] += minus ? -h.y : h.y;
+      u[5] += minus ? -h.z : h.z;
+    }, s);
+    V4<R> x, w;
+    gs.get(v, x, w);
+    x.x += s[0]; x.y += s[1]; x.z += s[2];
+    w.x += s[3]; w.y += s[4]; w.z += s[5];
+    gs.set(v, x, w);
   }
 }
 
@@ -863,7 +870,7 @@ __device__ __forceinline__ void advance_adjoint(const MsArgs<R>& a, const V4<R>&
 // Adjoint of substep t up to the controller outputs: x(t), v(t) from the
 // records (slot kslot), advance_toi adjoint, spring-force adjoint, then
 // dz of the output layer (recorded, and left in s.dz).
-template <typename R>
+template <typename R, bool TAB>
 __device__ __forceinline__ void rev_pre(const MsArgs<R>& a, const RobotDesc& rb, const EnvDesc& ed,
                                         const RevSmem<R>& s, int e, int t, int kslot) {
   const int tid = threadIdx.x, nt = blockDim.x;
@@ -901,7 +908,7 @@ __device__ __forceinline__ void rev_pre(const MsArgs<R>& a, const RobotDesc& rb,
     const bool act_seed = (a.loss_mask & LOSS_ACTUATION) && t < st_e && a.th[o] < R(0.1 + 1e-4);
     const R lim = act_seed ? dpow_half<R>(dabs<R>(a.tv[o].x) / R(0.08)) : R(0);
     const R act_scale = R(10) / R(st_e) / Br / R(rb.n_s);
-    if (s.adj)
+    if constexpr (TAB)
       spring_adjoint_table<R>(a, rb, s.xv, s.gvinc, s.bufA, s.bufB, s.adj, s.g, act_scale, lim, act_seed);
     else
       spring_adjoint_gather<R>(a, rb, s.xv, s.gvinc, s.bufA, s.bufB, s.g, act_scale, lim, act_seed);
@@ -1018,7 +1025,7 @@ __device__ __forceinline__ void rev_store_carry(const MsArgs<R>& a, const RobotD
   __syncthreads();
 }
 
-template <typename R, int MAXT>
+template <typename R, int MAXT, bool TAB>
 __global__ void __launch_bounds__(MAXT, 1)
 ms_reverse_kernel(MsArgs<R> a, int t_begin0, int t_end0, int last_seg0) {
   extern __shared__ __align__(256) char smem_raw[];
@@ -1045,7 +1052,7 @@ ms_reverse_kernel(MsArgs<R> a, int t_begin0, int t_end0, int last_seg0) {
     CLS_PHASE_START();
     for (int t = t_end - 1; t >= t_begin; --t) {
       const int kk = t - t_begin;
-      rev_pre<R>(a, rb, ed, s, e, t, kk);
+      rev_pre<R, TAB>(a, rb, ed, s, e, t, kk);
       CLS_PHASE(a, 3);
       // hidden layers of the MLP adjoint
       for (int l = L - 1; l >= 1; --l) {
