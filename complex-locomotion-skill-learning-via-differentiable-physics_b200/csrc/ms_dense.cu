@@ -56,12 +56,12 @@ void DenseLaunch<R>::step_rev(const MsArgs<R>& a, int grid, int threads, size_t 
 }
 
 template <typename R>
-void DenseLaunch<R>::gemm(const MsArgs<R>& a, bool adjoint, int n_jobs, const DenseJob* jobs, int kslot,
-                          cudaStream_t s) {
+void DenseLaunch<R>::gemm(const MsArgs<R>& a, bool adjoint, int n_jobs, const DenseJob* jobs, const TcJob* tc,
+                          int kslot, cudaStream_t s) {
   if constexpr (std::is_same<R, float>::value) {
     const size_t sm = umma::BulkShape<kDenseTN, kBulkStages>::kSmemBytes;
-    if (adjoint) ms_ctrl_gemm_tc_kernel<1><<<n_jobs, umma::kBulkThreads, sm, s>>>(a, jobs, kslot);
-    else ms_ctrl_gemm_tc_kernel<0><<<n_jobs, umma::kBulkThreads, sm, s>>>(a, jobs, kslot);
+    if (adjoint) ms_ctrl_gemm_tc_kernel<1><<<n_jobs, umma::kBulkThreads, sm, s>>>(a, tc, kslot);
+    else ms_ctrl_gemm_tc_kernel<0><<<n_jobs, umma::kBulkThreads, sm, s>>>(a, tc, kslot);
   } else {
     if (adjoint) ms_ctrl_gemm_simt_kernel<R, 1><<<n_jobs, 256, 0, s>>>(a, jobs, kslot);
     else ms_ctrl_gemm_simt_kernel<R, 0><<<n_jobs, 256, 0, s>>>(a, jobs, kslot);

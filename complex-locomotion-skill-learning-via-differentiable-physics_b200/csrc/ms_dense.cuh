@@ -327,60 +327,48 @@ __device__ __forceinline__ float4 mask4(float4 v, int col, int n) {
 
 template <int BWD>
 __global__ void __launch_bounds__(umma::kBulkThreads)
-ms_ctrl_gemm_tc_kernel(MsArgs<float> a, const DenseJob* jobs, int kslot) {
+ms_ctrl_gemm_tc_kernel(MsArgs<float> a, const TcJob* jobs, int kslot) {
   extern __shared__ __align__(1024) float smem_f[];
   __shared__ umma::BulkShared bs;
-  const DenseJob jb = jobs[blockIdx.x];
-  const RobotDesc& rb = a.robots[jb.robot];
-  const DenseDesc& dd = a.dense[jb.robot];
-  const EnvDesc& e0 = a.envs[rb.env_first];
-  const int l = jb.layer;
-  const int kin = BWD ? rb.width[l + 1] : rb.width[l];
-  const int nkt = (kin + 31) / 32;
-  const float* ab = a.tiles + (BWD ? dd.ta_b[l] : dd.ta_f[l]) + (size_t)(jb.m0 / umma::TM) * nkt * 64 * umma::TM;
-  const float* bb = a.tiles + (BWD ? dd.tb_b[l] : dd.tb_f[l]) + (size_t)(jb.n0 / kDenseTN) * nkt * 64 * kDenseTN;
-  const int m_valid = min(umma::TM, rb.n_env - jb.m0);
-  const int ncol = BWD ? (l > 0 ? rb.width[l] : 3 * rb.n_v) : rb.width[l + 1];
-  const int n_valid = min(kDenseTN, ncol - jb.n0);
-  const int act = a.act_hidden;
-  const bool ok = umma::tile_gemm_bulk<kDenseTN, kBulkStages>(smem_f, bs, ab, bb, nkt, [&](const float* cs, int ld) {
-    constexpr int C4 = kDenseTN / 4;
-    for (int q = threadIdx.x; q < umma::TM * C4; q += blockDim.x) {
-      const int i = q / C4, j = 4 * (q % C4);
-      if (i >= m_valid || j >= n_valid) continue;
-      const float4 v = *reinterpret_cast<const float4*>(cs + i * ld + j);
-      const int row = jb.m0 + i, col = jb.n0 + j;
-      if (!BWD) {
-        const int w = rb.width[l + 1];
-        float* zr = a.rec_z + a.z_base[l] + (size_t)kslot * a.z_total[l] + e0.z_off[l] + (size_t)row * pad4(w) + col;
-        *reinterpret_cast<float4*>(zr) = v;
-        if (l + 1 < rb.n_layers) {
-          const float4 b = *reinterpret_cast<const float4*>(a.bias + rb.b_off[l] + col);
-          const float4 y = make_float4(act_f<float>(act, v.x + b.x), act_f<float>(act, v.y + b.y),
-                                       act_f<float>(act, v.z + b.z), act_f<float>(act, v.w + b.w));
-          const umma::SplitTiles st{a.tiles + dd.ta_f[l + 1], umma::TM, (w + 31) / 32};
-          st.store4(row, col, mask4(y, col, w));
-        }
-      } else if (l > 0) {
-        const int w = rb.width[l];
-        const size_t o = a.z_base[l - 1] + (size_t)kslot * a.z_total[l - 1] + e0.z_off[l - 1] + (size_t)row * pad4(w) + col;
-        const float4 z = *reinterpret_cast<const float4*>(a.rec_z + o);
-        const float4 b = *reinterpret_cast<const float4*>(a.bias + rb.b_off[l - 1] + col);
-        const float4 dz = mask4(make_float4(v.x * act_d<float>(act, z.x + b.x), v.y * act_d<float>(act, z.y + b.y),
-                                            v.z * act_d<float>(act, z.z + b.z), v.w * act_d<float>(act, z.w + b.w)),
-                                col, w);
-        *reinterpret_cast<float4*>(a.rec_dz + o) = dz;
-        const umma::SplitTiles st{a.tiles + dd.ta_b[l - 1], umma::TM, (w + 31) / 32};
-        st.store4(row, col, dz);
-      } else {
-        float* dp = a.din + (size_t)3 * (e0.v_off + (size_t)row * rb.n_v) + col;
-        const float vv[4] = {v.x, v.y, v.z, v.w};
+  const TcJob jb = jobs[blockIdx.x];
+  const int act = a.act_hidden, w = jb.w;
+  const int zl = jb.z_layer < 0 ? 0 : jb.z_layer;
+  const size_t z0 = a.z_base[zl] + (size_t)kslot * a.z_total[zl] + jb.z_off;
+  const umma::SplitTiles st{a.tiles + (jb.split < 0 ? 0 : jb.split), umma::TM, (w + 31) / 32};
+  const bool ok = umma::tile_gemm_bulk<kDenseTN, kBulkStages>(
+      smem_f, bs, a.tiles + jb.a, a.tiles + jb.b, jb.nkt, [&](const float* cs, int ld) {
+        constexpr int C4 = kDenseTN / 4;
+        for (int q = threadIdx.x; q < umma::TM * C4; q += blockDim.x) {
+          const int i = q / C4, j = 4 * (q % C4);
+          if (i >= jb.m_valid || j >= jb.n_valid) continue;
+          const float4 v = *reinterpret_cast<const float4*>(cs + i * ld + j);
+          const int row = jb.m0 + i, col = jb.n0 + j;
+          const size_t o = z0 + (size_t)row * pad4(w) + col;
+          if (!BWD) {
+            *reinterpret_cast<float4*>(a.rec_z + o) = v;
+            if (jb.split >= 0) {
+              const float4 b = *reinterpret_cast<const float4*>(a.bias + jb.bias + col);
+              const float4 y = make_float4(act_f<float>(act, v.x + b.x), act_f<float>(act, v.y + b.y),
+                                           act_f<float>(act, v.z + b.z), act_f<float>(act, v.w + b.w));
+              st.store4(row, col, mask4(y, col, w));
+            }
+          } else if (jb.split >= 0) {
+            const float4 z = *reinterpret_cast<const float4*>(a.rec_z + o);
+            const float4 b = *reinterpret_cast<const float4*>(a.bias + jb.bias + col);
+            const float4 dz = mask4(make_float4(v.x * act_d<float>(act, z.x + b.x), v.y * act_d<float>(act, z.y + b.y),
+                                                v.z * act_d<float>(act, z.z + b.z), v.w * act_d<float>(act, z.w + b.w)),
+                                    col, w);
+            *reinterpret_cast<float4*>(a.rec_dz + o) = dz;
+            st.store4(row, col, dz);
+          } else {
+            float* dp = a.din + (size_t)3 * (jb.v_off + (size_t)row * jb.n_v) + col;
+            const float vv[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (j + u < n_valid) dp[u] = vv[u];
-      }
-    }
-  }, umma::WaitPolicy{a.gemm_wait_limit, a.gemm_starve});
+            for (int u = 0; u < 4; ++u)
+              if (j + u < jb.n_valid) dp[u] = vv[u];
+          }
+        }
+      }, umma::WaitPolicy{a.gemm_wait_limit, a.gemm_starve});
   if (!ok && threadIdx.x == 0) atomicOr(a.status, ERR_TIMEOUT);
   if (threadIdx.x < 32) umma::tmem_relinquish();
 }

@@ -28,7 +28,8 @@ struct DenseLaunch {
                        int t_end, int mode, int src_slot, int k_prev, int k_cur);
   static void step_rev(const MsArgs<R>& a, int grid, int threads, size_t smem, cudaStream_t s, int t_post,
                        int t_pre, int t_begin, int t_end, int last_seg);
-  static void gemm(const MsArgs<R>& a, bool adjoint, int n_jobs, const DenseJob* jobs, int kslot, cudaStream_t s);
+  // (FP32 takes the same tiles from `tc`)
+  static void gemm(const MsArgs<R>& a, bool adjoint, int n_jobs, const DenseJob* jobs, const TcJob* tc, int kslot, cudaStream_t s);
   // FP32 weight-gradient products of record slots [slot0, slot0 + nslots):
   // record transposes (grid grid_x x n_cols x slot groups) then the tensor-core
   // tiles (n_jobs CTAs), adding into gw / gb

@@ -87,6 +87,20 @@ struct DenseJob {
   int robot, layer, m0, n0;
 };
 
+// The same tile for the tensor-core kernel, with everything it would look up in
+// the robot, env and operand tables (a chain of four dependent loads).
+struct alignas(16) TcJob {
+  long long a, b;     // operand blocks in `tiles`: block (row tile, 0) of A and of B
+  long long split;    // next GEMM's A operand, written by the epilogue (< 0: none)
+  int nkt;            // K blocks of 32
+  int m_valid, n_valid, m0, n0;
+  int w;              // columns of the record row the epilogue writes
+  int z_layer, z_off; // record (rec_z forward, rec_dz adjoint) layer and the type's first row
+  int bias;           // bias offset of that record's layer
+  int v_off, n_v;     // d input positions (adjoint of layer 0): the type's first vertex
+  int pad;
+};
+
 // one (robot, layer) block of the pre-split weight packing
 struct SplitSeg {
   long long w_off, tf_off, tb_off;

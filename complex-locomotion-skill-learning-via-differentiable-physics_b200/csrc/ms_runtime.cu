@@ -1356,6 +1356,38 @@ class SimImpl final : public SimBase {
       d_ssegs_.alloc(std::max<size_t>(1, ssegs_.size()));
       CLS_CUDA(cudaMemcpy(d_ssegs_.p, ssegs_.data(), sizeof(SplitSeg) * ssegs_.size(), cudaMemcpyHostToDevice));
     }
+    if constexpr (f32) {
+      // the tensor-core kernel's form of the tiles (forward, then adjoint)
+      std::vector<TcJob> tc;
+      const int n_fwd = jb_off_[0];
+      for (size_t k = 0; k < jobs_h_.size(); ++k) {
+        const DenseJob& jb = jobs_h_[k];
+        const bool adj = (int)k >= n_fwd;
+        const RobotDesc& d = rd_host_[jb.robot];
+        const DenseDesc& dd = dd_host_[jb.robot];
+        const EnvDesc& e0 = ed_host_[d.env_first];
+        const int l = jb.layer, kin = adj ? d.width[l + 1] : d.width[l];
+        const int ncol = adj ? (l > 0 ? d.width[l] : 3 * d.n_v) : d.width[l + 1];
+        TcJob t{};
+        t.nkt = (kin + 31) / 32;
+        t.a = (adj ? dd.ta_b[l] : dd.ta_f[l]) + (long long)(jb.m0 / tm) * t.nkt * 64 * tm;
+        t.b = (adj ? dd.tb_b[l] : dd.tb_f[l]) + (long long)(jb.n0 / tn) * t.nkt * 64 * tn;
+        t.m0 = jb.m0;
+        t.n0 = jb.n0;
+        t.m_valid = std::min(tm, d.n_env - jb.m0);
+        t.n_valid = std::min(tn, ncol - jb.n0);
+        t.w = ncol;
+        t.z_layer = adj ? l - 1 : l;
+        t.z_off = t.z_layer >= 0 ? e0.z_off[t.z_layer] : 0;
+        t.bias = t.z_layer >= 0 ? d.b_off[t.z_layer] : 0;
+        t.split = adj ? (l > 0 ? dd.ta_b[l - 1] : -1) : (l + 1 < d.n_layers ? dd.ta_f[l + 1] : -1);
+        t.v_off = e0.v_off;
+        t.n_v = d.n_v;
+        tc.push_back(t);
+      }
+      d_tcjobs_.alloc(std::max<size_t>(1, tc.size()));
+      CLS_CUDA(cudaMemcpy(d_tcjobs_.p, tc.data(), sizeof(TcJob) * tc.size(), cudaMemcpyHostToDevice));
+    }
     d_dense_.alloc(std::max<size_t>(1, dd_host_.size()));
     CLS_CUDA(cudaMemcpy(d_dense_.p, dd_host_.data(), sizeof(DenseDesc) * dd_host_.size(), cudaMemcpyHostToDevice));
     // step kernels: one CTA per env, a thread per vertex up to kStepThreads (FP64:
@@ -1392,8 +1424,10 @@ class SimImpl final : public SimBase {
   void ctrl_gemm(const MsArgs<R>& a, bool bwd, int l, int kslot) {
     const int cnt = bwd ? jb_cnt_[l] : jf_cnt_[l];
     if (cnt == 0) return;
-    const DenseJob* jobs = d_jobs_.p + (bwd ? jb_off_[l] : jf_off_[l]);
-    timed(bwd ? PK_CGEMM_ADJ : PK_CGEMM, [&] { DenseLaunch<R>::gemm(a, bwd, cnt, jobs, kslot, stream); });
+    const int at = bwd ? jb_off_[l] : jf_off_[l];
+    const DenseJob* jobs = d_jobs_.p + at;
+    const TcJob* tc = d_tcjobs_.p ? d_tcjobs_.p + at : nullptr;
+    timed(bwd ? PK_CGEMM_ADJ : PK_CGEMM, [&] { DenseLaunch<R>::gemm(a, bwd, cnt, jobs, tc, kslot, stream); });
   }
 
   // forward over [t_first, t_end): a step launch per substep boundary and the
@@ -2398,6 +2432,7 @@ class SimImpl final : public SimBase {
   std::vector<DenseJob> jobs_h_;
   int jf_off_[kMaxLayers] = {0}, jf_cnt_[kMaxLayers] = {0}, jb_off_[kMaxLayers] = {0}, jb_cnt_[kMaxLayers] = {0};
   DevBuf<DenseJob> d_jobs_;
+  DevBuf<TcJob> d_tcjobs_;
   DevBuf<TransSeg> d_tsegs_;
   DevBuf<V4<R>> d_livex_, d_livev_;
   DevBuf<R> d_envout_, d_envobs_, d_envaux_;

@@ -217,7 +217,16 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t mbar, uint32_t by
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
 }
 
-constexpr int kBulkThreads = 128;  // 4 warps: warp w reads accumulator lanes [32 w, 32 w + 32)
+// 16 warps: warp w reads accumulator lanes [32 (w % 4), ..) of every fourth group of 8
+// columns, starting at group w / 4.  The K loop needs two threads; the rest are for
+// the epilogue, whose activations and splits took 4 warps longer than the products
+// (CLS_BULK_THREADS 128 / 256 / 512: 126 / 108 / 104 us per substep and its adjoint in a
+// graph of 256 spiders with four controller launches each, 450 / 428 / 424 at 4096)
+#ifndef CLS_BULK_THREADS
+#define CLS_BULK_THREADS 512
+#endif
+constexpr int kBulkThreads = CLS_BULK_THREADS;
+static_assert(kBulkThreads % 128 == 0, "whole groups of four warps");
 constexpr int kMaxStages = 6;
 
 template <int TN, int S>
@@ -313,13 +322,13 @@ __device__ bool tile_gemm_bulk(float* smem, BulkShared& bs, const float* a_block
   constexpr int ld = TN + 4;      // row pitch of the staged tile: 16-byte rows, no bank conflicts
   static_assert((size_t)TM * ld * 4 <= Sh::kRing, "staged tile must fit in the ring");
   if (ok) {
-    // lane i of warp w holds row 32 w + i: two 16-byte stores per 8 columns
-    const int i = warp * 32 + lane;
+    // lane i of warp w holds row 32 (w % 4) + i: two 16-byte stores per 8 columns
+    const int i = (warp & 3) * 32 + lane;
 #pragma unroll 1
-    for (int j0 = 0; j0 < TN; j0 += 8) {
+    for (int j0 = 8 * (warp >> 2); j0 < TN; j0 += 8 * (kBulkThreads / 128)) {
       float v[8];
       if (nkt > 0) {
-        tmem_ld8(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)j0, v);
+        tmem_ld8(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)j0, v);
       } else {
 #pragma unroll
         for (int q = 0; q < 8; ++q) v[q] = 0.0f;
