@@ -8,6 +8,29 @@
 
 namespace cls {
 
+namespace {
+// A launch of the substep chain: as a programmatic dependent, so that its
+// prologue (launch, tables, tensor memory) runs while the launch before it ends.
+// Each kernel of the chain releases its dependent at once and waits, before it
+// reads what an earlier launch wrote, until all of them have finished; the tables
+// read ahead of that wait are laid out when the batch is prepared.  4096 spiders, a
+// training step of 80 substeps: 35.5 -> 33.8 ms; 300: 14.6 -> 14.3.
+template <typename... P, typename... A>
+cudaError_t chain(void (*fn)(P...), int grid, int threads, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t c{};
+  cudaLaunchAttribute at{};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, fn, P(args)...);
+}
+}  // namespace
+
 template <typename R>
 int DenseLaunch<R>::tile_m() { return std::is_same<R, float>::value ? umma::TM : kSimtTile; }
 template <typename R>
@@ -42,29 +65,29 @@ cudaError_t DenseLaunch<R>::setup(size_t* fwd_static, size_t* rev_static, int op
 }
 
 template <typename R>
-void DenseLaunch<R>::step_fwd(const MsArgs<R>& a, int grid, int threads, size_t smem, cudaStream_t s, int t,
+cudaError_t DenseLaunch<R>::step_fwd(const MsArgs<R>& a, int grid, int threads, size_t smem, cudaStream_t s, int t,
                               int t_first, int t_end, int mode, int src_slot, int k_prev, int k_cur) {
   auto fn = a.imp_cap ? ms_step_fwd_kernel<R, kStepThreads, true> : ms_step_fwd_kernel<R, kStepThreads, false>;
-  fn<<<grid, threads, smem, s>>>(a, t, t_first, t_end, mode, src_slot, k_prev, k_cur);
+  return chain(fn, grid, threads, smem, s, a, t, t_first, t_end, mode, src_slot, k_prev, k_cur);
 }
 
 template <typename R>
-void DenseLaunch<R>::step_rev(const MsArgs<R>& a, int grid, int threads, size_t smem, cudaStream_t s, int t_post,
+cudaError_t DenseLaunch<R>::step_rev(const MsArgs<R>& a, int grid, int threads, size_t smem, cudaStream_t s, int t_post,
                               int t_pre, int t_begin, int t_end, int last_seg) {
   auto fn = a.adj_cap ? ms_step_rev_kernel<R, kStepThreads, true> : ms_step_rev_kernel<R, kStepThreads, false>;
-  fn<<<grid, threads, smem, s>>>(a, t_post, t_pre, t_begin, t_end, last_seg);
+  return chain(fn, grid, threads, smem, s, a, t_post, t_pre, t_begin, t_end, last_seg);
 }
 
 template <typename R>
-void DenseLaunch<R>::gemm(const MsArgs<R>& a, bool adjoint, int n_jobs, const DenseJob* jobs, const TcJob* tc,
-                          int kslot, cudaStream_t s) {
+cudaError_t DenseLaunch<R>::gemm(const MsArgs<R>& a, bool adjoint, int n_jobs, const DenseJob* jobs, const TcJob* tc,
+                                 int kslot, cudaStream_t s) {
   if constexpr (std::is_same<R, float>::value) {
     const size_t sm = umma::BulkShape<kDenseTN, kBulkStages>::kSmemBytes;
-    if (adjoint) ms_ctrl_gemm_tc_kernel<1><<<n_jobs, umma::kBulkThreads, sm, s>>>(a, tc, kslot);
-    else ms_ctrl_gemm_tc_kernel<0><<<n_jobs, umma::kBulkThreads, sm, s>>>(a, tc, kslot);
+    return chain(adjoint ? ms_ctrl_gemm_tc_kernel<1> : ms_ctrl_gemm_tc_kernel<0>, n_jobs, umma::kBulkThreads, sm, s, a,
+                 tc, kslot);
   } else {
-    if (adjoint) ms_ctrl_gemm_simt_kernel<R, 1><<<n_jobs, 256, 0, s>>>(a, jobs, kslot);
-    else ms_ctrl_gemm_simt_kernel<R, 0><<<n_jobs, 256, 0, s>>>(a, jobs, kslot);
+    return chain(adjoint ? ms_ctrl_gemm_simt_kernel<R, 1> : ms_ctrl_gemm_simt_kernel<R, 0>, n_jobs, 256, 0, s, a, jobs,
+                 kslot);
   }
 }
 

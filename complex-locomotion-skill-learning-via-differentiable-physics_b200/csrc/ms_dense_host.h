@@ -24,12 +24,13 @@ struct DenseLaunch {
   // shared-memory attributes of the step and GEMM kernels; the step kernels'
   // static shared bytes are returned for the capacity check
   static cudaError_t setup(size_t* fwd_static, size_t* rev_static, int optin);
-  static void step_fwd(const MsArgs<R>& a, int grid, int threads, size_t smem, cudaStream_t s, int t, int t_first,
+  static cudaError_t step_fwd(const MsArgs<R>& a, int grid, int threads, size_t smem, cudaStream_t s, int t, int t_first,
                        int t_end, int mode, int src_slot, int k_prev, int k_cur);
-  static void step_rev(const MsArgs<R>& a, int grid, int threads, size_t smem, cudaStream_t s, int t_post,
+  static cudaError_t step_rev(const MsArgs<R>& a, int grid, int threads, size_t smem, cudaStream_t s, int t_post,
                        int t_pre, int t_begin, int t_end, int last_seg);
   // (FP32 takes the same tiles from `tc`)
-  static void gemm(const MsArgs<R>& a, bool adjoint, int n_jobs, const DenseJob* jobs, const TcJob* tc, int kslot, cudaStream_t s);
+  static cudaError_t gemm(const MsArgs<R>& a, bool adjoint, int n_jobs, const DenseJob* jobs,
+                          const TcJob* tc, int kslot, cudaStream_t s);
   // FP32 weight-gradient products of record slots [slot0, slot0 + nslots):
   // record transposes (grid grid_x x n_cols x slot groups) then the tensor-core
   // tiles (n_jobs CTAs), adding into gw / gb

@@ -1427,7 +1427,7 @@ class SimImpl final : public SimBase {
     const int at = bwd ? jb_off_[l] : jf_off_[l];
     const DenseJob* jobs = d_jobs_.p + at;
     const TcJob* tc = d_tcjobs_.p ? d_tcjobs_.p + at : nullptr;
-    timed(bwd ? PK_CGEMM_ADJ : PK_CGEMM, [&] { DenseLaunch<R>::gemm(a, bwd, cnt, jobs, tc, kslot, stream); });
+    timed(bwd ? PK_CGEMM_ADJ : PK_CGEMM, [&] { CLS_CUDA(DenseLaunch<R>::gemm(a, bwd, cnt, jobs, tc, kslot, stream)); });
   }
 
   // forward over [t_first, t_end): a step launch per substep boundary and the
@@ -1440,8 +1440,8 @@ class SimImpl final : public SimBase {
       const int k_prev = t > t_first ? (first_pass ? (t - 1) % K_ : t - 1 - t_first) : 0;
       const int k_cur = t < t_end ? (first_pass ? t % K_ : t - t_first) : 0;
       timed(kind, [&] {
-        DenseLaunch<R>::step_fwd(step_args(a), step_grid(), dense_threads_, dfwd_smem_, stream, t, t_first, t_end, mode,
-                                 src_slot, k_prev, k_cur);
+        CLS_CUDA(DenseLaunch<R>::step_fwd(step_args(a), step_grid(), dense_threads_, dfwd_smem_, stream, t, t_first,
+                                          t_end, mode, src_slot, k_prev, k_cur));
       });
       if (t < t_end)
         for (int l = 0; l < L_; ++l) ctrl_gemm(a, false, l, k_cur);
@@ -1455,8 +1455,8 @@ class SimImpl final : public SimBase {
       const int t_post = (t + 1 < t1) ? t + 1 : -1;
       const int t_pre = (t >= t0) ? t : -1;
       timed(PK_REV, [&] {
-        DenseLaunch<R>::step_rev(step_args(a), step_grid(), dense_threads_, drev_smem_, stream, t_post, t_pre, t0, t1,
-                                 last ? 1 : 0);
+        CLS_CUDA(DenseLaunch<R>::step_rev(step_args(a), step_grid(), dense_threads_, drev_smem_, stream, t_post, t_pre,
+                                          t0, t1, last ? 1 : 0));
       });
       if (t_pre >= 0)
         for (int l = L_ - 1; l >= 0; --l) ctrl_gemm(a, true, l, t_pre - t0);

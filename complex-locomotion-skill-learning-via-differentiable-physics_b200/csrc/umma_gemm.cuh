@@ -131,6 +131,12 @@ __device__ __forceinline__ void tmem_relinquish() {
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 
+// Programmatic dependent launch: lets the next launch of the stream start its
+// prologue, and waits until the launches before this one have finished (no effect
+// in launches without the attribute).
+__device__ __forceinline__ void dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void dependents_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // 32 lanes x 8 consecutive 32-bit columns
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float v[8]) {
   uint32_t r[8];
@@ -279,6 +285,7 @@ __device__ bool tile_gemm_bulk(float* smem, BulkShared& bs, const float* a_block
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  dependents_wait();  // the operands come from the launches before this one
   const uint32_t tmem = bs.tmem_base;
   constexpr uint32_t idesc = instr_desc_tf32(TM, TN);
   if (tid == 0 && !wp.starve) {
