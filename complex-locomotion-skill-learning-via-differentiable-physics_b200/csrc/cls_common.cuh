@@ -55,6 +55,12 @@ __device__ __forceinline__ unsigned long long policy_evict_last() {
   return p;
 }
 
+// Programmatic dependent launch: lets the next launch of the stream start its
+// prologue, and waits until the launches before this one have finished (no effect
+// in launches without the attribute).
+__device__ __forceinline__ void dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void dependents_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 template <typename R> __device__ __forceinline__ V4<R> ldg4_hint(const V4<R>* p, unsigned long long pol);
 template <> __device__ __forceinline__ V4<float> ldg4_hint<float>(const V4<float>* p, unsigned long long pol) {
   V4<float> r;

@@ -431,6 +431,7 @@ ms_cluster_forward_kernel(MsArgs<R> a, ClusterCaps cap, int t_begin0, int t_end0
   __shared__ EnvDesc ed;
   const int C = (int)cl::size(), rank = (int)cl::rank();
   const int item = blockIdx.x / C;
+  dependents_launch();  // the single-CTA launch of the lighter envs, if there is one
   if (item >= a.n_items) return;
   cl::FwdShared<R> s;
   cl::carve<R>(smem_raw, cap, &s);
@@ -664,6 +665,7 @@ ms_cluster_reverse_kernel(MsArgs<R> a, ClusterCaps cap, int t_begin0, int t_end0
   __shared__ EnvDesc ed;
   const int C = (int)cl::size(), rank = (int)cl::rank();
   const int item = blockIdx.x / C;
+  dependents_launch();  // the single-CTA launch of the lighter envs, if there is one
   if (item >= a.n_items) return;
   cl::RevShared<R> s;
   cl::carve<R>(smem_raw, cap, C, blockDim.x, &s);

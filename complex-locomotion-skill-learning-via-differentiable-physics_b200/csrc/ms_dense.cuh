@@ -57,14 +57,14 @@ ms_step_fwd_kernel(MsArgs<R> a, int t, int t_first, int t_end, int mode, int src
   extern __shared__ __align__(256) char smem_raw[];
   __shared__ RobotDesc rb;
   __shared__ EnvDesc ed;
-  umma::dependents_launch();
+  dependents_launch();
   const int item = blockIdx.x;
   if (item >= a.n_items) return;
   FwdSmem<R> s = carve_fwd<R>(smem_raw, a);
   const int tid = threadIdx.x, nt = blockDim.x;
   const int e = a.order[item];
   load_descs<R>(a, e, rb, ed);
-  umma::dependents_wait();
+  dependents_wait();
   const int N = rb.n_v, L = rb.n_layers;
   CLS_PHASE_START();
   {
@@ -121,14 +121,14 @@ ms_step_rev_kernel(MsArgs<R> a, int t_post, int t_pre, int t_begin, int t_end, i
   extern __shared__ __align__(256) char smem_raw[];
   __shared__ RobotDesc rb;
   __shared__ EnvDesc ed;
-  umma::dependents_launch();
+  dependents_launch();
   const int item = blockIdx.x;
   if (item >= a.n_items) return;
   RevSmem<R> s = carve_rev<R>(smem_raw, a);
   const int tid = threadIdx.x, nt = blockDim.x;
   const int e = a.order[item];
   load_descs<R>(a, e, rb, ed);
-  umma::dependents_wait();
+  dependents_wait();
   const int N = rb.n_v;
   R hcarry = 0;
   CLS_PHASE_START();
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(umma::kBulkThreads)
 ms_ctrl_gemm_tc_kernel(MsArgs<float> a, const TcJob* jobs, int kslot) {
   extern __shared__ __align__(1024) float smem_f[];
   __shared__ umma::BulkShared bs;
-  umma::dependents_launch();
+  dependents_launch();
   const TcJob jb = jobs[blockIdx.x];
   const int act = a.act_hidden, w = jb.w;
   const int zl = jb.z_layer < 0 ? 0 : jb.z_layer;
@@ -560,8 +560,8 @@ __device__ __forceinline__ void simt_tile(const Op& op, int kpad, int m_valid, i
 
 template <typename R, int BWD>
 __global__ void __launch_bounds__(256) ms_ctrl_gemm_simt_kernel(MsArgs<R> a, const DenseJob* jobs, int kslot) {
-  umma::dependents_launch();
-  umma::dependents_wait();
+  dependents_launch();
+  dependents_wait();
   const DenseJob jb = jobs[blockIdx.x];
   int m_valid, n_valid, kpad;
   if (BWD) {

@@ -7,6 +7,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <memory>
 #include <numeric>
 #include <string>
@@ -747,7 +748,7 @@ class SimImpl final : public SimBase {
   };
   void plan_clusters(int optin) {
     plans_.clear();
-    batch_plan_ = -1;
+    batch_split_ = Split{};
     if (threads_ > ClusterLaunch<R>::max_threads()) return;
     size_t fwd_max = 0, rev_max = 0;
     CLS_CUDA(ClusterLaunch<R>::setup(optin, &fwd_max, &rev_max));
@@ -782,42 +783,83 @@ class SimImpl final : public SimBase {
       CLS_CUDA(ClusterLaunch<R>::resident(C, threads_, p.fwd_smem, p.rev_smem, &p.resident));
       if (p.resident > 0) plans_.push_back(p);
     }
-    const ClusterPlan* all = cluster_plan(order_host_.data(), E_);
-    batch_plan_ = all ? (int)(all - plans_.data()) : -1;
+    batch_split_ = split_envs(order_host_.data(), E_);
   }
 
-  // Cluster size for a launch over envs `ies` (heaviest first): the one with
-  // the shortest makespan when the envs are taken in order by the resident
-  // clusters (or single CTAs) and an env's substep costs kFixed plus its cost
-  // over the cluster's size.  Fitted to forward + reverse times per substep of
-  // 1-200 envs (quadruped, spider and random lattices, B200; one unit of cost
-  // is 0.105 ns, four in FP64): one CTA 20 / 44 / 88 / 195 us for robots of cost 47 k / 334 k
-  // / 601 k / 1.7 M, clusters of 8 17 / 25 / 34 / 51 us.  A cluster's share of
-  // an env costs 1.35 times its part: exchanges, and phases that every CTA
-  // repeats.  nullptr: one CTA per env.
-  const ClusterPlan* cluster_plan(const int* ies, int n) const {
+  // Which of the envs `ies` (heaviest first) of a launch run as one cluster each,
+  // and in clusters of which size: the choice with the shortest makespan when the
+  // envs are taken in order by the resident clusters or single CTAs and an env's
+  // substep costs kFixed plus its cost over the cluster's size.  Either every env
+  // runs as a cluster, or the heaviest do, all of them at once, and the others on
+  // single CTAs on the SMs that these leave free and, later, have left.
+  // Fitted to forward + reverse times per substep of 1-200 envs (quadruped, spider
+  // and random lattices, B200; one unit of cost is 0.105 ns, four in FP64): one CTA
+  // 20 / 44 / 88 / 195 us for robots of cost 47 k / 334 k / 601 k / 1.7 M, clusters
+  // of 8 17 / 25 / 34 / 51 us.  A cluster's share of an env costs 1.35 times its
+  // part: exchanges, and phases that every CTA repeats.  A split has to win by 7 %:
+  // with 300 random lattices of 50-2000 vertices, 40 substeps and their adjoint,
+  // 13.6 ms on single CTAs, 11.5 with the 16 heaviest on clusters of 4, 11.8 with 32
+  // on clusters of 2; with 512 such lattices 16.1 and 17.7, 18.8 (the weights'
+  // stream keeps every SM busy there: more than 3 envs per SM are not considered).
+  struct Split {
+    const ClusterPlan* plan = nullptr;
+    int heavy = 0;
+  };
+  Split split_envs(const int* ies, int n) const {
 #ifdef CLS_CLUSTER_SIZE
     for (const ClusterPlan& p : plans_)
-      if (p.size == CLS_CLUSTER_SIZE) return &p;
-    return nullptr;
+      if (p.size == CLS_CLUSTER_SIZE) return {&p, n};
+    return {};
 #endif
-    if (plans_.empty() || n > 2 * n_sm_) return nullptr;
-    std::vector<double> busy;
-    auto makespan = [&](double fixed, double per_cost, int slots) {
-      busy.assign((size_t)std::max(1, std::min(slots, n)), 0.0);
-      for (int k = 0; k < n; ++k)
-        *std::min_element(busy.begin(), busy.end()) += fixed + per_cost * cost_[ies[k]];
-      return *std::max_element(busy.begin(), busy.end());
+#ifdef CLS_SPLIT
+    for (const ClusterPlan& p : plans_)
+      if (p.size == 4) return {&p, std::min(n, CLS_SPLIT)};
+#endif
+    if (plans_.empty() || n > 3 * n_sm_) return {};
+    constexpr double kOne = 1.45e5, kCluster = 1.64e5, kShare = 1.35;
+    std::vector<double> free_at;  // heap, the next free worker first
+    // envs k0.. taken in order by the workers of free_at: when the last is done
+    auto last_done = [&](int k0, double fixed, double per_cost) {
+      double end = 0;
+      std::make_heap(free_at.begin(), free_at.end(), std::greater<double>());
+      for (int k = k0; k < n; ++k) {
+        std::pop_heap(free_at.begin(), free_at.end(), std::greater<double>());
+        free_at.back() += fixed + per_cost * cost_[ies[k]];
+        end = std::max(end, free_at.back());
+        std::push_heap(free_at.begin(), free_at.end(), std::greater<double>());
+      }
+      return end;
     };
-    const ClusterPlan* best = nullptr;
-    double t = makespan(1.45e5, 1.0, n_sm_);
+    Split best;
+    free_at.assign((size_t)n_sm_, 0.0);
+    const double single = last_done(0, kOne, 1.0);
+    double t = single;
     for (const ClusterPlan& p : plans_) {
-      const double tp = makespan(1.64e5, 1.35 / p.size, p.resident);
+      if (n > 2 * n_sm_) break;
+      free_at.assign((size_t)p.resident, 0.0);
+      const double tp = last_done(0, kCluster, kShare / p.size);
       if (tp < t) {
         t = tp;
-        best = &p;
+        best = {&p, n};
       }
     }
+    for (const ClusterPlan& p : plans_)
+      for (int q = 1; q <= 8; ++q) {
+        const int heavy = p.resident * q / 8;
+        if (heavy < 1 || heavy >= n || heavy * p.size > n_sm_) continue;
+        free_at.assign((size_t)(n_sm_ - heavy * p.size), 0.0);
+        double done = 0;
+        for (int k = 0; k < heavy; ++k) {
+          const double tk = kCluster + kShare / p.size * cost_[ies[k]];
+          free_at.insert(free_at.end(), p.size, tk);
+          done = std::max(done, tk);
+        }
+        done = std::max(done, last_done(heavy, kOne, 1.0));
+        if (done < t && done < 0.93 * single) {
+          t = done;
+          best = {&p, heavy};
+        }
+      }
     return best;
   }
 
@@ -843,20 +885,52 @@ class SimImpl final : public SimBase {
     CLS_CUDA(cudaLaunchKernelEx(&c, ms_wgrad_kernel<R>, a, tiles, kseg, d_gw_.p, d_gb_.p));
   }
 
-  // forward / reverse launches of the fused path over a.n_items envs: one
-  // cluster each with a plan, else one CTA each from the work queue
-  void launch_fwd(const MsArgs<R>& a, const ClusterPlan* p, int grid, int t0, int t1, int mode, int src) {
-    if (p) CLS_CUDA(ClusterLaunch<R>::forward(a, p->cap, p->size, threads_, p->fwd_smem, stream, t0, t1, mode, src));
-    else fwd_fn()<<<grid, threads_, fwd_smem_, stream>>>(a, t0, t1, mode, src);
+  // forward / reverse launches of the fused path over a.n_items envs: the heaviest
+  // ones of a split as one cluster each, the others one CTA each from the work
+  // queue.  The second launch is a programmatic dependent of the first, which
+  // releases it at its start: both run at once, on one stream, and the second ends
+  // last (ms_forward_kernel, ms_reverse_kernel).
+  void launch_fwd(const MsArgs<R>& a, const Split& sp, int grid, int t0, int t1, int mode, int src) {
+    launch_split(a, sp, grid, [&](const MsArgs<R>& h) {
+      const ClusterPlan* p = sp.plan;
+      return ClusterLaunch<R>::forward(h, p->cap, p->size, threads_, p->fwd_smem, stream, t0, t1, mode, src);
+    }, [&](const cudaLaunchConfig_t& c, const MsArgs<R>& l) {
+      return cudaLaunchKernelEx(&c, fwd_fn(), l, t0, t1, mode, src);
+    }, fwd_smem_);
   }
-  void launch_rev(const MsArgs<R>& a, const ClusterPlan* p, int grid, int t0, int t1, int last) {
-    if (p) CLS_CUDA(ClusterLaunch<R>::reverse(a, p->cap, p->size, threads_, p->rev_smem, stream, t0, t1, last));
-    else rev_fn()<<<grid, threads_, rev_smem_, stream>>>(a, t0, t1, last);
+  void launch_rev(const MsArgs<R>& a, const Split& sp, int grid, int t0, int t1, int last) {
+    launch_split(a, sp, grid, [&](const MsArgs<R>& h) {
+      const ClusterPlan* p = sp.plan;
+      return ClusterLaunch<R>::reverse(h, p->cap, p->size, threads_, p->rev_smem, stream, t0, t1, last);
+    }, [&](const cudaLaunchConfig_t& c, const MsArgs<R>& l) {
+      return cudaLaunchKernelEx(&c, rev_fn(), l, t0, t1, last);
+    }, rev_smem_);
+  }
+  template <typename Heavy, typename Light>
+  void launch_split(const MsArgs<R>& a, const Split& sp, int grid, Heavy heavy, Light light, size_t smem) {
+    const int nh = sp.plan ? std::min(sp.heavy, a.n_items) : 0;
+    MsArgs<R> part = a;
+    if (nh) {
+      part.n_items = nh;
+      CLS_CUDA(heavy(part));
+    }
+    if (nh == a.n_items) return;
+    part.order = a.order + nh;
+    part.n_items = a.n_items - nh;
+    cudaLaunchConfig_t c{};
+    cudaLaunchAttribute at{};
+    c.gridDim = dim3((unsigned)std::min(grid, part.n_items));
+    c.blockDim = dim3((unsigned)threads_);
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = nh ? 1 : 0;
+    CLS_CUDA(light(c, part));
   }
   // of the whole batch (per-env launches keep the single-CTA kernels)
-  const ClusterPlan* batch_plan(bool per_env) const {
-    return per_env || batch_plan_ < 0 ? nullptr : &plans_[batch_plan_];
-  }
+  Split batch_split(bool per_env) const { return per_env ? Split{} : batch_split_; }
 
   // Per-spring tables in shared memory (forward impulses, reverse adjoint
   // terms): -1 when the largest robot's impulse table fits kImpSmemMax (the
@@ -1214,9 +1288,9 @@ class SimImpl final : public SimBase {
     if (dense_ && !per_env) {
       dense_pass(a, 0, t_end, mode, 0, true, PK_FWD);
     } else {
-      const ClusterPlan* plan = batch_plan(per_env);
+      const Split split = batch_split(per_env);
       each_launch(per_env, a, qslot_, [&](const MsArgs<R>& b, int grid) {
-        timed(PK_FWD, [&] { launch_fwd(b, plan, grid, 0, t_end, mode, 0); });
+        timed(PK_FWD, [&] { launch_fwd(b, split, grid, 0, t_end, mode, 0); });
       });
     }
     CLS_CUDA(cudaGetLastError());
@@ -1538,13 +1612,13 @@ class SimImpl final : public SimBase {
         // the first pass recorded every substep's controller in this layout:
         // replay its outputs
         const int rmode = FWD_RECORD | (tail && episode ? FWD_REPLAY : 0);
-        const ClusterPlan* plan = batch_plan(per_env);
+        const Split split = batch_split(per_env);
         if (recompute)
           each_launch(per_env, a, qslot, [&](const MsArgs<R>& b, int grid) {
-            timed(PK_RECOMP, [&] { launch_fwd(b, plan, grid, t0, t1, rmode, s); });
+            timed(PK_RECOMP, [&] { launch_fwd(b, split, grid, t0, t1, rmode, s); });
           });
         each_launch(per_env, a, qslot, [&](const MsArgs<R>& b, int grid) {
-          timed(PK_REV, [&] { launch_rev(b, plan, grid, t0, t1, s == n_seg - 1 ? 1 : 0); });
+          timed(PK_REV, [&] { launch_rev(b, split, grid, t0, t1, s == n_seg - 1 ? 1 : 0); });
         });
       }
       if (episode) continue;
@@ -2147,8 +2221,8 @@ class SimImpl final : public SimBase {
     CLS_CUDA(cudaMemsetAsync(d_squeue_.p, 0, sizeof(int) * 2, stream));
     MsArgs<R> a = serve_args(n);
     a.queue = d_squeue_.p;
-    const ClusterPlan* plan = cluster_plan(serve_order_h_.data(), n);
-    timed(PK_FWD, [&] { launch_fwd(a, plan, grid_for(n), 0, 0, FWD_CKPT | FWD_OBS | FWD_CKEND, 0); });
+    const Split split = split_envs(serve_order_h_.data(), n);
+    timed(PK_FWD, [&] { launch_fwd(a, split, grid_for(n), 0, 0, FWD_CKPT | FWD_OBS | FWD_CKEND, 0); });
     CLS_CUDA(cudaGetLastError());
   }
 
@@ -2176,10 +2250,10 @@ class SimImpl final : public SimBase {
     CLS_CUDA(cudaMemsetAsync(d_squeue_.p, 0, sizeof(int) * 2, stream));
     MsArgs<R> a = serve_args(n);
     a.queue = d_squeue_.p;
-    const ClusterPlan* plan = cluster_plan(serve_order_h_.data(), n);
-    timed(PK_RECOMP, [&] { launch_fwd(a, plan, grid_for(n), 0, 0, FWD_RECORD, 0); });
+    const Split split = split_envs(serve_order_h_.data(), n);
+    timed(PK_RECOMP, [&] { launch_fwd(a, split, grid_for(n), 0, 0, FWD_RECORD, 0); });
     a.queue = d_squeue_.p + 1;
-    timed(PK_REV, [&] { launch_rev(a, plan, grid_for(n), 0, 0, 0); });
+    timed(PK_REV, [&] { launch_rev(a, split, grid_for(n), 0, 0, 0); });
     if (!tiles.empty()) {
       unsigned char *h, *d;
       int slot;
@@ -2378,7 +2452,7 @@ class SimImpl final : public SimBase {
   std::vector<double> cost_;       // per env: cost of a substep (processing order, cluster sizes)
   std::vector<int> inc_ptr_h_;     // incidence row starts of the robot types
   std::vector<ClusterPlan> plans_;
-  int batch_plan_ = -1;            // plans_ index for launches over the whole batch
+  Split batch_split_;              // for launches over the whole batch
   std::vector<int> perm_, user_voff_, env_robot_, order_host_;
   bool identity_perm_ = true;
   std::vector<EnvDesc> ed_host_;

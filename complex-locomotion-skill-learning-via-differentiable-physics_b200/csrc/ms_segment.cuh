@@ -465,6 +465,8 @@ ms_forward_kernel(MsArgs<R> a, int t_begin0, int t_end0, int mode, int src_slot0
     }
     fwd_finish<R>(a, rb, ed, s, t_begin, t_end, mode);
   }
+  // a cluster launch beside this one (launch_fwd) ends before this launch does
+  dependents_wait();
 }
 
 // -------------------------------------------------------------- loss seeds
@@ -1086,6 +1088,7 @@ ms_reverse_kernel(MsArgs<R> a, int t_begin0, int t_end0, int last_seg0) {
     }
     rev_store_carry<R>(a, rb, ed, s, e, hcarry);
   }
+  dependents_wait();  // as in the forward kernel
 }
 
 // ------------------------------------------------------------------ losses

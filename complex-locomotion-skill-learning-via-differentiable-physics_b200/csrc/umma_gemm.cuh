@@ -131,12 +131,6 @@ __device__ __forceinline__ void tmem_relinquish() {
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 
-// Programmatic dependent launch: lets the next launch of the stream start its
-// prologue, and waits until the launches before this one have finished (no effect
-// in launches without the attribute).
-__device__ __forceinline__ void dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void dependents_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // 32 lanes x 8 consecutive 32-bit columns
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float v[8]) {
   uint32_t r[8];

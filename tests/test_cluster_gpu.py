@@ -83,3 +83,57 @@ def test_cluster_equals_single_cta(case, precision):
     for g, r in zip(got[3] + list(got[4]), ref[3] + list(ref[4])):
         assert np.isfinite(g).all()
         assert _rel(g, r) < tol
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("graph", [False, True])
+def test_heaviest_on_clusters_beside_single_ctas(graph, precision):
+    """Few heavy envs among many light ones: the heavy ones run as clusters in a
+    launch beside that of the others.  Same bars as above; a captured step replays
+    the same two launches."""
+    import cls_b200
+    from cls_b200 import workloads
+    from cls_b200.batch import MassSpringBatch
+    import torch
+    steps, K = 15, 6
+    robots = [_lattice(n, (32, 16), seed=n) for n in (700, 30)]
+    p = cls_b200.default_params(**workloads._params(steps, K, precision=precision, run_period=5, turn_period=30,
+                                                    jump_period=4, loss=("velocity", "rotation", "height")))
+    b = MassSpringBatch(robots, [0] * 4 + [1] * 196, p)
+    rng = np.random.default_rng(5)
+    try:
+        b.set_controller_path("per_env")
+        b.weights_init(3)
+        b.set_spring_tables(0)
+        tv, th = workloads.targets(rng, b.T, b.n_envs)
+        b.set_targets(tv, th + 0.15, np.zeros((b.T, b.n_envs)))
+        x0 = np.concatenate([robots[0].objects] * 4 + [robots[1].objects] * 196)
+        x0[:, 1] -= 0.09
+        b.set_state(x0 + rng.uniform(-2e-3, 2e-3, x0.shape), rng.uniform(-0.1, 0.1, x0.shape))
+
+        def read():
+            return b.final_state(), [a for r in (0, 1) for l in range(b.n_layers(r)) for a in b.get_grads(r, l)]
+
+        def run(per_env):
+            b.simulate(steps, per_env=per_env)
+            b.loss()
+            return read()
+        ref = run(True)
+        if graph:
+            s = torch.cuda.Stream()
+            b.set_stream(s.cuda_stream)
+            b.graph_capture(steps, False)
+            for _ in range(2):
+                b.graph_launch(0)
+            torch.cuda.synchronize()
+            got = read()
+        else:
+            got = run(False)
+    finally:
+        b.close()
+    for g, r in zip(got[0], ref[0]):
+        assert np.array_equal(g, r)
+    tol = 1e-8 if precision == 64 else 1e-4
+    for g, r in zip(got[1], ref[1]):
+        assert np.isfinite(g).all()
+        assert _rel(g, r) < tol
