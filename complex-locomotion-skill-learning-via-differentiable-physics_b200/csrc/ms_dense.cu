@@ -36,6 +36,11 @@ int DenseLaunch<R>::tile_m() { return std::is_same<R, float>::value ? umma::TM :
 template <typename R>
 int DenseLaunch<R>::tile_n() { return std::is_same<R, float>::value ? kDenseTN : kSimtTile; }
 template <typename R>
+int DenseLaunch<R>::job_n(int n_tiles, int n_sm) {
+  if (!std::is_same<R, float>::value) return kSimtTile;
+  return 2 * n_tiles <= n_sm ? kDenseTNSmall : kDenseTN;
+}
+template <typename R>
 long long DenseLaunch<R>::split_floats(int rows, int tile_rows, int k) {
   return (long long)umma::split_tiles_floats(rows, tile_rows, k);
 }
@@ -57,8 +62,9 @@ cudaError_t DenseLaunch<R>::setup(size_t* fwd_static, size_t* rev_static, int op
   prepare(ms_step_rev_kernel<R, kStepThreads, true>, rev_static);
   if constexpr (std::is_same<R, float>::value) {
     const int sm = (int)umma::BulkShape<kDenseTN, kBulkStages>::kSmemBytes;
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(ms_ctrl_gemm_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(ms_ctrl_gemm_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    for (auto fn : {ms_ctrl_gemm_tc_kernel<0, kDenseTN>, ms_ctrl_gemm_tc_kernel<1, kDenseTN>,
+                    ms_ctrl_gemm_tc_kernel<0, kDenseTNSmall>, ms_ctrl_gemm_tc_kernel<1, kDenseTNSmall>})
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(ms_wgrad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
   }
   return e;
@@ -79,12 +85,14 @@ cudaError_t DenseLaunch<R>::step_rev(const MsArgs<R>& a, int grid, int threads, 
 }
 
 template <typename R>
-cudaError_t DenseLaunch<R>::gemm(const MsArgs<R>& a, bool adjoint, int n_jobs, const DenseJob* jobs, const TcJob* tc,
-                                 int kslot, cudaStream_t s) {
+cudaError_t DenseLaunch<R>::gemm(const MsArgs<R>& a, bool adjoint, int n_jobs, int job_cols, const DenseJob* jobs,
+                                 const TcJob* tc, int kslot, cudaStream_t s) {
   if constexpr (std::is_same<R, float>::value) {
-    const size_t sm = umma::BulkShape<kDenseTN, kBulkStages>::kSmemBytes;
-    return chain(adjoint ? ms_ctrl_gemm_tc_kernel<1> : ms_ctrl_gemm_tc_kernel<0>, n_jobs, umma::kBulkThreads, sm, s, a,
-                 tc, kslot);
+    if (job_cols == kDenseTNSmall)
+      return chain(adjoint ? ms_ctrl_gemm_tc_kernel<1, kDenseTNSmall> : ms_ctrl_gemm_tc_kernel<0, kDenseTNSmall>, n_jobs,
+                   umma::kBulkThreads, umma::BulkShape<kDenseTNSmall, kBulkStages>::kSmemBytes, s, a, tc, kslot);
+    return chain(adjoint ? ms_ctrl_gemm_tc_kernel<1, kDenseTN> : ms_ctrl_gemm_tc_kernel<0, kDenseTN>, n_jobs,
+                 umma::kBulkThreads, umma::BulkShape<kDenseTN, kBulkStages>::kSmemBytes, s, a, tc, kslot);
   } else {
     return chain(adjoint ? ms_ctrl_gemm_simt_kernel<R, 1> : ms_ctrl_gemm_simt_kernel<R, 0>, n_jobs, 256, 0, s, a, jobs,
                  kslot);

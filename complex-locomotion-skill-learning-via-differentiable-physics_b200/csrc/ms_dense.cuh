@@ -318,7 +318,8 @@ __device__ __forceinline__ BwdOperands<R> bwd_operands(const MsArgs<R>& a, const
 #ifndef CLS_BULK_STAGES
 #define CLS_BULK_STAGES 4
 #endif
-constexpr int kDenseTN = CLS_DENSE_TN;        // output columns per tensor-core tile
+constexpr int kDenseTN = CLS_DENSE_TN;        // output columns per tensor-core tile, and rows of a B operand block
+constexpr int kDenseTNSmall = 32;             // of launches whose tiles would leave SMs idle (DenseLaunch::job_n)
 constexpr int kBulkStages = CLS_BULK_STAGES;  // stages of the bulk-copy ring (4 x 48 KB at TN = 64)
 
 __device__ __forceinline__ float4 mask4(float4 v, int col, int n) {
@@ -329,7 +330,7 @@ __device__ __forceinline__ float4 mask4(float4 v, int col, int n) {
   return v;
 }
 
-template <int BWD>
+template <int BWD, int TN>
 __global__ void __launch_bounds__(umma::kBulkThreads)
 ms_ctrl_gemm_tc_kernel(MsArgs<float> a, const TcJob* jobs, int kslot) {
   extern __shared__ __align__(1024) float smem_f[];
@@ -340,9 +341,9 @@ ms_ctrl_gemm_tc_kernel(MsArgs<float> a, const TcJob* jobs, int kslot) {
   const int zl = jb.z_layer < 0 ? 0 : jb.z_layer;
   const size_t z0 = a.z_base[zl] + (size_t)kslot * a.z_total[zl] + jb.z_off;
   const umma::SplitTiles st{a.tiles + (jb.split < 0 ? 0 : jb.split), umma::TM, (w + 31) / 32};
-  const bool ok = umma::tile_gemm_bulk<kDenseTN, kBulkStages>(
+  const bool ok = umma::tile_gemm_bulk<TN, kBulkStages, kDenseTN>(
       smem_f, bs, a.tiles + jb.a, a.tiles + jb.b, jb.nkt, [&](const float* cs, int ld) {
-        constexpr int C4 = kDenseTN / 4;
+        constexpr int C4 = TN / 4;
         for (int q = threadIdx.x; q < umma::TM * C4; q += blockDim.x) {
           const int i = q / C4, j = 4 * (q % C4);
           if (i >= jb.m_valid || j >= jb.n_valid) continue;
@@ -469,7 +470,7 @@ ms_wgrad_tc_kernel(MsArgs<float> a, const WgJob* jobs, int nslots, float* gw, fl
   const int nout = rb.width[l + 1], nin = rb.width[l], pitch = rb.pitch[l];
   float* W = gw + rb.w_off[l];
   float* B = gb + rb.b_off[l];
-  const bool ok = umma::tile_gemm_bulk<kDenseTN, kBulkStages>(
+  const bool ok = umma::tile_gemm_bulk<kDenseTN, kBulkStages, kDenseTN>(
       smem_f, bs, ab, bb, k1 - k0, [&](const float* cs, int ld) {
         for (int q = threadIdx.x; q < umma::TM * kDenseTN; q += blockDim.x) {
           const int i = q / kDenseTN, j = q % kDenseTN;

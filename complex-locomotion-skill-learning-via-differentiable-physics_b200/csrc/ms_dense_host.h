@@ -16,9 +16,15 @@ constexpr int kStepThreads = 256;
 
 template <typename R>
 struct DenseLaunch {
-  // GEMM tile of one job (envs x outputs): tensor-core tile for FP32, SIMT for FP64
+  // GEMM tile of one job (envs x outputs): tensor-core tile for FP32, SIMT for
+  // FP64.  tile_n: the rows of an operand block; job_n: the columns of one job,
+  // half as many when the layer's tiles (n_tiles of them) leave half the SMs idle:
+  // the K loop is bound by one SM's rate over the tile, so twice the SMs shorten it
+  // (64 / 32 columns, us per substep and its adjoint in a graph of spiders: 102.0 / 98.4
+  // at 256 envs, 111.1 / 103.1 at 512, 151.0 / 144.0 at 1024, 242.3 / 237.9 at 2048)
   static int tile_m();
   static int tile_n();
+  static int job_n(int n_tiles, int n_sm);
   // floats of a pre-split operand (rows x k) in tiles of tile_rows rows (FP32)
   static long long split_floats(int rows, int tile_rows, int k);
   // shared-memory attributes of the step and GEMM kernels; the step kernels'
@@ -29,7 +35,7 @@ struct DenseLaunch {
   static cudaError_t step_rev(const MsArgs<R>& a, int grid, int threads, size_t smem, cudaStream_t s, int t_post,
                        int t_pre, int t_begin, int t_end, int last_seg);
   // (FP32 takes the same tiles from `tc`)
-  static cudaError_t gemm(const MsArgs<R>& a, bool adjoint, int n_jobs, const DenseJob* jobs,
+  static cudaError_t gemm(const MsArgs<R>& a, bool adjoint, int n_jobs, int job_cols, const DenseJob* jobs,
                           const TcJob* tc, int kslot, cudaStream_t s);
   // FP32 weight-gradient products of record slots [slot0, slot0 + nslots):
   // record transposes (grid grid_x x n_cols x slot groups) then the tensor-core

@@ -1323,25 +1323,24 @@ class SimImpl final : public SimBase {
     constexpr bool f32 = std::is_same<R, float>::value;
     const int tm = DenseLaunch<R>::tile_m(), tn = DenseLaunch<R>::tile_n();
     jobs_h_.clear();
-    for (int l = 0; l < L_; ++l) {
-      jf_off_[l] = (int)jobs_h_.size();
+    // a layer's tiles, all types: `off`, `cnt` and the columns of each (`jn`)
+    auto add_layer = [&](int l, bool adj, int* off, int* cnt, int* jn) {
+      auto cols = [&](const HostRobot& h) { return !adj ? h.width[l + 1] : (l > 0 ? h.width[l] : 3 * h.n_v); };
+      int n_tiles = 0;
+      for (int r = 0; r < (int)hr_.size(); ++r)
+        if (rd_host_[r].n_env > 0 && l < hr_[r].n_layers)
+          n_tiles += ((rd_host_[r].n_env + tm - 1) / tm) * ((cols(hr_[r]) + tn - 1) / tn);
+      *jn = DenseLaunch<R>::job_n(n_tiles, n_sm_);
+      *off = (int)jobs_h_.size();
       for (int r = 0; r < (int)hr_.size(); ++r) {
         if (rd_host_[r].n_env == 0 || l >= hr_[r].n_layers) continue;
         for (int m0 = 0; m0 < rd_host_[r].n_env; m0 += tm)
-          for (int n0 = 0; n0 < hr_[r].width[l + 1]; n0 += tn) jobs_h_.push_back({r, l, m0, n0});
+          for (int n0 = 0; n0 < cols(hr_[r]); n0 += *jn) jobs_h_.push_back({r, l, m0, n0});
       }
-      jf_cnt_[l] = (int)jobs_h_.size() - jf_off_[l];
-    }
-    for (int l = 0; l < L_; ++l) {
-      jb_off_[l] = (int)jobs_h_.size();
-      for (int r = 0; r < (int)hr_.size(); ++r) {
-        if (rd_host_[r].n_env == 0 || l >= hr_[r].n_layers) continue;
-        const int ncol = l > 0 ? hr_[r].width[l] : 3 * hr_[r].n_v;
-        for (int m0 = 0; m0 < rd_host_[r].n_env; m0 += tm)
-          for (int n0 = 0; n0 < ncol; n0 += tn) jobs_h_.push_back({r, l, m0, n0});
-      }
-      jb_cnt_[l] = (int)jobs_h_.size() - jb_off_[l];
-    }
+      *cnt = (int)jobs_h_.size() - *off;
+    };
+    for (int l = 0; l < L_; ++l) add_layer(l, false, &jf_off_[l], &jf_cnt_[l], &jf_n_[l]);
+    for (int l = 0; l < L_; ++l) add_layer(l, true, &jb_off_[l], &jb_cnt_[l], &jb_n_[l]);
     d_jobs_.alloc(std::max<size_t>(1, jobs_h_.size()));
     CLS_CUDA(cudaMemcpy(d_jobs_.p, jobs_h_.data(), sizeof(DenseJob) * jobs_h_.size(), cudaMemcpyHostToDevice));
     d_tsegs_.alloc(std::max<size_t>(1, tsegs_.size()));
@@ -1445,11 +1444,11 @@ class SimImpl final : public SimBase {
         TcJob t{};
         t.nkt = (kin + 31) / 32;
         t.a = (adj ? dd.ta_b[l] : dd.ta_f[l]) + (long long)(jb.m0 / tm) * t.nkt * 64 * tm;
-        t.b = (adj ? dd.tb_b[l] : dd.tb_f[l]) + (long long)(jb.n0 / tn) * t.nkt * 64 * tn;
+        t.b = (adj ? dd.tb_b[l] : dd.tb_f[l]) + (long long)(jb.n0 / tn) * t.nkt * 64 * tn + jb.n0 % tn * 32;
         t.m0 = jb.m0;
         t.n0 = jb.n0;
         t.m_valid = std::min(tm, d.n_env - jb.m0);
-        t.n_valid = std::min(tn, ncol - jb.n0);
+        t.n_valid = std::min(adj ? jb_n_[l] : jf_n_[l], ncol - jb.n0);
         t.w = ncol;
         t.z_layer = adj ? l - 1 : l;
         t.z_off = t.z_layer >= 0 ? e0.z_off[t.z_layer] : 0;
@@ -1501,7 +1500,9 @@ class SimImpl final : public SimBase {
     const int at = bwd ? jb_off_[l] : jf_off_[l];
     const DenseJob* jobs = d_jobs_.p + at;
     const TcJob* tc = d_tcjobs_.p ? d_tcjobs_.p + at : nullptr;
-    timed(bwd ? PK_CGEMM_ADJ : PK_CGEMM, [&] { CLS_CUDA(DenseLaunch<R>::gemm(a, bwd, cnt, jobs, tc, kslot, stream)); });
+    timed(bwd ? PK_CGEMM_ADJ : PK_CGEMM, [&] {
+      CLS_CUDA(DenseLaunch<R>::gemm(a, bwd, cnt, bwd ? jb_n_[l] : jf_n_[l], jobs, tc, kslot, stream));
+    });
   }
 
   // forward over [t_first, t_end): a step launch per substep boundary and the
@@ -2505,6 +2506,7 @@ class SimImpl final : public SimBase {
   std::vector<TransSeg> tsegs_;
   std::vector<DenseJob> jobs_h_;
   int jf_off_[kMaxLayers] = {0}, jf_cnt_[kMaxLayers] = {0}, jb_off_[kMaxLayers] = {0}, jb_cnt_[kMaxLayers] = {0};
+  int jf_n_[kMaxLayers] = {0}, jb_n_[kMaxLayers] = {0};  // columns of a layer's tiles
   DevBuf<DenseJob> d_jobs_;
   DevBuf<TcJob> d_tcjobs_;
   DevBuf<TransSeg> d_tsegs_;

@@ -250,15 +250,16 @@ struct BulkShared {
 };
 
 // One 128 x TN tile, C(i, j) = sum_k A(i, k) B(j, k) over the whole K range:
-// `a_blocks` / `b_blocks` point at block (rt, 0) / (nt, 0) of SplitTiles
-// operands with nkt K-blocks each (tile heights 128 / TN).  Thread 0 fills an
-// S-stage ring with bulk copies, thread 32 issues the MMAs (3 per K-step of
-// 8: lo*hi, hi*lo, hi*hi) and commits each stage back to the producer.  The
-// accumulator is then staged through the (idle) ring as a row-major
+// `a_blocks` points at block (rt, 0), `b_blocks` at row n0 mod BR of block (nt, 0),
+// of SplitTiles operands with nkt K-blocks each (tile heights 128 / BR; a tile of
+// fewer than BR columns takes its part of B's rows with one copy per precision
+// part).  Thread 0 fills an S-stage ring with bulk copies, thread 32 issues the
+// MMAs (3 per K-step of 8: lo*hi, hi*lo, hi*hi) and commits each stage back to the
+// producer.  The accumulator is then staged through the (idle) ring as a row-major
 // 128 x TN tile, C(i, j) at cs[i * ld + j], and epi(cs, ld) writes it out
 // with every thread of the CTA (so its global stores can run along rows).
 // kBulkThreads threads.  Returns false on a timeout (epi is not called then).
-template <int TN, int S, typename Epi>
+template <int TN, int S, int BR, typename Epi>
 __device__ bool tile_gemm_bulk(float* smem, BulkShared& bs, const float* a_blocks, const float* b_blocks,
                                int nkt, Epi epi, WaitPolicy wp = WaitPolicy{0u, 0}) {
   using Sh = BulkShape<TN, S>;
@@ -290,7 +291,13 @@ __device__ bool tile_gemm_bulk(float* smem, BulkShared& bs, const float* a_block
       const uint32_t st = ring + (uint32_t)s * Sh::kStageBytes;
       mbar_arrive_expect_tx(full0 + 8 * s, Sh::kStageBytes);
       bulk_g2s(st, a_blocks + (size_t)kt * (2 * TK * TM), Sh::kABytes, full0 + 8 * s);
-      bulk_g2s(st + Sh::kABytes, b_blocks + (size_t)kt * (2 * TK * TN), Sh::kBBytes, full0 + 8 * s);
+      const float* b = b_blocks + (size_t)kt * (2 * TK * BR);
+      if constexpr (TN == BR) {
+        bulk_g2s(st + Sh::kABytes, b, Sh::kBBytes, full0 + 8 * s);
+      } else {
+        bulk_g2s(st + Sh::kABytes, b, Sh::kBBytes / 2, full0 + 8 * s);
+        bulk_g2s(st + Sh::kABytes + Sh::kBBytes / 2, b + TK * BR, Sh::kBBytes / 2, full0 + 8 * s);
+      }
     }
   } else if (tid == 32) {
     // MMA issuer

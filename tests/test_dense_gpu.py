@@ -193,3 +193,22 @@ def test_batched_profile_counts_gemm_launches():
     assert n["ctrl_gemm"] == 2 * 19 * 3
     assert n["ctrl_gemm_adj"] == 19 * 3
     assert ms["ctrl_gemm"] > 0 and ms["ctrl_gemm_adj"] > 0
+
+
+@pytest.mark.parametrize("width", [500, 600])
+def test_batched_tile_widths_match_per_env(width):
+    """1030 envs (nine row tiles, the last of 6 rows): a layer of 500 outputs has
+    72 tiles of 64 columns, which leave half the SMs idle, and takes tiles of 32; one
+    of 600 has 90 and keeps 64.  The suite's FP32 bars."""
+    steps = 12
+    runs = []
+    for path in ("per_env", "batched"):
+        b = many_env_batch(32, 1030, [width], 9, 20, path)
+        runs.append(_run(b, steps, 2))
+        b.close()
+    ref, got = runs
+    assert abs(got[0] - ref[0]) <= TOL[32]["loss"] * abs(ref[0])
+    assert max_rel(got[2], ref[2]) < TOL[32]["traj"]
+    for (gW, gb), (rW, rb) in zip(got[1], ref[1]):
+        assert rel_err(gW, rW) < TOL[32]["grad"] and rel_err(gb, rb) < TOL[32]["grad"]
+    assert rel_err(got[3], ref[3]) < TOL[32]["grad"]
