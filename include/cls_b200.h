@@ -281,9 +281,12 @@ int cls_controller_batched(const cls_sim* sim, int32_t* on);
  * weights and biases into shared memory once per work item (the robot's
  * controller must fit beside the kernels' own shared memory), 0 reads them
  * from global memory every substep, -1 (the default at creation) chooses 1
- * when it fits without fewer resident CTAs.  Results do not depend on
- * ctas_per_sm or weights_shared, and depend on threads_per_block only through
- * the rounding of block-wide reductions.  No reference counterpart: Taichi
+ * when it fits without fewer resident CTAs.  With up to 512 threads, a launch of
+ * few envs, or the heaviest envs of an uneven one, runs each such env on a
+ * thread-block cluster of 2, 4 or 8 CTAs of that size where that is estimated to
+ * end earlier; those read the controller from global memory.  Results do not depend on
+ * ctas_per_sm or weights_shared, and depend on threads_per_block (and on the
+ * use of clusters: gradients) only through the rounding of reductions.  No reference counterpart: Taichi
  * chose its own block sizes per kernel (ti.loop_config).  A CUDA graph
  * captured earlier keeps the shape it was captured with.  CLS_ERR_INVALID
  * when a robot's shared memory does not fit the instance or no CTA of that
@@ -294,11 +297,12 @@ int cls_set_launch_shape(cls_sim* sim, int32_t threads_per_block, int32_t ctas_p
 int cls_get_launch_shape(const cls_sim* sim, int32_t* threads_per_block, int32_t* ctas_per_sm,
                          int32_t* weights_shared);
 
-/* Per-spring tables of the fused and step kernels: each spring's impulse
- * (forward) and adjoint terms (fused reverse) evaluated once into shared
- * memory and gathered per vertex, instead of evaluated from both of its
- * endpoints.  mode -1 (the default at creation): on when the largest robot's
- * table fits (<= 3072 springs in FP32); 0 off; 1 on (CLS_ERR_INVALID when it
+/* Per-spring tables of the fused single-CTA kernels and, in FP32, the batched
+ * step kernels: each spring's impulse (forward) and adjoint terms (reverse)
+ * evaluated once into shared memory and summed by a thread per vertex, instead of
+ * evaluated from both of its endpoints.  mode -1 (the default at creation): on
+ * when the largest robot's table fits (<= 3072 springs in FP32) and no vertex has
+ * more springs than 48 rows of the padded lists take; 0 off; 1 on (CLS_ERR_INVALID when it
  * does not fit).  The same results (each spring is evaluated in the same
  * argument order either way and gathered in the same order).  No reference
  * counterpart. */
@@ -550,11 +554,13 @@ int cls_mpm_profile_read(cls_mpm* sim, double* ms, int64_t* launches, int32_t re
  * Runs n_substeps of spring forces (atomic scatter into a velocity increment)
  * followed by the damped, ground-contact advance, in place on the caller's x
  * and v.  All pointers are device pointers owned by the caller; the call
- * allocates nothing (no cudaMalloc, no library allocator) and keeps its only
+ * allocates nothing (no cudaMalloc, no library allocator).  An env whose springs
+ * fit one CTA's shared memory (about 5000) runs all substeps there, one launch for
+ * the call; larger ones keep their only
  * scratch -- the velocity increment, n_envs * n_vertices * 3 floats -- in a
  * fixed 2^21-float (8 MiB) array inside the library that every GPU loading the
- * library holds until exit.  Larger problems are rejected with
- * CLS_ERR_INVALID and a message.  All calls share that array: calls that
+ * library holds until exit.  Problems larger than that array are rejected in
+ * either form with CLS_ERR_INVALID and a message.  Calls that use the array and
  * overlap on the GPU race and must be serialised by the caller.  Each call
  * clears the part it uses first.  The array's device address belongs to a CUDA
  * context: the first call in each context (a device's primary context, or one
