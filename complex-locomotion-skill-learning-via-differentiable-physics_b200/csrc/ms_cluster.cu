@@ -49,6 +49,11 @@ cudaError_t ClusterLaunch<R>::setup(int optin, size_t* fwd_max, size_t* rev_max)
   e = cudaFuncSetAttribute(ms_cluster_forward_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*fwd_max);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(ms_cluster_reverse_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*rev_max);
+  // clusters of 16 (8 is the portable maximum)
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(ms_cluster_forward_kernel<R>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(ms_cluster_reverse_kernel<R>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   return e;
 }
 

@@ -738,8 +738,8 @@ class SimImpl final : public SimBase {
     }
   }
 
-  // Shared-memory plans of the cluster-per-env kernels for clusters of 2, 4 and
-  // 8 CTAs of the current block size (invalid where a robot's share does not
+  // Shared-memory plans of the cluster-per-env kernels for clusters of 2, 4, 8 and
+  // 16 CTAs of the current block size (invalid where a robot's share does not
   // fit), and how many clusters can be resident.
   struct ClusterPlan {
     int size = 0, resident = 0;
@@ -752,7 +752,7 @@ class SimImpl final : public SimBase {
     if (threads_ > ClusterLaunch<R>::max_threads()) return;
     size_t fwd_max = 0, rev_max = 0;
     CLS_CUDA(ClusterLaunch<R>::setup(optin, &fwd_max, &rev_max));
-    for (int C : {2, 4, 8}) {
+    for (int C : {2, 4, 8, 16}) {
       ClusterPlan p;
       p.size = C;
       ClusterCaps& c = p.cap;
@@ -780,7 +780,12 @@ class SimImpl final : public SimBase {
         c.inc = 0;  // incidence records from global memory
         if (!sizes()) continue;
       }
-      CLS_CUDA(ClusterLaunch<R>::resident(C, threads_, p.fwd_smem, p.rev_smem, &p.resident));
+      const cudaError_t e = ClusterLaunch<R>::resident(C, threads_, p.fwd_smem, p.rev_smem, &p.resident);
+      if (e != cudaSuccess && C > 8) {  // beyond the portable size: only where the device takes it
+        cudaGetLastError();
+        continue;
+      }
+      CLS_CUDA(e);
       if (p.resident > 0) plans_.push_back(p);
     }
     batch_split_ = split_envs(order_host_.data(), E_);
@@ -796,7 +801,10 @@ class SimImpl final : public SimBase {
   // and random lattices, B200; one unit of cost is 0.105 ns, four in FP64): one CTA
   // 20 / 44 / 88 / 195 us for robots of cost 47 k / 334 k / 601 k / 1.7 M, clusters
   // of 8 17 / 25 / 34 / 51 us.  A cluster's share of an env costs 1.35 times its
-  // part: exchanges, and phases that every CTA repeats.  A split has to win by 7 %:
+  // part: exchanges, and phases that every CTA repeats.  Clusters of 16 pay more
+  // for each exchange and win on large robots only (of 8 / of 16, us per substep
+  // and its adjoint: 93 vertices 16.1 / 16.4, 200 24.6 / 25.0, 700 34.2 / 31.0,
+  // 2000 64.3 / 48.3).  A split has to win by 7 %:
   // with 300 random lattices of 50-2000 vertices, 40 substeps and their adjoint,
   // 13.6 ms on single CTAs, 11.5 with the 16 heaviest on clusters of 4, 11.8 with 32
   // on clusters of 2; with 512 such lattices 16.1 and 17.7, 18.8 (the weights'
@@ -816,7 +824,8 @@ class SimImpl final : public SimBase {
       if (p.size == 4) return {&p, std::min(n, CLS_SPLIT)};
 #endif
     if (plans_.empty() || n > 3 * n_sm_) return {};
-    constexpr double kOne = 1.45e5, kCluster = 1.64e5, kShare = 1.35;
+    constexpr double kOne = 1.45e5, kShare = 1.35;
+    auto cluster_fixed = [](int size) { return size > 8 ? 1.9e5 : 1.64e5; };
     std::vector<double> free_at;  // heap, the next free worker first
     // envs k0.. taken in order by the workers of free_at: when the last is done
     auto last_done = [&](int k0, double fixed, double per_cost) {
@@ -837,7 +846,7 @@ class SimImpl final : public SimBase {
     for (const ClusterPlan& p : plans_) {
       if (n > 2 * n_sm_) break;
       free_at.assign((size_t)p.resident, 0.0);
-      const double tp = last_done(0, kCluster, kShare / p.size);
+      const double tp = last_done(0, cluster_fixed(p.size), kShare / p.size);
       if (tp < t) {
         t = tp;
         best = {&p, n};
@@ -850,7 +859,7 @@ class SimImpl final : public SimBase {
         free_at.assign((size_t)(n_sm_ - heavy * p.size), 0.0);
         double done = 0;
         for (int k = 0; k < heavy; ++k) {
-          const double tk = kCluster + kShare / p.size * cost_[ies[k]];
+          const double tk = cluster_fixed(p.size) + kShare / p.size * cost_[ies[k]];
           free_at.insert(free_at.end(), p.size, tk);
           done = std::max(done, tk);
         }

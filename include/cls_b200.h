@@ -283,7 +283,7 @@ int cls_controller_batched(const cls_sim* sim, int32_t* on);
  * from global memory every substep, -1 (the default at creation) chooses 1
  * when it fits without fewer resident CTAs.  With up to 512 threads, a launch of
  * few envs, or the heaviest envs of an uneven one, runs each such env on a
- * thread-block cluster of 2, 4 or 8 CTAs of that size where that is estimated to
+ * thread-block cluster of 2, 4, 8 or 16 CTAs of that size where that is estimated to
  * end earlier; those read the controller from global memory.  Results do not depend on
  * ctas_per_sm or weights_shared, and depend on threads_per_block (and on the
  * use of clusters: gradients) only through the rounding of reductions.  No reference counterpart: Taichi
