@@ -391,9 +391,13 @@ extern "C" int cls_ms_advance_noalloc(const cls_noalloc_advance* a, void* stream
   // one CTA per env when an env's springs fit in its shared memory (up to about
   // 5000 springs); larger ones keep a launch per phase over the scratch array
   const size_t smem = carve_fused(nullptr, a->n_vertices, a->n_springs, nullptr);
-  if (a->n_substeps > 0 && a->n_vertices <= kFusedMax && a->n_springs <= kFusedMax && smem <= fused_capacity()) {
+  const size_t fused_max = fused_capacity();
+  if (a->n_substeps > 0 && a->n_vertices <= kFusedMax && a->n_springs <= kFusedMax && smem <= fused_max) {
+    // the limit belongs to the kernel in the whole process: always the device's
+    // maximum, so that a call with a smaller robot on another host thread never
+    // lowers it between this call's raise and its launch
     cudaError_t e = smem > 48 * 1024
-                        ? cudaFuncSetAttribute(na_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                        ? cudaFuncSetAttribute(na_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_max)
                         : cudaSuccess;
     if (e == cudaSuccess) {
       const int work = a->n_springs > a->n_vertices ? a->n_springs : a->n_vertices;
@@ -401,6 +405,7 @@ extern "C" int cls_ms_advance_noalloc(const cls_noalloc_advance* a, void* stream
       e = cudaGetLastError();
     }
     if (e != cudaSuccess) {
+      cudaGetLastError();  // this call's own error: reported here, not left for the next call
       set_message(a, cudaGetErrorString(e));
       return CLS_ERR_CUDA;
     }
