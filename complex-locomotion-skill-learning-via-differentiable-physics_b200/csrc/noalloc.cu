@@ -210,6 +210,7 @@ constexpr int kFusedMax = 32767;   // springs (2 s + side in 16 bits) and vertic
 // with 900 of them, one substep: 2830 us when its thread sorted and summed them
 // alone, 44 now)
 constexpr int kThreadRow = 48;
+constexpr int kFillMax = 12;       // incidences per thread while the rows are sorted
 
 __host__ __device__ inline size_t carve_fused(char* base, int nv, int ns, FusedShared* s) {
   size_t off = 0;
@@ -281,8 +282,8 @@ __global__ void __launch_bounds__(1024) na_fused(cls_noalloc_advance a, float dr
     }
   }
   __syncthreads();
-  // rows in any order, then sorted by their vertex's thread; the long rows of hub
-  // vertices are written in order by a warp each (na_hubs)
+  // rows in any order, then sorted; the long rows of hub vertices are written in
+  // order by a warp each (na_hubs)
   bool long_row = false;
   for (int i = tid; i < N; i += nt) long_row |= s.ptr[i + 1] - s.ptr[i] > kThreadRow;
   const bool hubs = __syncthreads_or(long_row);
@@ -295,17 +296,6 @@ __global__ void __launch_bounds__(1024) na_fused(cls_noalloc_advance a, float dr
     if (ab.x == kNone) continue;
     if (by_thread(ab.x)) s.inc[atomicAdd(fill + ab.x, 1)] = (unsigned short)(2 * q);
     if (by_thread(ab.y)) s.inc[atomicAdd(fill + ab.y, 1)] = (unsigned short)(2 * q + 1);
-  }
-  __syncthreads();
-  for (int i = tid; i < N; i += nt) {
-    const int b = s.ptr[i], e = s.ptr[i + 1];
-    if (e - b > kThreadRow) continue;
-    for (int p = b + 1; p < e; ++p) {
-      const unsigned short c = s.inc[p];
-      int r = p;
-      for (; r > b && s.inc[r - 1] > c; --r) s.inc[r] = s.inc[r - 1];
-      s.inc[r] = c;
-    }
   }
   const int lane = tid & 31;
   const unsigned below = (1u << lane) - 1u;
@@ -322,6 +312,34 @@ __global__ void __launch_bounds__(1024) na_fused(cls_noalloc_advance a, float dr
         at += __popc(in_a) + __popc(in_b);
       }
     });
+  __syncthreads();
+  // a thread per incidence: its place in its row is the number of smaller ones (one
+  // quadruped, 608 springs, one substep: 10.4 us a call, 18.7 with a row sorted by its
+  // vertex's thread)
+  {
+    unsigned short code[kFillMax];
+    int to[kFillMax];
+    const int n_inc = s.ptr[N];
+#pragma unroll
+    for (int k = 0; k < kFillMax; ++k) {
+      const int at = tid + k * nt;
+      to[k] = -1;
+      if (at >= n_inc) continue;
+      code[k] = s.inc[at];
+      const ushort2 ab = s.ab[code[k] >> 1];
+      const int i = (code[k] & 1) ? ab.y : ab.x;
+      const int b = s.ptr[i], e = s.ptr[i + 1];
+      if (e - b > kThreadRow) continue;
+      int rank = 0;
+#pragma unroll 8
+      for (int p = b; p < e; ++p) rank += s.inc[p] < code[k];
+      to[k] = b + rank;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kFillMax; ++k)
+      if (to[k] >= 0) s.inc[to[k]] = code[k];
+  }
   for (int i = tid; i < N; i += nt) {
     cls::V4<float> v;
     v.x = ve[3 * i]; v.y = ve[3 * i + 1]; v.z = ve[3 * i + 2]; v.w = 0;
@@ -405,6 +423,11 @@ size_t fused_capacity() {
   return (size_t)optin;
 }
 
+int fused_threads(const cls_noalloc_advance& a) {
+  const int work = a.n_springs > a.n_vertices ? a.n_springs : a.n_vertices;
+  return work <= 256 ? 256 : (work <= 1024 ? 512 : 1024);
+}
+
 int grid_for(long long n) {
   long long g = (n + 255) / 256;
   if (g > 148 * 16) g = 148 * 16;
@@ -454,7 +477,8 @@ extern "C" int cls_ms_advance_noalloc(const cls_noalloc_advance* a, void* stream
   // 5000 springs); larger ones keep a launch per phase over the scratch array
   const size_t smem = carve_fused(nullptr, a->n_vertices, a->n_springs, nullptr);
   const size_t fused_max = fused_capacity();
-  if (a->n_substeps > 0 && a->n_vertices <= kFusedMax && a->n_springs <= kFusedMax && smem <= fused_max) {
+  if (a->n_substeps > 0 && a->n_vertices <= kFusedMax && 2 * a->n_springs <= kFillMax * fused_threads(*a) &&
+      smem <= fused_max) {
     // the limit belongs to the kernel in the whole process: always the device's
     // maximum, so that a call with a smaller robot on another host thread never
     // lowers it between this call's raise and its launch
@@ -462,8 +486,7 @@ extern "C" int cls_ms_advance_noalloc(const cls_noalloc_advance* a, void* stream
                         ? cudaFuncSetAttribute(na_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_max)
                         : cudaSuccess;
     if (e == cudaSuccess) {
-      const int work = a->n_springs > a->n_vertices ? a->n_springs : a->n_vertices;
-      na_fused<<<a->n_envs, work <= 256 ? 256 : (work <= 1024 ? 512 : 1024), smem, s>>>(*a, drag_s);
+      na_fused<<<a->n_envs, fused_threads(*a), smem, s>>>(*a, drag_s);
       e = cudaGetLastError();
     }
     if (e != cudaSuccess) {
