@@ -8,13 +8,16 @@
 #include <cstdio>
 #include <cstring>
 #include <functional>
+#include <initializer_list>
 #include <memory>
+#include <mutex>
 #include <numeric>
 #include <string>
 #include <type_traits>
 #include <vector>
 
 #include "../../include/cls_b200.h"
+#include "cls_context.h"
 #include "cls_profile.cuh"
 #include "ms_cluster_host.h"
 #include "ms_dense_host.h"
@@ -134,33 +137,84 @@ struct StageRing {
   }
 };
 
+// Page-locked host memory blocks that closed handles leave for new ones: making one
+// takes the driver 2 ms, several times a small rollout.  At most kKeep bytes are kept
+// (the rest goes back to the system), each for handles of the context that made
+// it.  A block belongs to one handle at a time.
+class MappedPool {
+ public:
+  struct Block {
+    unsigned char* p = nullptr;
+    size_t bytes = 0;
+    unsigned long long ctx = 0;
+  };
+  static MappedPool& get() {
+    static MappedPool* pool = new MappedPool;  // outlives every handle: never destroyed
+    return *pool;
+  }
+  Block take(size_t bytes) {
+    Block b;
+    b.bytes = kSmallest;
+    while (b.bytes < bytes) b.bytes *= 2;
+    const bool known = current_ctx_id(&b.ctx) && b.ctx;
+    if (known) {
+      std::lock_guard<std::mutex> hold(lock_);
+      for (size_t k = 0; k < free_.size(); ++k)
+        if (free_[k].ctx == b.ctx && free_[k].bytes == b.bytes) {
+          b = free_[k];
+          free_.erase(free_.begin() + k);
+          kept_ -= b.bytes;
+          return b;
+        }
+    }
+    if (cudaHostAlloc(reinterpret_cast<void**>(&b.p), b.bytes, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();  // no page-locked memory to be had: the handle copies instead
+      b = Block{};
+    }
+    return b;
+  }
+  void give_back(const Block& b) {
+    if (!b.p) return;
+    if (b.ctx) {
+      std::lock_guard<std::mutex> hold(lock_);
+      if (kept_ + b.bytes <= kKeep) {
+        free_.push_back(b);
+        kept_ += b.bytes;
+        return;
+      }
+    }
+    cudaFreeHost(b.p);
+  }
+
+ private:
+  static constexpr size_t kSmallest = size_t(1) << 16, kKeep = size_t(8) << 20;
+  std::mutex lock_;
+  std::vector<Block> free_;
+  size_t kept_ = 0;
+};
+
 // Page-locked host memory that kernels read and write in place, for the small
 // results and inputs of latency-bound calls: a kernel's stores and one stream
 // synchronisation instead of a copy per array through pageable memory (an
-// observables + final-state read of one env, 100 steps: 120 -> 40 us).  Grows to
-// the largest request of its handle, at most kMax bytes.
+// observables + final-state read of one env, 100 steps: 120 -> 40 us).  Sized when the
+// handle is made, so that no later call allocates; transfers of more than kMax bytes
+// are copies.
 struct HostMapped {
   static constexpr size_t kMax = size_t(1) << 20;
-  unsigned char* p = nullptr;
-  size_t bytes = 0;
-  // `n` bytes, or null when that is more than a mapped transfer is good for
+  MappedPool::Block block;
+  // room for the largest of the handle's transfers that are small enough
+  void reserve(std::initializer_list<size_t> transfers) {
+    size_t need = 0;
+    for (size_t n : transfers)
+      if (n <= kMax) need = std::max(need, n);
+    block = MappedPool::get().take(need);
+  }
+  // `n` values, or null when that is more than a mapped transfer is good for
   template <typename T>
-  T* get(size_t n) {
-    const size_t need = sizeof(T) * n;
-    if (need > kMax) return nullptr;
-    if (need > bytes) {
-      if (p) cudaFreeHost(p);
-      p = nullptr;
-      bytes = 0;
-      const size_t b = std::max<size_t>(need, 1 << 16);
-      CLS_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&p), b, cudaHostAllocMapped | cudaHostAllocPortable));
-      bytes = b;
-    }
-    return reinterpret_cast<T*>(p);
+  T* get(size_t n) const {
+    return sizeof(T) * n <= block.bytes ? reinterpret_cast<T*>(block.p) : nullptr;
   }
-  ~HostMapped() {
-    if (p) cudaFreeHost(p);
-  }
+  ~HostMapped() { MappedPool::get().give_back(block); }
 };
 
 class SimBase {
@@ -601,6 +655,15 @@ class SimImpl final : public SimBase {
     stage = std::max<size_t>(stage, (size_t)boff);
     d_stage_.alloc(stage);
     d_tns_.alloc(1);
+    {
+      int outs = 1, ins = 1;
+      for (const HostRobot& h : hr_) {
+        outs = std::max(outs, h.width[L_]);
+        ins = std::max(ins, h.full_cols[0]);
+      }
+      mapped_.reserve({sizeof(double) * 8 * E, sizeof(double) * 6 * V_, sizeof(double) * 6 * T_ * (size_t)E,
+                       sizeof(R) * (size_t)E * (outs + ins + 4)});  // loss, states, observables, env steps
+    }
     // uploads
     CLS_CUDA(cudaMemcpy(d_robots_.p, rd.data(), sizeof(RobotDesc) * nr, cudaMemcpyHostToDevice));
     CLS_CUDA(cudaMemcpy(d_envs_.p, ed.data(), sizeof(EnvDesc) * E, cudaMemcpyHostToDevice));
@@ -1698,7 +1761,8 @@ class SimImpl final : public SimBase {
     CLS_REQUIRE(bwd_done_, "cls_adam_step needs gradients (cls_backward) first");
     adam_device(iter, true, tns ? d_tns_.p : nullptr);
     if (tns) {
-      double* m = mapped_.template get<double>(1);
+      double v = 0, *m = mapped_.template get<double>(1);
+      if (!m) m = &v;
       CLS_CUDA(cudaMemcpyAsync(m, d_tns_.p, sizeof(double), cudaMemcpyDeviceToHost, stream));
       CLS_CUDA(cudaStreamSynchronize(stream));
       *tns = *m;

@@ -36,13 +36,13 @@
 //   * a CUDA error already pending when the call starts (from the caller's
 //     earlier work) is left in place and reported as CLS_ERR_CUDA without
 //     launching anything.
-#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstdio>
 #include <mutex>
 
 #include "../../include/cls_b200.h"
+#include "cls_context.h"
 #include "ms_kernels.cuh"
 
 namespace {
@@ -63,45 +63,13 @@ ScratchEntry g_scratch[kMaxContexts] = {};
 int g_scratch_used = 0, g_scratch_next = 0;
 std::mutex g_scratch_mutex;
 
-// driver entry points, resolved through the runtime so that the library does
-// not link libcuda (it must load on machines without a driver)
-typedef CUresult (*CtxGetCurrentFn)(CUcontext*);
-typedef CUresult (*CtxGetIdFn)(CUcontext, unsigned long long*);
-CtxGetCurrentFn g_ctx_get_current = nullptr;
-CtxGetIdFn g_ctx_get_id = nullptr;
-
-bool resolve_driver_calls() {
-  if (g_ctx_get_current && g_ctx_get_id) return true;
-  void* f0 = nullptr;
-  void* f1 = nullptr;
-  cudaDriverEntryPointQueryResult q0, q1;
-  if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f0, cudaEnableDefault, &q0) != cudaSuccess ||
-      q0 != cudaDriverEntryPointSuccess || !f0)
-    return false;
-  if (cudaGetDriverEntryPoint("cuCtxGetId", &f1, cudaEnableDefault, &q1) != cudaSuccess ||
-      q1 != cudaDriverEntryPointSuccess || !f1)
-    return false;
-  g_ctx_get_current = reinterpret_cast<CtxGetCurrentFn>(f0);
-  g_ctx_get_id = reinterpret_cast<CtxGetIdFn>(f1);
-  return true;
-}
-
-// id of the current context (0 when none is current)
-unsigned long long current_ctx_id() {
-  CUcontext ctx = nullptr;
-  unsigned long long id = 0;
-  if (g_ctx_get_current(&ctx) != CUDA_SUCCESS || !ctx) return 0;
-  if (g_ctx_get_id(ctx, &id) != CUDA_SUCCESS) return 0;
-  return id;
-}
-
 // The scratch's device address in the current context; on the first call in a
 // context, cudaGetSymbolAddress (which also makes the device's primary context
 // current when no context is) resolves it with that context current.
 cudaError_t scratch_address(float** out) {
   std::lock_guard<std::mutex> lock(g_scratch_mutex);
-  if (!resolve_driver_calls()) return cudaErrorNotSupported;
-  unsigned long long id = current_ctx_id();
+  unsigned long long id = 0;
+  if (!cls::current_ctx_id(&id)) return cudaErrorNotSupported;
   if (id) {
     for (int i = 0; i < g_scratch_used; ++i)
       if (g_scratch[i].ctx_id == id) {
@@ -113,7 +81,7 @@ cudaError_t scratch_address(float** out) {
   const cudaError_t e = cudaGetSymbolAddress(&p, g_vinc_scratch);
   if (e != cudaSuccess) return e;
   if (!p) return cudaErrorInvalidSymbol;
-  if (!id) id = current_ctx_id();   // the lookup made the primary context current
+  if (!id) cls::current_ctx_id(&id);   // the lookup made the primary context current
   if (id) {
     int slot = g_scratch_used < kMaxContexts ? g_scratch_used++ : g_scratch_next;
     if (g_scratch_used == kMaxContexts) g_scratch_next = (slot + 1) % kMaxContexts;
