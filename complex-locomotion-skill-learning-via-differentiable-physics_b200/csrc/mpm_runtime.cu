@@ -75,6 +75,7 @@ class MpmBase {
   virtual void graph_launch() = 0;
   virtual void profile_enable(bool on) = 0;
   virtual void profile_read(double* ms, long long* launches, bool reset) = 0;
+  virtual long long record_bytes() const = 0;
 };
 
 // launch categories of the per-kernel profile (CLS_MPM_PROFILE_KINDS)
@@ -85,7 +86,7 @@ class MpmImpl final : public MpmBase {
   using V = V4<R>;
 
  public:
-  MpmImpl(const cls_mpm_body& b, const cls_mpm_params& p, int n_envs) : p_(p) {
+  MpmImpl(const cls_mpm_body& b, const cls_mpm_params& p, int n_envs, long long record_bytes) : p_(p) {
     E_ = n_envs;
     P_ = b.n_particles;
     M_ = std::max(1, b.n_muscles);
@@ -114,15 +115,19 @@ class MpmImpl final : public MpmBase {
     // Record slots for every step of the longest rollout, written by the first
     // pass, so that the reverse pass recomputes nothing (27 % of an 8-env
     // legged-body iteration): when that takes no more slots than two segment
-    // records, or at most a sixteenth of the free device memory.
+    // records, or at most the caller's record_bytes.  What else is in memory
+    // counts only where the record would take more than half of what is free.
     {
-      const double per_slot = sizeof(R) * ((double)E_ * P_ * 2 * (D + D * D) + 4.0 * E_ * nblk_ * Blk<D>::NODES);
+      const double need = (double)T_ * sizeof(R) *
+                          ((double)E_ * P_ * 2 * (D + D * D) + 4.0 * E_ * nblk_ * Blk<D>::NODES);
       size_t free_b = 0, total_b = 0;
       MPM_CUDA(cudaMemGetInfo(&free_b, &total_b));
-      whole_ = T_ <= 2 * slots_ || T_ * per_slot <= free_b / 16.0;
+      const double budget = record_bytes < 0 ? (double)CLS_MPM_RECORD_BYTES : (double)record_bytes;
+      whole_ = (record_bytes < 0 && T_ <= 2 * slots_) || (need <= budget && need <= 0.5 * free_b);
       if (whole_) {
         slots_ = std::max(T_, 2);
         n_ckpt_ = 1;
+        record_bytes_ = (long long)need;
       }
     }
     build_order(b);
@@ -672,6 +677,8 @@ class MpmImpl final : public MpmBase {
     if (gF0) down_planes(out_aF_.p, gF0, D * D);
   }
 
+  long long record_bytes() const override { return record_bytes_; }
+
   void centers(double* c) override {
     MPM_CUDA(cudaMemcpyAsync(c, csum_.p, sizeof(double) * (T_ + 1) * E_ * D, cudaMemcpyDeviceToHost, stream));
     MPM_CUDA(cudaStreamSynchronize(stream));
@@ -699,6 +706,7 @@ class MpmImpl final : public MpmBase {
   std::vector<int> chunk_start_h_, chunk_len_h_;
   bool runs_ = false;  // CLS_MPM_ORDER_BASE_RUNS
   bool whole_ = false;  // every step recorded by the first pass
+  long long record_bytes_ = 0;  // of that record
   bool small_ = false;  // one CTA per env (mpm_small.cuh)
   int small_cap_[2] = {0, 0};  // its scatter tables' sizes
   bool fwd_done_ = false, bwd_done_ = false;
@@ -759,6 +767,11 @@ void cls_mpm_default_params(cls_mpm_params* p) {
 
 int cls_mpm_create(const cls_mpm_body* body, const cls_mpm_params* params, int32_t n_envs,
                    cls_mpm** out) {
+  return cls_mpm_create_recorded(body, params, n_envs, -1, out);
+}
+
+int cls_mpm_create_recorded(const cls_mpm_body* body, const cls_mpm_params* params, int32_t n_envs,
+                            int64_t record_bytes, cls_mpm** out) {
   using namespace cls::mpm;
   if (!out) return CLS_ERR_INVALID;
   *out = nullptr;
@@ -778,11 +791,11 @@ int cls_mpm_create(const cls_mpm_body* body, const cls_mpm_params* params, int32
     auto* s = new cls_mpm;
     try {
       if (params->precision == 32) {
-        if (body->dim == 2) s->impl.reset(new MpmImpl<float, 2>(*body, *params, n_envs));
-        else s->impl.reset(new MpmImpl<float, 3>(*body, *params, n_envs));
+        if (body->dim == 2) s->impl.reset(new MpmImpl<float, 2>(*body, *params, n_envs, record_bytes));
+        else s->impl.reset(new MpmImpl<float, 3>(*body, *params, n_envs, record_bytes));
       } else {
-        if (body->dim == 2) s->impl.reset(new MpmImpl<double, 2>(*body, *params, n_envs));
-        else s->impl.reset(new MpmImpl<double, 3>(*body, *params, n_envs));
+        if (body->dim == 2) s->impl.reset(new MpmImpl<double, 2>(*body, *params, n_envs, record_bytes));
+        else s->impl.reset(new MpmImpl<double, 3>(*body, *params, n_envs, record_bytes));
       }
     } catch (...) {
       delete s;
@@ -836,6 +849,10 @@ int cls_mpm_get_final_state(cls_mpm* s, double* x, double* v, double* C, double*
 }
 int cls_mpm_get_grads(cls_mpm* s, double* gact, double* gx0, double* gv0, double* gC0, double* gF0) {
   return mguard(s, [&](cls::mpm::MpmBase& b) { b.grads(gact, gx0, gv0, gC0, gF0); });
+}
+int cls_mpm_record_bytes(cls_mpm* s, int64_t* bytes) {
+  if (!bytes) return CLS_ERR_INVALID;
+  return mguard(s, [&](cls::mpm::MpmBase& b) { *bytes = b.record_bytes(); });
 }
 int cls_mpm_get_centers(cls_mpm* s, double* centers) {
   return mguard(s, [&](cls::mpm::MpmBase& b) { b.centers(centers); });

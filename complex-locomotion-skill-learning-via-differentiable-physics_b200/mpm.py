@@ -32,6 +32,9 @@ _SIGS = {
     "cls_mpm_default_params": (None, [ctypes.POINTER(MPMParams)]),
     "cls_mpm_create": (_i32, [ctypes.POINTER(MPMBody), ctypes.POINTER(MPMParams), _i32,
                               ctypes.POINTER(ctypes.c_void_p)]),
+    "cls_mpm_create_recorded": (_i32, [ctypes.POINTER(MPMBody), ctypes.POINTER(MPMParams), _i32, ctypes.c_int64,
+                                       ctypes.POINTER(ctypes.c_void_p)]),
+    "cls_mpm_record_bytes": (_i32, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int64)]),
     "cls_mpm_destroy": (_i32, [ctypes.c_void_p]),
     "cls_mpm_last_error": (ctypes.c_char_p, [ctypes.c_void_p]),
     "cls_mpm_set_stream": (_i32, [ctypes.c_void_p, ctypes.c_void_p]),
@@ -88,13 +91,25 @@ def default_params(**over):
     return p
 
 
+def record_bytes(n_particles, dim, n_grid, steps, n_envs=1, precision=32):
+    """Device bytes of a whole-rollout record (``MPMBatch(record_bytes=...)``): particle
+    state and grid (blocks of 8 x 8 or 4 x 4 x 4 nodes) of every step."""
+    side = 8 if dim == 2 else 4
+    nodes = (-(-n_grid // side) * side) ** dim
+    return steps * n_envs * (precision // 8) * (n_particles * 2 * (dim + dim * dim) + 4 * nodes)
+
+
 def _f64(a, shape):
     return np.ascontiguousarray(np.asarray(a, dtype=np.float64).reshape(shape))
 
 
 class MPMBatch:
+    """record_bytes bounds the device memory of a record of the whole rollout, with
+    which the reverse pass recomputes nothing (cls_mpm_create_recorded; None: the
+    library's bound, 0: none, segments of checkpoint_every steps are recomputed)."""
+
     def __init__(self, positions, muscle, n_envs, *, dim, fibre=None, n_muscles=None,
-                 params=None, **over):
+                 params=None, record_bytes=None, **over):
         self.lib = _lib()
         self.dim = dim
         self.positions = _f64(positions, (-1, dim))
@@ -108,8 +123,8 @@ class MPMBatch:
         body = MPMBody(dim, self.P, _capi.ptr(self.positions), _capi.ptr(self.muscle, _capi.P_I),
                        _capi.ptr(self.fibre), self.M)
         h = ctypes.c_void_p()
-        rc = self.lib.cls_mpm_create(ctypes.byref(body), ctypes.byref(self.params), n_envs,
-                                     ctypes.byref(h))
+        rc = self.lib.cls_mpm_create_recorded(ctypes.byref(body), ctypes.byref(self.params), n_envs,
+                                              -1 if record_bytes is None else int(record_bytes), ctypes.byref(h))
         self._check(rc, None)
         self.h = h
 
@@ -132,6 +147,13 @@ class MPMBatch:
             self.close()
         except Exception:
             pass
+
+    @property
+    def record_bytes(self):
+        """Device bytes of the handle's whole-rollout record (0: it recomputes segments)."""
+        n = ctypes.c_int64()
+        self._c(self.lib.cls_mpm_record_bytes(self.h, ctypes.byref(n)))
+        return n.value
 
     def set_stream(self, s):
         self._c(self.lib.cls_mpm_set_stream(self.h, ctypes.c_void_p(s)))

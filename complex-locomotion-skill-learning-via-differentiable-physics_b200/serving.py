@@ -119,7 +119,9 @@ def footprint_bytes(robot, steps, grad, K, dtype_bytes=4):
 class MpmType:
     """A registered MPM body type: particle positions [P][dim], muscle id
     per particle (-1 passive), fibre directions, and MPMBatch keyword
-    arguments of the solver (material, n_grid, dt, mu, la, ...)."""
+    arguments of the solver (material, n_grid, dt, mu, la, ...).  A slot records
+    its whole rollout only where the solver's record_bytes allows it (default:
+    none, it keeps one segment's records)."""
     positions: np.ndarray
     muscle: np.ndarray
     fibre: Optional[np.ndarray] = None
@@ -144,10 +146,16 @@ def mpm_request_inputs(seed, T, steps, n_muscles, dt, dim=3):
 def mpm_footprint_bytes(mt, T, K, dtype_bytes=4):
     """HBM bytes of one MPM slot: particle checkpoints (x, v, C, F) every K
     steps over T, one segment's records, the actuation and centre tracks, and
-    the grid (n_grid^dim nodes of 16 bytes, twice for the adjoint)."""
+    the grid (n_grid^dim nodes of 16 bytes, twice for the adjoint); with room for
+    it in the type's record_bytes, the record of the whole rollout instead of the
+    checkpoints and the segment's."""
+    from .mpm import record_bytes
     P, D = mt.positions.shape
     n_grid = int(mt.solver.get("n_grid", 64))
     per_p = (2 * D + 2 * D * D) * dtype_bytes
+    whole = record_bytes(P, D, n_grid, T, precision=int(mt.solver.get("precision", 32)))
+    if whole <= int(mt.solver.get("record_bytes", 0)):
+        return int(whole + P * per_p + 2 * 16 * n_grid ** D + T * (mt.n_muscles + 2 * D) * dtype_bytes)
     return int(P * per_p * (T // K + 2) + P * per_p * K + 2 * 16 * n_grid ** D
                + T * (mt.n_muscles + 2 * D) * dtype_bytes)
 
@@ -164,9 +172,10 @@ class MpmSlotBackend:
         dim = mt.positions.shape[1]
         self.dim = dim
         self.batches, self.streams, self.events = [], [], []
+        solver = {"record_bytes": 0, **mt.solver}   # what mpm_footprint_bytes counts
         for _ in range(n_slots):
             b = MPMBatch(mt.positions, mt.muscle, 1, dim=dim, fibre=mt.fibre, n_muscles=mt.n_muscles,
-                         max_steps=self.T, checkpoint_every=self.K, **mt.solver)
+                         max_steps=self.T, checkpoint_every=self.K, **solver)
             st = None
             if streams:
                 import torch

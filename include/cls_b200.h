@@ -495,6 +495,21 @@ void cls_mpm_default_params(cls_mpm_params* p);
 /* Replaces SolverMPM.__init__ + initialize_robot (solver_mpm.py:7-58). */
 int cls_mpm_create(const cls_mpm_body* body, const cls_mpm_params* params, int32_t n_envs,
                    cls_mpm** out);
+/* The same with a bound on the device memory of the whole-rollout record.  A
+ * handle keeps checkpoints every checkpoint_every steps and the records of two
+ * segments, and the reverse pass recomputes each segment -- or, where the states
+ * and grids of all max_steps steps take at most record_bytes, it records every
+ * step in the first pass and recomputes nothing (the legged body, 8 envs: 27 % of
+ * an iteration; 7 MB per env and step on a 64^3 grid).  0: never.  Negative, and
+ * cls_mpm_create: at most CLS_MPM_RECORD_BYTES, or where max_steps slots are no
+ * more than the two segments'.  A record that would take more than half of the
+ * free device memory is not made.  Rollouts that never run in reverse (the record
+ * costs them up to 6 %) and callers with many handles pass 0. */
+#define CLS_MPM_RECORD_BYTES (8LL << 30)
+int cls_mpm_create_recorded(const cls_mpm_body* body, const cls_mpm_params* params, int32_t n_envs,
+                            int64_t record_bytes, cls_mpm** out);
+/* Bytes of the handle's whole-rollout record (0: it recomputes segments). */
+int cls_mpm_record_bytes(cls_mpm* sim, int64_t* bytes);
 int cls_mpm_destroy(cls_mpm* sim);
 const char* cls_mpm_last_error(const cls_mpm* sim);
 int cls_mpm_set_stream(cls_mpm* sim, void* stream);
