@@ -1,7 +1,9 @@
-"""The MPM handle's whole-rollout record: bounded by the caller."""
+"""The MPM handle's whole-rollout record: bounded by the caller, and the recomputing
+reverse pass that handles without one take, on the same references as the recorded."""
 import numpy as np
 import pytest
 
+import test_mpm_gpu as recorded
 from test_mpm_oracle import body3d
 
 pytestmark = pytest.mark.gpu
@@ -44,3 +46,42 @@ def test_serving_slot_memory():
     took = before - torch.cuda.mem_get_info()[0]
     backend.close()
     assert took < 2 << 30
+
+
+@pytest.fixture
+def segments(monkeypatch):
+    """Handles without a record, counted."""
+    from cls_b200 import mpm
+    made = []
+    real = mpm.MPMBatch
+
+    def make(*a, **k):
+        b = real(*a, record_bytes=0, **k)
+        assert b.record_bytes == 0
+        made.append(b)
+        return b
+
+    monkeypatch.setattr(mpm, "MPMBatch", make)
+    yield made
+    assert made
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("material", ["fixed_corotated", "neo_hookean"])
+def test_2d_gradients(segments, material, precision):
+    recorded.test_mpm2d_gradients_match_oracle(material, precision)
+
+
+@pytest.mark.parametrize("precision, tile, order", [(64, 0, "cells"), (32, 0, "cells"), (64, 256, "cells"),
+                                                    (32, 48, "cells"), (64, 0, "base_runs"), (32, 0, "base_runs")])
+def test_3d(segments, precision, tile, order):
+    recorded.test_mpm3d_neo_hookean_fibre_matches_oracle(precision, tile, order)
+
+
+def test_forward_golden(segments):
+    for precision in (64, 32):
+        recorded.test_mpm2d_forward_matches_reference_golden(precision)
+
+
+def test_intervals_and_graph_replay(segments):
+    recorded.test_mpm_checkpoint_interval_and_graph_replay()
