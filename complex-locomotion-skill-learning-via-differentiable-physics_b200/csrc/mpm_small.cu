@@ -29,11 +29,12 @@ int threads(int P) {
 template <typename R, int D>
 cudaError_t SmallLaunch<R, D>::plan(int E, int P, int n_grid, bool* ok, int* fwd_cap, int* adj_cap) {
   *ok = false;
-  if (!small_body(E, P) || n_grid < 3 || n_grid > 1000 || node_count(D, n_grid) > (1 << 15)) return cudaSuccess;
-  int dev = 0, optin = 0;
+  if (n_grid < 3 || n_grid > 1000 || node_count(D, n_grid) > (1 << 15)) return cudaSuccess;
+  int dev = 0, optin = 0, n_sm = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (e != cudaSuccess) return e;
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess || !small_body(D, E, P, n_sm)) return e;
   // a run per particle at most; smaller tables where that does not fit, down to
   // one per four particles (the voxelised bodies' runs), else the general kernels
   int caps[2] = {0, 0};
@@ -53,7 +54,17 @@ cudaError_t SmallLaunch<R, D>::plan(int E, int P, int n_grid, bool* ok, int* fwd
   e = cudaFuncSetAttribute(mpm_small_fwd_kernel<R, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(mpm_small_adj_kernel<R, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-  *ok = e == cudaSuccess;
+  // more envs than SMs: only where an SM holds two
+  int nf = 2, nr = 2;
+  if (E > n_sm) {
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nf, mpm_small_fwd_kernel<R, D>, threads(P),
+                                                        fwd_bytes<R, D>(P, n_grid, caps[0]));
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nr, mpm_small_adj_kernel<R, D>, threads(P),
+                                                        adj_bytes<R, D>(P, n_grid, caps[1]));
+  }
+  *ok = e == cudaSuccess && nf >= 2 && nr >= 2;
   *fwd_cap = caps[0];
   *adj_cap = caps[1];
   return e;

@@ -9,14 +9,20 @@ namespace cls {
 namespace mpm {
 
 constexpr int kSmallThreads = 512;
-// Particles per env up to which one CTA takes a whole env: forward + reverse per
-// substep, B200, one CTA per env / the general kernels: 1-16 envs of 400, 1000,
-// 2000 particles 12 / 22, 23 / 23, 47 / 23 us (a lone CTA issues everything), 148
-// envs 13 / 27, 25 / 42, 49 / 67 us (every SM has its env), 600 envs 57 / 60, 121 /
-// 113, 241 / 227 us.
-constexpr int kSmallParticles = 896, kSmallParticlesMany = 2048;
-__host__ inline bool small_body(int E, int P) {
-  return P <= kSmallParticles || (E >= 64 && E <= 296 && P <= kSmallParticlesMany);
+// Bodies that one CTA takes whole, by dimension, envs E, particles P and the device's
+// SMs.  Times over those of the general kernels with a record, forward / forward and
+// reverse, B200, voxelised and random bodies (24 substeps).  2D, 32 x 32 grid: up to 512
+// particles 0.41-0.60 / 0.46-0.62 at 1-148 envs, 0.75-0.97 / 0.82-0.97 at 600-1000 while
+// two CTAs fit an SM (the caller checks), beyond 8 envs per SM no gain; on a
+// 64 x 64 grid, one CTA per SM, 0.5-0.6 / 0.6-0.7 up to 148 envs and 0.9-1.4 / 0.9-1.5 at
+// 200-600.  Up to 896: 0.63-0.96 / 0.55-1.02 at 1-148, 1.1-1.5 / 1.0-1.3 at 200 and 600.  Up
+// to 2048 only with an env for most SMs: 148 envs 0.75 / 0.65, 64 1.0-1.1 / 0.95, 1 env 1.8.
+// 3D (8 particles per cell, 27 sums per run): 300-512 particles and 148 envs 0.7-0.8 /
+// 0.7-0.87, else 0.8-2.4 / 1.0-2.3.
+__host__ inline bool small_body(int D, int E, int P, int n_sm) {
+  const bool one_each = 3LL * E >= 2LL * n_sm && E <= n_sm;  // an env for most SMs
+  if (D == 3) return one_each && P > 256 && P <= 512;
+  return P <= 512 ? E <= 8LL * n_sm : (P <= 896 ? E <= n_sm : P <= 2048 && one_each);
 }
 
 template <typename R>
