@@ -181,7 +181,6 @@ class MpmImpl final : public MpmBase {
     MPM_CUDA(cudaMemcpy(pw_.p, pw.data(), sizeof(R) * P_, cudaMemcpyHostToDevice));
     loss_w_.assign(T_ + 1, 0.0);
     seed_w_.alloc(T_ + 1);
-    MPM_CUDA(cudaMemset(seed_w_.p, 0, sizeof(R) * (T_ + 1)));
     MPM_CUDA(cudaMemset(act_.p, 0, sizeof(R) * act_.n));
     MPM_CUDA(cudaMemset(target_.p, 0, sizeof(R) * target_.n));
     // shared-memory opt-in for the tile
@@ -520,6 +519,7 @@ class MpmImpl final : public MpmBase {
       a.target = target_.p;
       a.pw_sum = (R)pw_sum_;
       a.out_ax = out_ax_.p; a.out_av = out_av_.p; a.out_aC = out_aC_.p; a.out_aF = out_aF_.p;
+      timed(MK_OTHER, [&] { MPM_CUDA((SmallLaunch<R, D>::seeds(loss_w_.data(), steps + 1, seed_w_.p, stream))); });
       timed(MK_PADJ, [&] { MPM_CUDA((SmallLaunch<R, D>::reverse(a, stream))); });
       bwd_done_ = true;
       return;
@@ -643,10 +643,7 @@ class MpmImpl final : public MpmBase {
   void set_actuation(const double* act_h) override { up(act_h, act_.p, (size_t)T_ * E_ * M_); }
 
   void set_loss(const double* w, const double* target, const double* pw) override {
-    if (w) {
-      loss_w_.assign(w, w + T_ + 1);
-      up(w, seed_w_.p, T_ + 1);
-    }
+    if (w) loss_w_.assign(w, w + T_ + 1);
     if (target) up(target, target_.p, (size_t)(T_ + 1) * E_ * D);
     if (pw) {
       std::vector<double> pi(P_);

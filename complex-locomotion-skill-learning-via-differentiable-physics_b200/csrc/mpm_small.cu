@@ -19,6 +19,11 @@ template <typename R, int D>
 size_t adj_bytes(int P, int n_grid, int cap) {
   return carve<R, D>(nullptr, P, (int)node_count(D, n_grid), cap, (SmallAdjShared<R, D>*)nullptr);
 }
+template <typename R>
+__global__ void seed_kernel(SeedChunk<R> c) {
+  for (int i = threadIdx.x; i < c.n; i += blockDim.x) c.out[i] = c.w[i];
+}
+
 // one warp per 32 particles, enough threads for the grid phase
 int threads(int P) {
   const int t = (P + 31) / 32 * 32;
@@ -78,6 +83,18 @@ cudaError_t SmallLaunch<R, D>::forward(const SmallFwdArgs<R>& a, cudaStream_t s)
 template <typename R, int D>
 cudaError_t SmallLaunch<R, D>::reverse(const SmallAdjArgs<R>& a, cudaStream_t s) {
   mpm_small_adj_kernel<R, D><<<a.c.E, threads(a.c.P), adj_bytes<R, D>(a.c.P, a.c.n_grid, a.cap), s>>>(a);
+  return cudaGetLastError();
+}
+
+template <typename R, int D>
+cudaError_t SmallLaunch<R, D>::seeds(const double* w, int n, R* out, cudaStream_t s) {
+  SeedChunk<R> c;
+  for (int i0 = 0; i0 < n; i0 += c.kMax) {
+    c.n = n - i0 < c.kMax ? n - i0 : c.kMax;
+    c.out = out + i0;
+    for (int i = 0; i < c.n; ++i) c.w[i] = (R)w[i0 + i];
+    seed_kernel<R><<<1, 256, 0, s>>>(c);
+  }
   return cudaGetLastError();
 }
 

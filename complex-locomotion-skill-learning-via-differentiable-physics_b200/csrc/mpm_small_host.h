@@ -53,6 +53,16 @@ struct SmallAdjArgs {
   R* out_ax; R* out_av; R* out_aC; R* out_aF;
 };
 
+// Loss weights of a launch, by value as the general kernels take theirs, so that a
+// captured reverse pass keeps the weights of its capture.
+template <typename R>
+struct SeedChunk {
+  static constexpr int kMax = 3840 / sizeof(R);   // kernel parameters: 4 KB
+  R w[kMax];
+  int n;
+  R* out;
+};
+
 template <typename R, int D>
 struct SmallLaunch {
   // whether E envs of P particles on an n_grid^D grid fit one CTA each on
@@ -61,6 +71,8 @@ struct SmallLaunch {
   static cudaError_t plan(int E, int P, int n_grid, bool* ok, int* fwd_cap, int* adj_cap);
   static cudaError_t forward(const SmallFwdArgs<R>& a, cudaStream_t s);
   static cudaError_t reverse(const SmallAdjArgs<R>& a, cudaStream_t s);
+  // w[0 .. n) into `out` on the device, for SmallAdjArgs::seed_w
+  static cudaError_t seeds(const double* w, int n, R* out, cudaStream_t s);
 };
 
 }  // namespace mpm
