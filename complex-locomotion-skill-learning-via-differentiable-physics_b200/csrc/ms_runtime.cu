@@ -811,7 +811,7 @@ class SimImpl final : public SimBase {
   };
   void plan_clusters(int optin) {
     plans_.clear();
-    batch_split_ = Split{};
+    batch_split_ = serve_rev_ = Split{};
     if (threads_ > ClusterLaunch<R>::max_threads()) return;
     size_t fwd_max = 0, rev_max = 0;
     CLS_CUDA(ClusterLaunch<R>::setup(optin, &fwd_max, &rev_max));
@@ -852,6 +852,7 @@ class SimImpl final : public SimBase {
       if (p.resident > 0) plans_.push_back(p);
     }
     batch_split_ = split_envs(order_host_.data(), E_);
+    serve_rev_ = split_envs(order_host_.data(), E_, false);
   }
 
   // Which of the envs `ies` (heaviest first) of a launch run as one cluster each,
@@ -876,7 +877,8 @@ class SimImpl final : public SimBase {
     const ClusterPlan* plan = nullptr;
     int heavy = 0;
   };
-  Split split_envs(const int* ies, int n) const {
+  // mixed: the second form too, else all of the envs or none.
+  Split split_envs(const int* ies, int n, bool mixed = true) const {
 #ifdef CLS_CLUSTER_SIZE
     for (const ClusterPlan& p : plans_)
       if (p.size == CLS_CLUSTER_SIZE) return {&p, n};
@@ -916,7 +918,7 @@ class SimImpl final : public SimBase {
       }
     }
     for (const ClusterPlan& p : plans_)
-      for (int q = 1; q <= 8; ++q) {
+      for (int q = 1; mixed && q <= 8; ++q) {
         const int heavy = p.resident * q / 8;
         if (heavy < 1 || heavy >= n || heavy * p.size > n_sm_) continue;
         free_at.assign((size_t)(n_sm_ - heavy * p.size), 0.0);
@@ -2327,7 +2329,7 @@ class SimImpl final : public SimBase {
     const Split split = split_envs(serve_order_h_.data(), n);
     timed(PK_RECOMP, [&] { launch_fwd(a, split, grid_for(n), 0, 0, FWD_RECORD, 0); });
     a.queue = d_squeue_.p + 1;
-    timed(PK_REV, [&] { launch_rev(a, split, grid_for(n), 0, 0, 0); });
+    timed(PK_REV, [&] { launch_rev(a, Split{serve_rev_.plan, n}, grid_for(n), 0, 0, 0); });
     if (!tiles.empty()) {
       unsigned char *h, *d;
       int slot;
@@ -2527,6 +2529,11 @@ class SimImpl final : public SimBase {
   std::vector<int> inc_ptr_h_;     // incidence row starts of the robot types
   std::vector<ClusterPlan> plans_;
   Split batch_split_;              // for launches over the whole batch
+  // For the reverse windows of serving, whatever envs are in them: the forward pass
+  // computes the same bits on one CTA and on clusters of any size, the reverse pass
+  // sums in another order on each, and a request's gradients must not depend on
+  // which others share its window.  All slots on clusters of one size, or none.
+  Split serve_rev_;
   std::vector<int> perm_, user_voff_, env_robot_, order_host_;
   bool identity_perm_ = true;
   std::vector<EnvDesc> ed_host_;
