@@ -337,6 +337,20 @@ class MassSpringBatch:
                                               ptr(w, _capi.P_I)))
         return int(t[0]), int(c[0]), int(w[0])
 
+    def set_clusters(self, size=-1, heavy=0):
+        """Thread-block clusters of the fused path: chosen for every launch (-1), none
+        (1), or the ``heavy`` heaviest envs (0: all) on clusters of ``size`` CTAs
+        (``cls_set_clusters``)."""
+        self._c(self.lib.cls_set_clusters(self.h, int(size), int(heavy)))
+
+    @property
+    def clusters(self):
+        """(cluster size, envs on clusters) of a launch over the whole batch; (1, 0)
+        without clusters."""
+        s, h = (np.zeros(1, dtype=np.int32) for _ in range(2))
+        self._c(self.lib.cls_get_clusters(self.h, ptr(s, _capi.P_I), ptr(h, _capi.P_I)))
+        return int(s[0]), int(h[0])
+
     def set_spring_tables(self, mode=-1):
         """Per-spring tables in shared memory: -1 when they fit (default), 0
         off (direct gathers from both endpoints), 1 on (``cls_set_spring_tables``)."""

@@ -276,6 +276,8 @@ class SimBase {
   virtual void set_launch_shape(int threads, int ctas, int wsh) = 0;
   virtual void launch_shape(int* threads, int* ctas, int* wsh) const = 0;
   virtual void autotune(int steps, int repeats, std::vector<cls_launch_shape>& table) = 0;
+  virtual void set_clusters(int size, int heavy) = 0;
+  virtual void clusters(int* size, int* heavy) const = 0;
   virtual void set_spring_tables(int mode) = 0;
   virtual bool spring_tables() const = 0;
 };
@@ -790,15 +792,18 @@ class SimImpl final : public SimBase {
                   "the controller (" + std::to_string(ctrl) + " bytes) does not fit in shared memory "
                   "beside the kernels' own");
       const bool on = wsh == 1 || (wsh == -1 && r_on >= 1 && r_on >= r_off);
+      std::vector<ClusterPlan> plans = plan_clusters(optin);
+      check_forced(plans, force_size_);
       fwd_smem_ = fwd_base_ + (on ? ctrl : 0);
       rev_smem_ = rev0 + (on ? ctrl : 0);
       resident_ = on ? r_on : r_off;
       wsh_on_ = on;
-      plan_clusters(optin);
+      plans_.swap(plans);
     } catch (...) {
       threads_ = keep;
       throw;
     }
+    choose_splits();
   }
 
   // Shared-memory plans of the cluster-per-env kernels for clusters of 2, 4, 8 and
@@ -809,10 +814,9 @@ class SimImpl final : public SimBase {
     ClusterCaps cap{};
     size_t fwd_smem = 0, rev_smem = 0;
   };
-  void plan_clusters(int optin) {
-    plans_.clear();
-    batch_split_ = serve_rev_ = Split{};
-    if (threads_ > ClusterLaunch<R>::max_threads()) return;
+  std::vector<ClusterPlan> plan_clusters(int optin) const {
+    std::vector<ClusterPlan> plans;
+    if (threads_ > ClusterLaunch<R>::max_threads()) return plans;
     size_t fwd_max = 0, rev_max = 0;
     CLS_CUDA(ClusterLaunch<R>::setup(optin, &fwd_max, &rev_max));
     for (int C : {2, 4, 8, 16}) {
@@ -849,10 +853,38 @@ class SimImpl final : public SimBase {
         continue;
       }
       CLS_CUDA(e);
-      if (p.resident > 0) plans_.push_back(p);
+      if (p.resident > 0) plans.push_back(p);
     }
+    return plans;
+  }
+  // choices made once for all envs of the handle
+  void choose_splits() {
     batch_split_ = split_envs(order_host_.data(), E_);
     serve_rev_ = split_envs(order_host_.data(), E_, false);
+  }
+
+  // Clusters as the caller wants them (cls_set_clusters): -1 the estimate below, 1
+  // single CTAs, else the `heavy` heaviest envs of every launch (0: all) on clusters
+  // of that size.
+  static void check_forced(const std::vector<ClusterPlan>& plans, int size) {
+    bool ok = size <= 1;
+    for (const ClusterPlan& p : plans) ok = ok || p.size == size;
+    CLS_REQUIRE(ok, "no cluster of " + std::to_string(size) + " CTAs of this launch shape can take the largest robot");
+  }
+  void set_clusters(int size, int heavy) override {
+    CLS_REQUIRE(!capturing_, "the clusters cannot change during graph capture");
+    CLS_REQUIRE(size == -1 || size == 1 || size == 2 || size == 4 || size == 8 || size == 16,
+                "the cluster size is -1 (automatic), 1, 2, 4, 8 or 16");
+    CLS_REQUIRE(heavy >= 0, "the number of envs on clusters must not be negative");
+    check_forced(plans_, size);
+    force_size_ = size;
+    force_heavy_ = heavy;
+    choose_splits();
+  }
+  void clusters(int* size, int* heavy) const override {
+    const Split sp = dense_ ? Split{} : batch_split_;
+    *size = sp.heavy ? plans_[sp.plan].size : 1;
+    *heavy = sp.heavy;
   }
 
   // Which of the envs `ies` (heaviest first) of a launch run as one cluster each,
@@ -874,20 +906,18 @@ class SimImpl final : public SimBase {
   // on clusters of 2; with 512 such lattices 16.1 and 17.7, 18.8 (the weights'
   // stream keeps every SM busy there: more than 3 envs per SM are not considered).
   struct Split {
-    const ClusterPlan* plan = nullptr;
-    int heavy = 0;
+    int plan = 0;    // of plans_
+    int heavy = 0;   // 0: single CTAs
   };
   // mixed: the second form too, else all of the envs or none.
   Split split_envs(const int* ies, int n, bool mixed = true) const {
-#ifdef CLS_CLUSTER_SIZE
-    for (const ClusterPlan& p : plans_)
-      if (p.size == CLS_CLUSTER_SIZE) return {&p, n};
-    return {};
-#endif
-#ifdef CLS_SPLIT
-    for (const ClusterPlan& p : plans_)
-      if (p.size == 4) return {&p, std::min(n, CLS_SPLIT)};
-#endif
+    if (force_size_ == 1) return {};
+    if (force_size_ > 1) {
+      const int heavy = force_heavy_ ? std::min(force_heavy_, n) : n;
+      if (!mixed && heavy < n) return {};
+      for (size_t k = 0; k < plans_.size(); ++k)
+        if (plans_[k].size == force_size_) return {(int)k, heavy};
+    }
     if (plans_.empty() || n > 3 * n_sm_) return {};
     constexpr double kOne = 1.45e5, kShare = 1.35;
     auto cluster_fixed = [](int size) { return size > 8 ? 1.9e5 : 1.64e5; };
@@ -908,30 +938,31 @@ class SimImpl final : public SimBase {
     free_at.assign((size_t)n_sm_, 0.0);
     const double single = last_done(0, kOne, 1.0);
     double t = single;
-    for (const ClusterPlan& p : plans_) {
-      if (n > 2 * n_sm_) break;
+    for (size_t k = 0; k < plans_.size() && n <= 2 * n_sm_; ++k) {
+      const ClusterPlan& p = plans_[k];
       free_at.assign((size_t)p.resident, 0.0);
       const double tp = last_done(0, cluster_fixed(p.size), kShare / p.size);
       if (tp < t) {
         t = tp;
-        best = {&p, n};
+        best = {(int)k, n};
       }
     }
-    for (const ClusterPlan& p : plans_)
-      for (int q = 1; mixed && q <= 8; ++q) {
+    for (size_t k = 0; mixed && k < plans_.size(); ++k)
+      for (int q = 1; q <= 8; ++q) {
+        const ClusterPlan& p = plans_[k];
         const int heavy = p.resident * q / 8;
         if (heavy < 1 || heavy >= n || heavy * p.size > n_sm_) continue;
         free_at.assign((size_t)(n_sm_ - heavy * p.size), 0.0);
         double done = 0;
-        for (int k = 0; k < heavy; ++k) {
-          const double tk = cluster_fixed(p.size) + kShare / p.size * cost_[ies[k]];
+        for (int i = 0; i < heavy; ++i) {
+          const double tk = cluster_fixed(p.size) + kShare / p.size * cost_[ies[i]];
           free_at.insert(free_at.end(), p.size, tk);
           done = std::max(done, tk);
         }
         done = std::max(done, last_done(heavy, kOne, 1.0));
         if (done < t && done < 0.93 * single) {
           t = done;
-          best = {&p, heavy};
+          best = {(int)k, heavy};
         }
       }
     return best;
@@ -966,7 +997,7 @@ class SimImpl final : public SimBase {
   // last (ms_forward_kernel, ms_reverse_kernel).
   void launch_fwd(const MsArgs<R>& a, const Split& sp, int grid, int t0, int t1, int mode, int src) {
     launch_split(a, sp, grid, [&](const MsArgs<R>& h) {
-      const ClusterPlan* p = sp.plan;
+      const ClusterPlan* p = &plans_[sp.plan];
       return ClusterLaunch<R>::forward(h, p->cap, p->size, threads_, p->fwd_smem, stream, t0, t1, mode, src);
     }, [&](const cudaLaunchConfig_t& c, const MsArgs<R>& l) {
       return cudaLaunchKernelEx(&c, fwd_fn(), l, t0, t1, mode, src);
@@ -974,7 +1005,7 @@ class SimImpl final : public SimBase {
   }
   void launch_rev(const MsArgs<R>& a, const Split& sp, int grid, int t0, int t1, int last) {
     launch_split(a, sp, grid, [&](const MsArgs<R>& h) {
-      const ClusterPlan* p = sp.plan;
+      const ClusterPlan* p = &plans_[sp.plan];
       return ClusterLaunch<R>::reverse(h, p->cap, p->size, threads_, p->rev_smem, stream, t0, t1, last);
     }, [&](const cudaLaunchConfig_t& c, const MsArgs<R>& l) {
       return cudaLaunchKernelEx(&c, rev_fn(), l, t0, t1, last);
@@ -982,7 +1013,7 @@ class SimImpl final : public SimBase {
   }
   template <typename Heavy, typename Light>
   void launch_split(const MsArgs<R>& a, const Split& sp, int grid, Heavy heavy, Light light, size_t smem) {
-    const int nh = sp.plan ? std::min(sp.heavy, a.n_items) : 0;
+    const int nh = std::min(sp.heavy, a.n_items);
     MsArgs<R> part = a;
     if (nh) {
       part.n_items = nh;
@@ -2329,7 +2360,7 @@ class SimImpl final : public SimBase {
     const Split split = split_envs(serve_order_h_.data(), n);
     timed(PK_RECOMP, [&] { launch_fwd(a, split, grid_for(n), 0, 0, FWD_RECORD, 0); });
     a.queue = d_squeue_.p + 1;
-    timed(PK_REV, [&] { launch_rev(a, Split{serve_rev_.plan, n}, grid_for(n), 0, 0, 0); });
+    timed(PK_REV, [&] { launch_rev(a, Split{serve_rev_.plan, serve_rev_.heavy ? n : 0}, grid_for(n), 0, 0, 0); });
     if (!tiles.empty()) {
       unsigned char *h, *d;
       int slot;
@@ -2534,6 +2565,7 @@ class SimImpl final : public SimBase {
   // sums in another order on each, and a request's gradients must not depend on
   // which others share its window.  All slots on clusters of one size, or none.
   Split serve_rev_;
+  int force_size_ = -1, force_heavy_ = 0;  // set_clusters
   std::vector<int> perm_, user_voff_, env_robot_, order_host_;
   bool identity_perm_ = true;
   std::vector<EnvDesc> ed_host_;
@@ -3077,6 +3109,19 @@ int cls_get_launch_shape(const cls_sim* sim, int32_t* threads_per_block, int32_t
   *threads_per_block = t;
   *ctas_per_sm = c;
   if (weights_shared) *weights_shared = w;
+  return CLS_OK;
+}
+
+int cls_set_clusters(cls_sim* sim, int32_t size, int32_t heavy) {
+  return guarded(sim, [&](cls::SimBase& s) { s.set_clusters(size, heavy); });
+}
+
+int cls_get_clusters(const cls_sim* sim, int32_t* size, int32_t* heavy) {
+  if (!sim || !sim->impl || !size || !heavy) return CLS_ERR_INVALID;
+  int c = 0, h = 0;
+  sim->impl->clusters(&c, &h);
+  *size = c;
+  *heavy = h;
   return CLS_OK;
 }
 

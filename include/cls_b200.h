@@ -297,6 +297,17 @@ int cls_set_launch_shape(cls_sim* sim, int32_t threads_per_block, int32_t ctas_p
 int cls_get_launch_shape(const cls_sim* sim, int32_t* threads_per_block, int32_t* ctas_per_sm,
                          int32_t* weights_shared);
 
+/* Which envs of the fused path run as thread-block clusters: size -1 (the default at
+ * creation) chooses for every launch, 1 runs every env on one CTA, 2, 4, 8 or 16 runs
+ * the `heavy` heaviest envs of every launch (0: all of them) on clusters of that many
+ * CTAs, the others on one each (CLS_ERR_INVALID when the device cannot hold such a
+ * cluster with the largest robot's share; the previous choice stays).  Launches per env
+ * and the batched controller's path use no clusters.  cls_get_clusters: what a launch
+ * over the whole batch takes (size 1, heavy 0: no clusters).  A CUDA graph captured
+ * earlier keeps its choice.  No reference counterpart. */
+int cls_set_clusters(cls_sim* sim, int32_t size, int32_t heavy);
+int cls_get_clusters(const cls_sim* sim, int32_t* size, int32_t* heavy);
+
 /* Per-spring tables of the fused single-CTA kernels and, in FP32, the batched
  * step kernels: each spring's impulse (forward) and adjoint terms (reverse)
  * evaluated once into shared memory and summed by a thread per vertex, instead of
