@@ -55,6 +55,40 @@ __device__ __forceinline__ unsigned long long policy_evict_last() {
   return p;
 }
 
+// Thread-block clusters (a launch without the attribute is a cluster of one).
+namespace cl {
+__device__ __forceinline__ unsigned rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned size() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+// all threads of all CTAs of the cluster; orders their shared-memory accesses
+__device__ __forceinline__ void arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void sync() {
+  arrive();
+  wait();
+}
+// the same shared-memory variable of CTA `r` of the cluster
+template <typename T>
+__device__ __forceinline__ T* peer(T* p, int r) {
+  T* q;
+  asm volatile("mapa.u64 %0, %1, %2;" : "=l"(q) : "l"(p), "r"(r));
+  return q;
+}
+}  // namespace cl
+
 // Programmatic dependent launch: lets the next launch of the stream start its
 // prologue, and waits until the launches before this one have finished (no effect
 // in launches without the attribute).

@@ -35,36 +35,6 @@ constexpr int kClusterMaxThreads = 512;
 
 namespace cl {
 
-__device__ __forceinline__ unsigned rank() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ unsigned size() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
-}
-// all threads of all CTAs of the cluster; orders their shared-memory accesses
-__device__ __forceinline__ void arrive() {
-  __syncwarp();
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void wait() {
-  __syncwarp();
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void sync() {
-  arrive();
-  wait();
-}
-// the same shared-memory variable of CTA `r` of the cluster
-template <typename T>
-__device__ __forceinline__ T* peer(T* p, int r) {
-  T* q;
-  asm volatile("mapa.u64 %0, %1, %2;" : "=l"(q) : "l"(p), "r"(r));
-  return q;
-}
 __device__ __forceinline__ void copy16(void* dst_shared, const void* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst_shared);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");

@@ -987,7 +987,8 @@ class SimImpl final : public SimBase {
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     c.attrs = &at;
     c.numAttrs = C > 1 ? 1 : 0;
-    CLS_CUDA(cudaLaunchKernelEx(&c, ms_wgrad_kernel<R>, a, tiles, kseg, d_gw_.p, d_gb_.p));
+    auto fn = C > 1 ? ms_wgrad_kernel<R, true> : ms_wgrad_kernel<R, false>;
+    CLS_CUDA(cudaLaunchKernelEx(&c, fn, a, tiles, kseg, d_gw_.p, d_gb_.p));
   }
 
   // forward / reverse launches of the fused path over a.n_items envs: the heaviest
@@ -2369,7 +2370,7 @@ class SimImpl final : public SimBase {
       CLS_CUDA(stage_.upload(slot, sizeof(GemmTile) * tiles.size(), stream));
       const GemmTile* dt = reinterpret_cast<const GemmTile*>(d);
       timed(PK_WGRAD, [&] {
-        ms_wgrad_kernel<R><<<(int)tiles.size(), 256, 0, stream>>>(a, dt, 0, d_gw_.p, d_gb_.p);
+        ms_wgrad_kernel<R, false><<<(int)tiles.size(), 256, 0, stream>>>(a, dt, 0, d_gw_.p, d_gb_.p);
       });
     }
     CLS_CUDA(cudaGetLastError());

@@ -1194,29 +1194,26 @@ __global__ void ms_loss_kernel(MsArgs<R> a, double* out, const int* envs) {
 // dW_l[i, j] += sum over rows rho = (substep k of the segment, env of the type)
 //   dz_l[rho, i] * a_l[rho, j]
 // with a_0 the compact input record and a_l = act(z_{l-1} + b_{l-1}).  One CTA
-// computes a 64 x 64 tile; 256 threads, 4 x 4 outputs each.  Launched with
+// computes a 64 x 64 tile; 256 threads, 4 x 4 outputs each.  CLUSTER: launched with
 // clusters of C CTAs, a tile's rows are split over its cluster and the partial
 // tiles summed in rank order through distributed shared memory (the same result
 // every run, unlike atomics): a batch that shares one controller has a handful of
 // tiles and thousands of rows (32 quadrupeds x 99 substeps: 6 tiles, 0.29 ms with
-// C = 1, 0.06 ms with C = 8).
+// C = 1, 0.06 ms with C = 8).  An instance of its own: the exchange's 8 KB of shared memory cost batches
+// whose tiles need no cluster 2 % (512 lattices, 121 substeps: 2.17 ms, 2.12 without).
 struct GemmTile {
   int robot, layer, i0, j0;
   int split, nsplit;  // split-K: this tile sums rows [rows*split/nsplit, rows*(split+1)/nsplit)
 };
 
-template <typename R>
+template <typename R, bool CLUSTER>
 __global__ void __launch_bounds__(256)
 ms_wgrad_kernel(MsArgs<R> a, const GemmTile* tiles, int kseg, R* gw, R* gb) {
   constexpr int TM = 64, TN = 64, TK = 16;
   static_assert(TK * TM / 4 == 256 && TK * TN / 4 == 256, "one 4-value group per thread and operand");
   __shared__ __align__(32) R sA[TK][TM];
   __shared__ __align__(32) R sB[TK][TN];
-  constexpr int kHalf = TM * TN / 2;      // half a tile, then the tile's bias sums
-  __shared__ R part[kHalf + TM];
-  unsigned C, rank;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(C));
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const unsigned C = CLUSTER ? cl::size() : 1, rank = CLUSTER ? cl::rank() : 0;
   const GemmTile tl = tiles[blockIdx.x / C];
   const RobotDesc& rb = a.robots[tl.robot];
   const int l = tl.layer;
@@ -1295,19 +1292,12 @@ ms_wgrad_kernel(MsArgs<R> a, const GemmTile* tiles, int kseg, R* gw, R* gb) {
   }
   R* W = gw + rb.w_off[l];
   const bool split = tl.nsplit > 1;  // several CTAs add into this tile
-  if (C > 1) {
-    auto sync = [] {
-      __syncwarp();
-      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    };
+  if constexpr (CLUSTER) {
+    constexpr int kHalf = TM * TN / 2;      // half a tile, then the tile's bias sums
+    __shared__ R part[kHalf + TM];
     auto total = [&](int v) {  // of `part` over the cluster
       R s = 0;
-      for (unsigned r = 0; r < C; ++r) {
-        R* o;
-        asm volatile("mapa.u64 %0, %1, %2;" : "=l"(o) : "l"(part + v), "r"(r));
-        s += *o;
-      }
+      for (unsigned r = 0; r < C; ++r) s += *cl::peer(part + v, (int)r);
       return s;
     };
     for (int h = 0; h < 2; ++h) {  // rows 4 ty + 2 h and 4 ty + 2 h + 1 of the tile
@@ -1321,7 +1311,7 @@ ms_wgrad_kernel(MsArgs<R> a, const GemmTile* tiles, int kseg, R* gw, R* gb) {
 #pragma unroll
         for (int p = 0; p < 4; ++p) part[kHalf + ty * 4 + p] = bacc[p];
       }
-      sync();
+      cl::sync();
       for (int v = (int)(kHalf / C * rank) + threadIdx.x; v < (int)(kHalf / C * (rank + 1)); v += 256) {
         const int i = tl.i0 + 4 * (v / TN % 16) + 2 * h + v / TN / 16, j = tl.j0 + v % TN;
         if (i >= M || j >= Ncol) continue;
@@ -1335,7 +1325,7 @@ ms_wgrad_kernel(MsArgs<R> a, const GemmTile* tiles, int kseg, R* gw, R* gb) {
         if (split) atomicAdd(b, s);
         else *b += s;
       }
-      sync();
+      cl::sync();
     }
     return;
   }
