@@ -5,6 +5,7 @@
 
 #include "ms_dense.cuh"
 #include "ms_dense_host.h"
+#include "ms_hubs_host.h"
 
 namespace cls {
 
@@ -46,7 +47,7 @@ long long DenseLaunch<R>::split_floats(int rows, int tile_rows, int k) {
 }
 
 template <typename R>
-cudaError_t DenseLaunch<R>::setup(size_t* fwd_static, size_t* rev_static, int optin) {
+cudaError_t DenseLaunch<R>::setup(bool hubs, size_t* fwd_static, size_t* rev_static, int optin) {
   *fwd_static = *rev_static = 0;
   cudaError_t e = cudaSuccess;
   auto prepare = [&](auto fn, size_t* st) {
@@ -56,10 +57,12 @@ cudaError_t DenseLaunch<R>::setup(size_t* fwd_static, size_t* rev_static, int op
     *st = std::max(*st, fa.sharedSizeBytes);
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((size_t)optin - fa.sharedSizeBytes));
   };
-  prepare(ms_step_fwd_kernel<R, kStepThreads, false>, fwd_static);
-  prepare(ms_step_fwd_kernel<R, kStepThreads, true>, fwd_static);
-  prepare(ms_step_rev_kernel<R, kStepThreads, false>, rev_static);
-  prepare(ms_step_rev_kernel<R, kStepThreads, true>, rev_static);
+  prepare(ms_step_fwd_kernel<R, kStepThreads, TAB_NONE>, fwd_static);
+  prepare(ms_step_fwd_kernel<R, kStepThreads, TAB_ROWS>, fwd_static);
+  if (hubs) prepare(HubKernels<R>::step_fwd(), fwd_static);
+  prepare(ms_step_rev_kernel<R, kStepThreads, TAB_NONE>, rev_static);
+  prepare(ms_step_rev_kernel<R, kStepThreads, TAB_ROWS>, rev_static);
+  if (hubs) prepare(HubKernels<R>::step_rev(), rev_static);
   if constexpr (std::is_same<R, float>::value) {
     const int sm = (int)umma::BulkShape<kDenseTN, kBulkStages>::kSmemBytes;
     for (auto fn : {ms_ctrl_gemm_tc_kernel<0, kDenseTN>, ms_ctrl_gemm_tc_kernel<1, kDenseTN>,
@@ -71,16 +74,18 @@ cudaError_t DenseLaunch<R>::setup(size_t* fwd_static, size_t* rev_static, int op
 }
 
 template <typename R>
-cudaError_t DenseLaunch<R>::step_fwd(const MsArgs<R>& a, int grid, int threads, size_t smem, cudaStream_t s, int t,
+cudaError_t DenseLaunch<R>::step_fwd(const MsArgs<R>& a, bool hubs, int grid, int threads, size_t smem, cudaStream_t s, int t,
                               int t_first, int t_end, int mode, int src_slot, int k_prev, int k_cur) {
-  auto fn = a.imp_cap ? ms_step_fwd_kernel<R, kStepThreads, true> : ms_step_fwd_kernel<R, kStepThreads, false>;
+  auto fn = !a.imp_cap ? ms_step_fwd_kernel<R, kStepThreads, TAB_NONE>
+                       : (hubs ? HubKernels<R>::step_fwd() : ms_step_fwd_kernel<R, kStepThreads, TAB_ROWS>);
   return chain(fn, grid, threads, smem, s, a, t, t_first, t_end, mode, src_slot, k_prev, k_cur);
 }
 
 template <typename R>
-cudaError_t DenseLaunch<R>::step_rev(const MsArgs<R>& a, int grid, int threads, size_t smem, cudaStream_t s, int t_post,
+cudaError_t DenseLaunch<R>::step_rev(const MsArgs<R>& a, bool hubs, int grid, int threads, size_t smem, cudaStream_t s, int t_post,
                               int t_pre, int t_begin, int t_end, int last_seg) {
-  auto fn = a.adj_cap ? ms_step_rev_kernel<R, kStepThreads, true> : ms_step_rev_kernel<R, kStepThreads, false>;
+  auto fn = !a.adj_cap ? ms_step_rev_kernel<R, kStepThreads, TAB_NONE>
+                       : (hubs ? HubKernels<R>::step_rev() : ms_step_rev_kernel<R, kStepThreads, TAB_ROWS>);
   return chain(fn, grid, threads, smem, s, a, t_post, t_pre, t_begin, t_end, last_seg);
 }
 

@@ -27,12 +27,13 @@ struct DenseLaunch {
   static int job_n(int n_tiles, int n_sm);
   // floats of a pre-split operand (rows x k) in tiles of tile_rows rows (FP32)
   static long long split_floats(int rows, int tile_rows, int k);
-  // shared-memory attributes of the step and GEMM kernels; the step kernels'
+  // shared-memory attributes of the step and GEMM kernels (hubs: a robot of the
+  // batch has hub vertices, see kEllRows); the step kernels'
   // static shared bytes are returned for the capacity check
-  static cudaError_t setup(size_t* fwd_static, size_t* rev_static, int optin);
-  static cudaError_t step_fwd(const MsArgs<R>& a, int grid, int threads, size_t smem, cudaStream_t s, int t, int t_first,
+  static cudaError_t setup(bool hubs, size_t* fwd_static, size_t* rev_static, int optin);
+  static cudaError_t step_fwd(const MsArgs<R>& a, bool hubs, int grid, int threads, size_t smem, cudaStream_t s, int t, int t_first,
                        int t_end, int mode, int src_slot, int k_prev, int k_cur);
-  static cudaError_t step_rev(const MsArgs<R>& a, int grid, int threads, size_t smem, cudaStream_t s, int t_post,
+  static cudaError_t step_rev(const MsArgs<R>& a, bool hubs, int grid, int threads, size_t smem, cudaStream_t s, int t_post,
                        int t_pre, int t_begin, int t_end, int last_seg);
   // (FP32 takes the same tiles from `tc`)
   static cudaError_t gemm(const MsArgs<R>& a, bool adjoint, int n_jobs, int job_cols, const DenseJob* jobs,

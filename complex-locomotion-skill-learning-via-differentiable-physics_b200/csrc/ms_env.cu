@@ -45,8 +45,8 @@ ms_env_step_kernel(MsArgs<R> a, int t, int from_ckpt, const R* __restrict__ outs
     const R* o = outs + (size_t)e * out_pitch;
     for (int q = tid; q < rb.n_out; q += nt) s.buf0[q] = o[q];
     __syncthreads();
-    if (s.imp) fwd_post<R, true>(a, rb, ed, s, t - 1, FWD_OBS, 0, s.buf0);
-    else fwd_post<R, false>(a, rb, ed, s, t - 1, FWD_OBS, 0, s.buf0);
+    if (s.imp) fwd_post<R, TAB_ROWS>(a, rb, ed, s, t - 1, FWD_OBS, 0, s.buf0);
+    else fwd_post<R, TAB_NONE>(a, rb, ed, s, t - 1, FWD_OBS, 0, s.buf0);
   }
   R hprev = (t > 0) ? a.obs_height[(size_t)(t - 1) * a.n_envs + e] : R(0);
   load_head_smem<R>(a, rb, ed, s, t, FWD_OBS);

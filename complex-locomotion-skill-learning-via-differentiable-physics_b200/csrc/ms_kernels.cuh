@@ -43,7 +43,7 @@ struct RobotDesc {
   int env_first;                     // envs are sorted by type
   int rot_idx[4];                    // heading vertices for robot 100
   int ell_off, ell_rows;             // per-vertex spring lists for the tables: start (in groups of 8
-                                     // entries), entries per vertex (largest degree)
+                                     // entries), entries per vertex (largest degree but hubs')
 };
 
 // Batched-controller offsets of one robot type, kept out of RobotDesc (which
@@ -160,11 +160,13 @@ struct MsArgs {
   const int* spring_out;             // per spring: MLP output index or -1
   const uint4* inc_ell;              // [vertex][ceil(rows / 8)] groups of 8 incidences, 2 spring + side
                                      // (0: a, 1: b) in 16 bits, 2 n_s where a vertex has fewer (robots
-                                     // with spring tables)
+                                     // with spring tables); of hub k only 2 (n_s + 1 + k) + 1.  Before a
+                                     // robot's rows a group with its number of hubs, behind them the
+                                     // hubs' vertices
   const int4* spr_ab;                // per spring {a, b, MLP output or -1, 0} (spr_off)
   const V4<R>* spr_p;                // per spring {rest length, stiffness, actuation coef, 0}
-  int imp_cap;                       // entries of the shared impulse table, springs + 1 (0: none)
-  int adj_cap;                       // entries of the shared adjoint table, springs + 1 (0: none)
+  int imp_cap;                       // entries of the shared impulse table, springs + 1 + hubs (0: none)
+  int adj_cap;                       // entries of the shared adjoint table, the same (0: none)
   const R* w;                        // compact weights
   const R* bias;
   const R* sin_table;                // [T + 1][n_sin], sin(omega (t) dt + 2 pi j / n_sin)
@@ -550,6 +552,19 @@ __device__ __forceinline__ void advance_vertex(const MsArgs<R>& a, V4<R>& x, V4<
   v.x = nv0; v.y = nv1; v.z = nv2;
 }
 
+// Entries per vertex of the lists that one thread walks, at most: twice the cube
+// lattices' largest degree.  Every thread of a robot walks its longest list, so a
+// vertex with more springs, a hub, is summed by a half-warp into an entry of its own
+// behind the springs', and its list holds that entry alone (600 robots with one vertex of
+// 60 / 92 / 200 springs on single CTAs, 41 substeps and their adjoint: 4.7 / 4.7 / 6.7 ms,
+// without tables 6.0 / 6.3 / 10.0).
+constexpr int kEllRows = 48;
+// Spring tables of a kernel instance: none, without hubs, with hubs.  The hubs'
+// instances are a module of their own (ms_hubs.cu): in one kernel the hubs' sums cost
+// robots without any registers (4096 spiders, 80 substeps: 33.9 -> 34.0 to 34.4 ms),
+// and in one module every process's first handle the time to load them (30 -> 47 ms).
+enum Tables { TAB_NONE = 0, TAB_ROWS = 1, TAB_HUBS = 2 };
+
 // A vertex's list of incidences: the first 24 in registers (loaded together, ahead
 // of the barrier before their use), the rest read as they are needed.
 struct EllRow {
@@ -601,14 +616,44 @@ __device__ __forceinline__ void ell_tree(const EllRow& e, int rows, Add add, R (
   }
 }
 
+// The hubs' sums by half-warps, with gather_vinc_all's lanes and tree, from the
+// springs' entries of a table (all of the CTA's threads; add as in ell_tree) into
+// the hubs': put(entry, s).
+template <typename R, int M, typename Add, typename Put>
+__device__ __forceinline__ void hub_sums(const MsArgs<R>& a, const RobotDesc& rb, Add add, Put put) {
+  const uint4* ell = a.inc_ell + rb.ell_off;
+  const unsigned short* hubs = reinterpret_cast<const unsigned short*>(ell + rb.n_v * ((rb.ell_rows + 7) >> 3));
+  const int n = (int)__ldg(ell - 1).x;
+  const int lane = threadIdx.x & 31, l16 = lane & 15, half = lane >> 4;
+  const int* ptr = a.inc_ptr + rb.ptr_off;
+  __syncthreads();
+  for (int k0 = (threadIdx.x >> 5) * 2; k0 < n; k0 += (blockDim.x >> 5) * 2) {
+    const int k = k0 + half;
+    const int v = k < n ? hubs[k] : 0;
+    R s[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) s[m] = 0;
+    for (int q = k < n ? ptr[v] + l16 : 0, end = k < n ? ptr[v + 1] : 0; q < end; q += 16) {
+      const int4 in = __ldg(a.inc_i + rb.inc_off + q);
+      add((unsigned)(2 * in.z + in.y), s);
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+#pragma unroll
+      for (int m = 0; m < M; ++m) s[m] += __shfl_xor_sync(0xffffffffu, s[m], o);
+    }
+    if (k < n && l16 == 0) put(rb.n_s + 1 + k, s);
+  }
+}
+
 // apply_spring_force and advance_toi with each spring's impulse computed once:
 // phase A evaluates every spring (spring-parallel, a -> b order as both of its
 // incidences do) into imp[], phase B sums each vertex's impulses in
-// gather_vinc_all's order and advances it, one thread per vertex.  For robots
-// whose impulse table fits in shared memory (MsArgs::imp_cap).  The batched step
+// gather_vinc_all's order and advances it, one thread per vertex (hubs: hub_sums).
+// For robots whose impulse table fits in shared memory (MsArgs::imp_cap).  The batched step
 // kernel (4096 spiders: 236 vertices, 1378 springs) is bound by its instructions;
 // the half-warp gather took 7 k of its warp instructions per env, this one 1.5 k.
-template <typename R>
+template <typename R, int TAB>
 __device__ __forceinline__ void springs_table(const MsArgs<R>& a, const RobotDesc& rb, int N, V4<R>* xs, V4<R>* vs,
                                               const R* out, V4<R>* imp, V4<R>* rec) {
   const unsigned long long pol = policy_evict_last();
@@ -644,19 +689,25 @@ __device__ __forceinline__ void springs_table(const MsArgs<R>& a, const RobotDes
   }
   const int rows = rb.ell_rows, groups = (rows + 7) >> 3;
   const uint4* ell = a.inc_ell + rb.ell_off;
+  auto add = [&](unsigned c, R (&u)[3]) {
+    const V4<R> im = imp[c >> 1];
+    const bool plus = c & 1;
+    u[0] += plus ? im.x : -im.x;
+    u[1] += plus ? im.y : -im.y;
+    u[2] += plus ? im.z : -im.z;
+  };
+  if constexpr (TAB == TAB_HUBS)
+    hub_sums<R, 3>(a, rb, add, [&](int entry, const R (&s)[3]) {
+      V4<R> r; r.x = s[0]; r.y = s[1]; r.z = s[2]; r.w = 0;
+      imp[entry] = r;
+    });
   EllRow er;
   if (tid < N) er.load(ell + tid * groups, groups);
   __syncthreads();
   for (int v = tid; v < N; v += nt) {
     if (v != tid) er.load(ell + v * groups, groups);
     R s[3];
-    ell_tree<R, 3, 0, 1>(er, rows, [&](unsigned c, R (&u)[3]) {
-      const V4<R> im = imp[c >> 1];
-      const bool plus = c & 1;
-      u[0] += plus ? im.x : -im.x;
-      u[1] += plus ? im.y : -im.y;
-      u[2] += plus ? im.z : -im.z;
-    }, s);
+    ell_tree<R, 3, 0, 1>(er, rows, add, s);
     V4<R> vi; vi.x = s[0]; vi.y = s[1]; vi.z = s[2]; vi.w = 0;
     if (rec) rec[v] = vi;
     advance_vertex<R>(a, xs[v], vs[v], vi);

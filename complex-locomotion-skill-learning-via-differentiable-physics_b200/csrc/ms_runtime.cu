@@ -22,6 +22,7 @@
 #include "ms_cluster_host.h"
 #include "ms_dense_host.h"
 #include "ms_env_host.h"
+#include "ms_hubs_host.h"
 #include "ms_sched.h"
 #include "ms_segment.cuh"
 
@@ -326,6 +327,7 @@ class SimImpl final : public SimBase {
     nmax_ = 0;
     int p0max = 4, dmax = 4, amax = 4, omax = 4;
     m_off_.assign(nr, std::vector<long long>(L_));
+    std::vector<int> hub_steps(nr, 0);  // half-warp steps over the largest hub's springs
     dd_host_.assign(nr, DenseDesc{});
     for (int r = 0; r < nr; ++r) {
       const HostRobot& h = hr_[r];
@@ -408,16 +410,29 @@ class SimImpl final : public SimBase {
       }
       inc_ptr.push_back(run);
       // the springs per vertex as rows for the tables' sums (robots whose table fits)
+      inc_ell.resize(inc_ell.size() + 8);  // the group of its number of hubs
       d.ell_off = (int)(inc_ell.size() / 8);
       if ((size_t)(h.n_s + 1) * sizeof(V4<R>) <= kImpSmemMax) {
-        for (const std::vector<int>& p : per) d.ell_rows = std::max(d.ell_rows, (int)p.size());
+        std::vector<unsigned short> hubs;
+        for (int i = 0; i < h.n_v; ++i) {
+          if ((int)per[i].size() > kEllRows) {
+            hub_steps[r] = std::max(hub_steps[r], ((int)per[i].size() + 15) / 16);
+            per[i].assign(1, 2 * (h.n_s + 1 + (int)hubs.size()) + 1);
+            hubs.push_back((unsigned short)i);
+          }
+          d.ell_rows = std::max(d.ell_rows, (int)per[i].size());
+        }
         const size_t width = ((size_t)d.ell_rows + 7) / 8 * 8;
         const size_t at = inc_ell.size();
-        CLS_REQUIRE(at / 8 + width * h.n_v / 8 < (1LL << 31), "too many incidences");
+        CLS_REQUIRE(at / 8 + width * h.n_v / 8 + hubs.size() < (1LL << 31), "too many incidences");
         inc_ell.resize(at + width * h.n_v, (unsigned short)(2 * h.n_s));
         for (int i = 0; i < h.n_v; ++i)
           for (size_t p = 0; p < per[i].size(); ++p) inc_ell[at + i * width + p] = (unsigned short)per[i][p];
-        ell_rows_max_ = std::max(ell_rows_max_, d.ell_rows);
+        inc_ell[at - 8] = (unsigned short)hubs.size();
+        inc_ell.insert(inc_ell.end(), hubs.begin(), hubs.end());
+        inc_ell.resize((inc_ell.size() + 7) / 8 * 8);
+        hubs_ = hubs_ || !hubs.empty();
+        table_max_ = std::max(table_max_, h.n_s + 1 + (int)hubs.size());
       }
       for (int s = 0; s < h.n_s; ++s) {
         spring_out.push_back(h.out[s]);
@@ -548,6 +563,9 @@ class SimImpl final : public SimBase {
                      [&](int a, int b) { return cost(a) > cost(b); });
     cost_.resize(E);
     for (int ie = 0; ie < E; ++ie) cost_[ie] = (std::is_same<R, double>::value ? 4 : 1) * cost(ie);
+    hub_cost_.assign(E, 0.0);
+    for (int ie = 0; ie < E; ++ie)
+      hub_cost_[ie] = (std::is_same<R, double>::value ? 4 : 1) * 1.2e4 * std::max(0, hub_steps[ed_host_[ie].robot] - 2);
     inc_ptr_h_ = inc_ptr;
     // launch shape
     smem_p0max_ = p0max;
@@ -557,7 +575,7 @@ class SimImpl final : public SimBase {
     // spring impulses computed once per spring into shared memory when the
     // largest robot's table is small (the forward gathers then read them)
     smax_ = smax;
-    imp_cap_ = table_fits() && ell_rows_max_ <= kEllRowsAuto ? smax + 1 : 0;
+    imp_cap_ = table_fits() ? table_max_ : 0;
     fwd_base_ = fwd_smem_bytes<R>(nmax_, dmax, p0max, imp_cap_);
     int dev = 0;
     CLS_CUDA(cudaGetDevice(&dev));
@@ -724,18 +742,25 @@ class SimImpl final : public SimBase {
   // kernel instances by block size (the register budget follows MAXT)
   using FwdFn = void (*)(MsArgs<R>, int, int, int, int);
   using RevFn = void (*)(MsArgs<R>, int, int, int);
-  template <bool TAB>
+  template <int TAB>
   FwdFn fwd_of() const {
     return threads_ <= 256 ? ms_forward_kernel<R, 256, TAB>
                            : (threads_ <= 512 ? ms_forward_kernel<R, 512, TAB> : ms_forward_kernel<R, 1024, TAB>);
   }
-  template <bool TAB>
+  template <int TAB>
   RevFn rev_of() const {
     return threads_ <= 256 ? ms_reverse_kernel<R, 256, TAB>
                            : (threads_ <= 512 ? ms_reverse_kernel<R, 512, TAB> : ms_reverse_kernel<R, 1024, TAB>);
   }
-  FwdFn fwd_fn() const { return imp_cap_ ? fwd_of<true>() : fwd_of<false>(); }
-  RevFn rev_fn() const { return adj_entries(threads_) ? rev_of<true>() : rev_of<false>(); }
+  FwdFn fwd_fn() const {
+    if (imp_cap_ && hubs_) return HubKernels<R>::forward(threads_);
+    return imp_cap_ ? fwd_of<TAB_ROWS>() : fwd_of<TAB_NONE>();
+  }
+  RevFn rev_fn() const {
+    const bool table = adj_entries(threads_) > 0;
+    if (table && hubs_) return HubKernels<R>::reverse(threads_);
+    return table ? rev_of<TAB_ROWS>() : rev_of<TAB_NONE>();
+  }
   // entries of the fused reverse kernel's adjoint table: none for robots so small
   // that the direct gather's half-warps take their vertices in two rounds (160
   // robots of 44 vertices, 512 threads: reverse 1.29 ms with the table, 1.22 without)
@@ -905,6 +930,10 @@ class SimImpl final : public SimBase {
   // 13.6 ms on single CTAs, 11.5 with the 16 heaviest on clusters of 4, 11.8 with 32
   // on clusters of 2; with 512 such lattices 16.1 and 17.7, 18.8 (the weights'
   // stream keeps every SM busy there: more than 3 envs per SM are not considered).
+  // A hub vertex's springs are one half-warp's, in a cluster evaluated by it too, where
+  // the single CTA reads its tables: 1.25 us per 16 springs (one robot with a vertex of
+  // 92 / 200 / 400 springs, 41 substeps and their adjoint, cluster of 8 1.02 / 1.37 / 2.13
+  // ms, single CTA 0.96 / 1.22 / 1.74).
   struct Split {
     int plan = 0;    // of plans_
     int heavy = 0;   // 0: single CTAs
@@ -922,13 +951,14 @@ class SimImpl final : public SimBase {
     constexpr double kOne = 1.45e5, kShare = 1.35;
     auto cluster_fixed = [](int size) { return size > 8 ? 1.9e5 : 1.64e5; };
     std::vector<double> free_at;  // heap, the next free worker first
+    const bool hubs = imp_cap_ > 0;
     // envs k0.. taken in order by the workers of free_at: when the last is done
-    auto last_done = [&](int k0, double fixed, double per_cost) {
+    auto last_done = [&](int k0, double fixed, double per_cost, bool hub = false) {
       double end = 0;
       std::make_heap(free_at.begin(), free_at.end(), std::greater<double>());
       for (int k = k0; k < n; ++k) {
         std::pop_heap(free_at.begin(), free_at.end(), std::greater<double>());
-        free_at.back() += fixed + per_cost * cost_[ies[k]];
+        free_at.back() += fixed + per_cost * cost_[ies[k]] + (hub ? hub_cost_[ies[k]] : 0.0);
         end = std::max(end, free_at.back());
         std::push_heap(free_at.begin(), free_at.end(), std::greater<double>());
       }
@@ -941,7 +971,7 @@ class SimImpl final : public SimBase {
     for (size_t k = 0; k < plans_.size() && n <= 2 * n_sm_; ++k) {
       const ClusterPlan& p = plans_[k];
       free_at.assign((size_t)p.resident, 0.0);
-      const double tp = last_done(0, cluster_fixed(p.size), kShare / p.size);
+      const double tp = last_done(0, cluster_fixed(p.size), kShare / p.size, hubs);
       if (tp < t) {
         t = tp;
         best = {(int)k, n};
@@ -955,7 +985,7 @@ class SimImpl final : public SimBase {
         free_at.assign((size_t)(n_sm_ - heavy * p.size), 0.0);
         double done = 0;
         for (int i = 0; i < heavy; ++i) {
-          const double tk = cluster_fixed(p.size) + kShare / p.size * cost_[ies[i]];
+          const double tk = cluster_fixed(p.size) + kShare / p.size * cost_[ies[i]] + (hubs ? hub_cost_[ies[i]] : 0.0);
           free_at.insert(free_at.end(), p.size, tk);
           done = std::max(done, tk);
         }
@@ -1045,7 +1075,7 @@ class SimImpl final : public SimBase {
   void set_spring_tables(int mode) override {
     CLS_REQUIRE(!capturing_, "the spring tables cannot change during graph capture");
     CLS_REQUIRE(mode >= -1 && mode <= 1, "spring_tables must be -1 (automatic), 0 or 1");
-    const size_t fit = table_fits() ? (size_t)smax_ + 1 : 0;
+    const size_t fit = table_fits() ? (size_t)table_max_ : 0;
     CLS_REQUIRE(mode != 1 || fit, "the spring tables do not fit in shared memory");
     const size_t keep = imp_cap_;
     auto apply = [&](size_t cap) {
@@ -1059,13 +1089,13 @@ class SimImpl final : public SimBase {
         CLS_CUDA(cudaGetDevice(&dev));
         CLS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
         size_t fwd_static = 0, rev_static = 0;
-        CLS_CUDA(DenseLaunch<R>::setup(&fwd_static, &rev_static, optin));
+        CLS_CUDA(DenseLaunch<R>::setup(hubs_, &fwd_static, &rev_static, optin));
         CLS_REQUIRE(dfwd_smem_ + fwd_static <= (size_t)optin,
                     "robot too large for the batched controller's step kernels");
       }
     };
     try {
-      apply(mode == 0 || (mode < 0 && ell_rows_max_ > kEllRowsAuto) ? 0 : fit);
+      apply(mode == 0 ? 0 : fit);
     } catch (...) {
       try {
         apply(keep);
@@ -1077,9 +1107,6 @@ class SimImpl final : public SimBase {
   }
   bool spring_tables() const override { return imp_cap_ > 0; }
   bool table_fits() const { return (size_t)(smax_ + 1) * sizeof(V4<R>) <= kImpSmemMax; }
-  // a thread walks as many rows as the robot's largest degree: tables by default
-  // only up to twice the cube lattices' (24)
-  static constexpr int kEllRowsAuto = 48;
 
   void set_launch_shape(int threads, int ctas, int wsh) override {
     CLS_REQUIRE(!capturing_, "the launch shape cannot change during graph capture");
@@ -1580,7 +1607,7 @@ class SimImpl final : public SimBase {
     CLS_CUDA(cudaGetDevice(&dev));
     CLS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     size_t fwd_static = 0, rev_static = 0;
-    CLS_CUDA(DenseLaunch<R>::setup(&fwd_static, &rev_static, optin));
+    CLS_CUDA(DenseLaunch<R>::setup(hubs_, &fwd_static, &rev_static, optin));
     CLS_REQUIRE(dfwd_smem_ + fwd_static <= (size_t)optin && drev_smem_ + rev_static <= (size_t)optin,
                 "robot too large for the batched controller's step kernels");
     transpose_weights();
@@ -1621,7 +1648,7 @@ class SimImpl final : public SimBase {
       const int k_prev = t > t_first ? (first_pass ? (t - 1) % K_ : t - 1 - t_first) : 0;
       const int k_cur = t < t_end ? (first_pass ? t % K_ : t - t_first) : 0;
       timed(kind, [&] {
-        CLS_CUDA(DenseLaunch<R>::step_fwd(step_args(a), step_grid(), dense_threads_, dfwd_smem_, stream, t, t_first,
+        CLS_CUDA(DenseLaunch<R>::step_fwd(step_args(a), hubs_, step_grid(), dense_threads_, dfwd_smem_, stream, t, t_first,
                                           t_end, mode, src_slot, k_prev, k_cur));
       });
       if (t < t_end)
@@ -1636,7 +1663,7 @@ class SimImpl final : public SimBase {
       const int t_post = (t + 1 < t1) ? t + 1 : -1;
       const int t_pre = (t >= t0) ? t : -1;
       timed(PK_REV, [&] {
-        CLS_CUDA(DenseLaunch<R>::step_rev(step_args(a), step_grid(), dense_threads_, drev_smem_, stream, t_post, t_pre,
+        CLS_CUDA(DenseLaunch<R>::step_rev(step_args(a), hubs_, step_grid(), dense_threads_, drev_smem_, stream, t_post, t_pre,
                                           t0, t1, last ? 1 : 0));
       });
       if (t_pre >= 0)
@@ -2102,7 +2129,8 @@ class SimImpl final : public SimBase {
     a.b_smem = 0;
     a.live_x = d_livex_.p;
     a.live_v = d_livev_.p;
-    const size_t smem = fwd_smem_bytes<R>(nmax_, smem_dmax_, smem_p0max_, imp_cap_);
+    if (hubs_) a.imp_cap = 0;  // the env step kernel's tables know no hubs
+    const size_t smem = fwd_smem_bytes<R>(nmax_, smem_dmax_, smem_p0max_, a.imp_cap);
     CLS_CUDA(EnvLaunch<R>::step(a, smem, stream, t, outputs ? 0 : 1, outputs ? dout : nullptr, omax, dobs, imax, daux));
     if (!m) {
       CLS_CUDA(cudaMemcpyAsync(hob, dobs, sizeof(R) * n_obs, cudaMemcpyDeviceToHost, stream));
@@ -2558,6 +2586,7 @@ class SimImpl final : public SimBase {
   size_t fwd_smem_ = 0, rev_smem_ = 0, n_queue_ = 0;
   HostMapped mapped_;
   std::vector<double> cost_;       // per env: cost of a substep (processing order, cluster sizes)
+  std::vector<double> hub_cost_;   // per env: what a cluster takes longer for its hub vertices
   std::vector<int> inc_ptr_h_;     // incidence row starts of the robot types
   std::vector<ClusterPlan> plans_;
   Split batch_split_;              // for launches over the whole batch
@@ -2603,7 +2632,8 @@ class SimImpl final : public SimBase {
   size_t imp_cap_ = 0;
   int smax_ = 0;
   static constexpr size_t kImpSmemMax = 48 * 1024 + 32;  // 3072 springs in FP32 and the zero entry
-  int ell_rows_max_ = 0;
+  int table_max_ = 1;  // entries of the largest robot's table
+  bool hubs_ = false;  // a robot has vertices of more than kEllRows springs
   DevBuf<unsigned short> d_inc_ell_;
   DevBuf<V4<R>> d_inc_f_, d_ckx_, d_ckv_, d_finx_, d_finv_, d_recx_, d_recv_, d_recvinc_, d_obsc_, d_xfull_,
       d_tv_, d_init_, d_adjx_, d_adjv_;

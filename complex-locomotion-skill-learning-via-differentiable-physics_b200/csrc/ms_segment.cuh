@@ -334,7 +334,7 @@ __device__ __forceinline__ void fwd_pre(const MsArgs<R>& a, const RobotDesc& rb,
 // tables (MsArgs::imp_cap > 0) or not -- kernel instances of their own, because
 // either form's registers cost the other's products their loads in flight (the
 // uneven batch's first pass 18.9 -> 25.4 ms with both in one kernel).
-template <typename R, bool TAB>
+template <typename R, int TAB>
 __device__ __forceinline__ void fwd_post(const MsArgs<R>& a, const RobotDesc& rb, const EnvDesc& ed,
                                          const FwdSmem<R>& s, int t, int mode, int kslot, const R* out) {
   const int tid = threadIdx.x, nt = blockDim.x;
@@ -345,7 +345,7 @@ __device__ __forceinline__ void fwd_post(const MsArgs<R>& a, const RobotDesc& rb
   }
   V4<R>* rec = (mode & FWD_RECORD) ? a.rec_vinc + (size_t)kslot * a.v_total + ed.v_off : nullptr;
   if constexpr (TAB) {
-    springs_table<R>(a, rb, N, s.xs, s.vs, out, s.imp, rec);
+    springs_table<R, TAB>(a, rb, N, s.xs, s.vs, out, s.imp, rec);
   } else {
     gather_vinc_all<R>(a, rb, N, s.xs, s.vs, out, s.vinc, rec);
     __syncthreads();
@@ -379,7 +379,7 @@ __device__ __forceinline__ void fwd_finish(const MsArgs<R>& a, const RobotDesc& 
 
 // Advances every env from t_begin (state in checkpoint slot src_slot) through
 // t_end (exclusive), i.e. runs pre_advance/nn_input/forward/advance for each t.
-template <typename R, int MAXT, bool TAB>
+template <typename R, int MAXT, int TAB>
 __global__ void __launch_bounds__(MAXT, 1)
 ms_forward_kernel(MsArgs<R> a, int t_begin0, int t_end0, int mode, int src_slot0) {
   extern __shared__ __align__(256) char smem_raw[];
@@ -687,10 +687,10 @@ __device__ __forceinline__ void spring_adjoint_one(const MsArgs<R>& a, const Inc
 // The same with each spring's adjoint evaluated once: phase A (spring-
 // parallel) stores gd and h per spring in adj and adds the actuation gradient,
 // phase B sums each vertex's terms in spring_adjoint_gather's order, one thread
-// per vertex (ell_tree).  For robots whose table fits in shared memory
+// per vertex (ell_tree; hubs: hub_sums).  For robots whose table fits in shared memory
 // (MsArgs::adj_cap).  4096 spiders' reverse step, 2756 incidences per env: the
 // direct gather issues 43.8 k warp instructions per env, this form half of them.
-template <typename R>
+template <typename R, int TAB>
 __device__ __forceinline__ void spring_adjoint_table(const MsArgs<R>& a, const RobotDesc& rb,
                                                      const PairRows<R>& xv, const V4<R>* gvinc, const R* outv,
                                                      R* gout, const PairRows<R>& adj, const PairRows<R>& gs,
@@ -732,23 +732,30 @@ __device__ __forceinline__ void spring_adjoint_table(const MsArgs<R>& a, const R
   }
   const int N = rb.n_v, rows = rb.ell_rows, groups = (rows + 7) >> 3;
   const uint4* ell = a.inc_ell + rb.ell_off;
+  auto add = [&](unsigned c, R (&u)[6]) {
+    V4<R> g, h;
+    adj.get(c >> 1, g, h);
+    const bool minus = c & 1;
+    u[0] += minus ? -g.x : g.x;
+    u[1] += minus ? -g.y : g.y;
+    u[2] += minus ? -g.z : g.z;
+    u[3] += minus ? -h.x : h.x;
+    u[4] += minus ? -h.y : h.y;
+    u[5] += minus ? -h.z : h.z;
+  };
+  if constexpr (TAB == TAB_HUBS)
+    hub_sums<R, 6>(a, rb, add, [&](int entry, const R (&s)[6]) {
+      V4<R> g; g.x = -s[0]; g.y = -s[1]; g.z = -s[2]; g.w = 0;  // the hub's list takes it away
+      V4<R> h; h.x = -s[3]; h.y = -s[4]; h.z = -s[5]; h.w = 0;
+      adj.set(entry, g, h);
+    });
   EllRow er;
   if (tid < N) er.load(ell + tid * groups, groups);
   __syncthreads();
   for (int v = tid; v < N; v += nt) {
     if (v != tid) er.load(ell + v * groups, groups);
     R s[6];
-    ell_tree<R, 6, 0, 1>(er, rows, [&](unsigned c, R (&u)[6]) {
-      V4<R> g, h;
-      adj.get(c >> 1, g, h);
-      const bool minus = c & 1;
-      u[0] += minus ? -g.x : g.x;
-      u[1] += minus ? -g.y : g.y;
-      u[2] += minus ? -g.z : g.z;
-      u[3] += minus ? -h.x : h.x;
-      u[4] += minus ? -h.y : h.y;
-      u[5] += minus ? -h.z : h.z;
-    }, s);
+    ell_tree<R, 6, 0, 1>(er, rows, add, s);
     V4<R> x, w;
     gs.get(v, x, w);
     x.x += s[0]; x.y += s[1]; x.z += s[2];
@@ -872,7 +879,7 @@ __device__ __forceinline__ void advance_adjoint(const MsArgs<R>& a, const V4<R>&
 // Adjoint of substep t up to the controller outputs: x(t), v(t) from the
 // records (slot kslot), advance_toi adjoint, spring-force adjoint, then
 // dz of the output layer (recorded, and left in s.dz).
-template <typename R, bool TAB>
+template <typename R, int TAB>
 __device__ __forceinline__ void rev_pre(const MsArgs<R>& a, const RobotDesc& rb, const EnvDesc& ed,
                                         const RevSmem<R>& s, int e, int t, int kslot) {
   const int tid = threadIdx.x, nt = blockDim.x;
@@ -911,7 +918,7 @@ __device__ __forceinline__ void rev_pre(const MsArgs<R>& a, const RobotDesc& rb,
     const R lim = act_seed ? dpow_half<R>(dabs<R>(a.tv[o].x) / R(0.08)) : R(0);
     const R act_scale = R(10) / R(st_e) / Br / R(rb.n_s);
     if constexpr (TAB)
-      spring_adjoint_table<R>(a, rb, s.xv, s.gvinc, s.bufA, s.bufB, s.adj, s.g, act_scale, lim, act_seed);
+      spring_adjoint_table<R, TAB>(a, rb, s.xv, s.gvinc, s.bufA, s.bufB, s.adj, s.g, act_scale, lim, act_seed);
     else
       spring_adjoint_gather<R>(a, rb, s.xv, s.gvinc, s.bufA, s.bufB, s.g, act_scale, lim, act_seed);
   }
@@ -1027,7 +1034,7 @@ __device__ __forceinline__ void rev_store_carry(const MsArgs<R>& a, const RobotD
   __syncthreads();
 }
 
-template <typename R, int MAXT, bool TAB>
+template <typename R, int MAXT, int TAB>
 __global__ void __launch_bounds__(MAXT, 1)
 ms_reverse_kernel(MsArgs<R> a, int t_begin0, int t_end0, int last_seg0) {
   extern __shared__ __align__(256) char smem_raw[];
@@ -1199,8 +1206,9 @@ __global__ void ms_loss_kernel(MsArgs<R> a, double* out, const int* envs) {
 // tiles summed in rank order through distributed shared memory (the same result
 // every run, unlike atomics): a batch that shares one controller has a handful of
 // tiles and thousands of rows (32 quadrupeds x 99 substeps: 6 tiles, 0.29 ms with
-// C = 1, 0.06 ms with C = 8).  An instance of its own: the exchange's 8 KB of shared memory cost batches
-// whose tiles need no cluster 2 % (512 lattices, 121 substeps: 2.17 ms, 2.12 without).
+// C = 1, 0.06 ms with C = 8).  An instance of its own: the exchange's 8 KB of shared
+// memory cost batches whose tiles need no cluster 2 % (512 lattices, 121 substeps:
+// 2.17 ms, 2.12 without).
 struct GemmTile {
   int robot, layer, i0, j0;
   int split, nsplit;  // split-K: this tile sums rows [rows*split/nsplit, rows*(split+1)/nsplit)
