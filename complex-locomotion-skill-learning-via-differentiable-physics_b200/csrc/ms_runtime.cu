@@ -765,10 +765,26 @@ class SimImpl final : public SimBase {
   // that the direct gather's half-warps take their vertices in two rounds (160
   // robots of 44 vertices, 512 threads: reverse 1.29 ms with the table, 1.22 without)
   size_t adj_entries(int threads) const { return 8 * nmax_ > threads ? imp_cap_ : 0; }
-  // the batched step kernels' tables: FP32 only (300 FP64 robots of 44 vertices:
-  // forward + reverse 3.8 ms with tables, 2.7 without)
-  size_t dense_entries() const { return std::is_same<R, float>::value ? imp_cap_ : 0; }
-
+  // Shared memory of the batched step kernels: tables as the fused kernels have them,
+  // where they fit beside the rest (a caller's small blocks leave the fused kernels
+  // more room), and in FP64 only on demand (300 FP64 robots of 44 vertices: forward +
+  // reverse 3.8 ms with tables, 2.7 without).
+  void size_dense() {
+    int dev = 0, optin = 0;
+    CLS_CUDA(cudaGetDevice(&dev));
+    CLS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    size_t fwd_static = 0, rev_static = 0;
+    CLS_CUDA(DenseLaunch<R>::setup(hubs_, &fwd_static, &rev_static, optin));
+    auto fits = [&](size_t entries) {
+      dense_entries_ = entries;
+      dfwd_smem_ = fwd_smem_bytes<R>(nmax_, smem_omax_, smem_p0max_, entries);
+      drev_smem_ = rev_smem_bytes<R>(nmax_, smem_amax_, smem_omax_, smem_omax_, dense_threads_, entries);
+      return dfwd_smem_ + fwd_static <= (size_t)optin && drev_smem_ + rev_static <= (size_t)optin;
+    };
+    const bool wanted = std::is_same<R, float>::value || tables_forced_;
+    CLS_REQUIRE((wanted && fits(imp_cap_)) || fits(0),
+                "robot too large for the batched controller's step kernels");
+  }
 
   // Launch shape of the fused kernels: threads per CTA select the kernel
   // instance; its dynamic shared-memory limit is raised, the largest robot
@@ -1082,22 +1098,15 @@ class SimImpl final : public SimBase {
       imp_cap_ = cap;
       fwd_base_ = fwd_smem_bytes<R>(nmax_, smem_dmax_, smem_p0max_, imp_cap_);
       use_shape(threads_, wsh_on_ ? 1 : 0);
-      if (d_wt_.p) {  // the batched step kernels carve with the same table
-        dfwd_smem_ = fwd_smem_bytes<R>(nmax_, smem_omax_, smem_p0max_, dense_entries());
-        drev_smem_ = rev_smem_bytes<R>(nmax_, smem_amax_, smem_omax_, smem_omax_, dense_threads_, dense_entries());
-        int dev = 0, optin = 0;
-        CLS_CUDA(cudaGetDevice(&dev));
-        CLS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        size_t fwd_static = 0, rev_static = 0;
-        CLS_CUDA(DenseLaunch<R>::setup(hubs_, &fwd_static, &rev_static, optin));
-        CLS_REQUIRE(dfwd_smem_ + fwd_static <= (size_t)optin,
-                    "robot too large for the batched controller's step kernels");
-      }
+      if (d_wt_.p) size_dense();
     };
+    const bool keep_forced = tables_forced_;
     try {
+      tables_forced_ = mode == 1;
       apply(mode == 0 ? 0 : fit);
     } catch (...) {
       try {
+        tables_forced_ = keep_forced;
         apply(keep);
       } catch (...) {
       }
@@ -1105,7 +1114,7 @@ class SimImpl final : public SimBase {
     }
     fwd_done_ = bwd_done_ = false;
   }
-  bool spring_tables() const override { return imp_cap_ > 0; }
+  bool spring_tables() const override { return (dense_ ? dense_entries_ : imp_cap_) > 0; }
   bool table_fits() const { return (size_t)(smax_ + 1) * sizeof(V4<R>) <= kImpSmemMax; }
 
   void set_launch_shape(int threads, int ctas, int wsh) override {
@@ -1454,6 +1463,12 @@ class SimImpl final : public SimBase {
 
   void enable_dense() {
     constexpr bool f32 = std::is_same<R, float>::value;
+    // step kernels: one CTA per env, a thread per vertex up to kStepThreads (FP64:
+    // 128, its 180 registers leave no second CTA of 256); per
+    // CTA the fused kernels' shared-memory carve with the controller buffers
+    // sized for the output layer only (step_args)
+    dense_threads_ = std::min(f32 ? kStepThreads : 128, std::max(128, (nmax_ + 31) / 32 * 32));
+    size_dense();
     const int tm = DenseLaunch<R>::tile_m(), tn = DenseLaunch<R>::tile_n();
     jobs_h_.clear();
     // a layer's tiles, all types: `off`, `cnt` and the columns of each (`jn`)
@@ -1596,20 +1611,6 @@ class SimImpl final : public SimBase {
     }
     d_dense_.alloc(std::max<size_t>(1, dd_host_.size()));
     CLS_CUDA(cudaMemcpy(d_dense_.p, dd_host_.data(), sizeof(DenseDesc) * dd_host_.size(), cudaMemcpyHostToDevice));
-    // step kernels: one CTA per env, a thread per vertex up to kStepThreads (FP64:
-    // 128, its 180 registers leave no second CTA of 256); per
-    // CTA the fused kernels' shared-memory carve with the controller buffers
-    // sized for the output layer only (step_args)
-    dense_threads_ = std::min(f32 ? kStepThreads : 128, std::max(128, (nmax_ + 31) / 32 * 32));
-    dfwd_smem_ = fwd_smem_bytes<R>(nmax_, smem_omax_, smem_p0max_, dense_entries());
-    drev_smem_ = rev_smem_bytes<R>(nmax_, smem_amax_, smem_omax_, smem_omax_, dense_threads_, dense_entries());
-    int dev = 0, optin = 0;
-    CLS_CUDA(cudaGetDevice(&dev));
-    CLS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    size_t fwd_static = 0, rev_static = 0;
-    CLS_CUDA(DenseLaunch<R>::setup(hubs_, &fwd_static, &rev_static, optin));
-    CLS_REQUIRE(dfwd_smem_ + fwd_static <= (size_t)optin && drev_smem_ + rev_static <= (size_t)optin,
-                "robot too large for the batched controller's step kernels");
     transpose_weights();
     CLS_CUDA(cudaStreamSynchronize(stream));
   }
@@ -1620,7 +1621,7 @@ class SimImpl final : public SimBase {
     MsArgs<R> b = a;
     b.smem_dmax = smem_omax_;
     b.w_smem = b.b_smem = 0;  // the step kernels read the controller from its GEMM tiles
-    b.imp_cap = b.adj_cap = (int)dense_entries();
+    b.imp_cap = b.adj_cap = (int)dense_entries_;
     b.n_items = E_;
     return b;
   }
@@ -2633,6 +2634,8 @@ class SimImpl final : public SimBase {
   int smax_ = 0;
   static constexpr size_t kImpSmemMax = 48 * 1024 + 32;  // 3072 springs in FP32 and the zero entry
   int table_max_ = 1;  // entries of the largest robot's table
+  bool tables_forced_ = false;  // set_spring_tables(1)
+  size_t dense_entries_ = 0;    // of the batched step kernels' tables
   bool hubs_ = false;  // a robot has vertices of more than kEllRows springs
   DevBuf<unsigned short> d_inc_ell_;
   DevBuf<V4<R>> d_inc_f_, d_ckx_, d_ckv_, d_finx_, d_finv_, d_recx_, d_recv_, d_recvinc_, d_obsc_, d_xfull_,

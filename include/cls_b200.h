@@ -308,14 +308,15 @@ int cls_get_launch_shape(const cls_sim* sim, int32_t* threads_per_block, int32_t
 int cls_set_clusters(cls_sim* sim, int32_t size, int32_t heavy);
 int cls_get_clusters(const cls_sim* sim, int32_t* size, int32_t* heavy);
 
-/* Per-spring tables of the fused single-CTA kernels and, in FP32, the batched
- * step kernels: each spring's impulse (forward) and adjoint terms (reverse)
+/* Per-spring tables of the fused single-CTA kernels and the batched step kernels
+ * (in FP64 there only with mode 1): each spring's impulse (forward) and adjoint terms (reverse)
  * evaluated once into shared memory and summed by a thread per vertex (a vertex of
  * more than 48 springs: by a half-warp), instead of evaluated from both of its
  * endpoints.  mode -1 (the default at creation): on when the largest robot's table
  * fits (<= 3072 springs in FP32); 0 off; 1 on (CLS_ERR_INVALID when it does not
  * fit).  The same results (each spring is evaluated in the same argument order
- * either way and gathered in the same order).  No reference counterpart. */
+ * either way and gathered in the same order).  cls_spring_tables: whether the kernels
+ * of the controller path in use have them.  No reference counterpart. */
 int cls_set_spring_tables(cls_sim* sim, int32_t mode);
 int cls_spring_tables(const cls_sim* sim, int32_t* on);
 
