@@ -465,8 +465,9 @@ ms_forward_kernel(MsArgs<R> a, int t_begin0, int t_end0, int mode, int src_slot0
     }
     fwd_finish<R>(a, rb, ed, s, t_begin, t_end, mode);
   }
-  // a cluster launch beside this one (launch_fwd) ends before this launch does
-  dependents_wait();
+  // a cluster launch beside this one (launch_fwd) ends before this launch does: one
+  // CTA waits for it, the others leave their SMs when they are out of work
+  if (blockIdx.x == 0) dependents_wait();
 }
 
 // -------------------------------------------------------------- loss seeds
@@ -1095,7 +1096,7 @@ ms_reverse_kernel(MsArgs<R> a, int t_begin0, int t_end0, int last_seg0) {
     }
     rev_store_carry<R>(a, rb, ed, s, e, hcarry);
   }
-  dependents_wait();  // as in the forward kernel
+  if (blockIdx.x == 0) dependents_wait();  // as in the forward kernel
 }
 
 // ------------------------------------------------------------------ losses
