@@ -96,8 +96,10 @@ template <typename R>
 cudaError_t EnvLaunch<R>::step(const MsArgs<R>& a, size_t smem, cudaStream_t s, int t, int from_ckpt,
                                const R* outs, int out_pitch, R* obs, int obs_pitch, R* aux) {
   auto fn = ms_env_step_kernel<R>;
-  // above the default limit the attribute is set on every call (it is per kernel
-  // and process, and handles differ); the queries cost more than the launch
+  // above the default limit the attribute is set on every call, to the device's
+  // maximum: it is per kernel and process, and a smaller handle's call on another
+  // thread must not lower it before this launch.  (Not for small robots: the queries
+  // cost more than the launch.)
   if (smem > 40 * 1024) {
     int dev = 0, optin = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -106,7 +108,7 @@ cudaError_t EnvLaunch<R>::step(const MsArgs<R>& a, size_t smem, cudaStream_t s, 
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fn);
     if (e != cudaSuccess) return e;
     if (smem + fa.sharedSizeBytes > (size_t)optin) return cudaErrorInvalidConfiguration;
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
     if (e != cudaSuccess) return e;
   }
   fn<<<a.n_envs, kEnvThreads, smem, s>>>(a, t, from_ckpt, outs, out_pitch, obs, obs_pitch, aux);
