@@ -322,14 +322,28 @@ class MpmImpl final : public MpmBase {
     MPM_CUDA(prof_.run(kind, stream, std::forward<F>(f)));
   }
 
+  // The limit belongs to a kernel in the whole process: raised to the device's
+  // maximum, so that a handle with smaller tiles, or none, never lowers it for others.
+  template <typename Fn>
+  static void raise_smem(Fn fn, size_t need) {
+    if (need == 0) return;
+    int dev = 0, optin = 0;
+    cudaFuncAttributes fa{};
+    MPM_CUDA(cudaGetDevice(&dev));
+    MPM_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    MPM_CUDA(cudaFuncGetAttributes(&fa, fn));
+    const size_t most = (size_t)optin - fa.sharedSizeBytes;
+    MPM_CUDA(need > most ? cudaErrorInvalidValue : cudaSuccess);
+    MPM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+  }
   template <int SM>
   void set_smem_attrs() {
-    MPM_CUDA(cudaFuncSetAttribute(mpm_fwd_kernel<R, D, 1, SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem_));
-    MPM_CUDA(cudaFuncSetAttribute(mpm_fwd_kernel<R, D, 2, SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem_));
-    MPM_CUDA(cudaFuncSetAttribute(mpm_fwd_kernel<R, D, 3, SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem_));
-    MPM_CUDA(cudaFuncSetAttribute(mpm_adj_kernel<R, D, 1, SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adj_smem_));
-    MPM_CUDA(cudaFuncSetAttribute(mpm_adj_kernel<R, D, 2, SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adj_smem_));
-    MPM_CUDA(cudaFuncSetAttribute(mpm_adj_kernel<R, D, 3, SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adj_smem_));
+    raise_smem(mpm_fwd_kernel<R, D, 1, SM>, fwd_smem_);
+    raise_smem(mpm_fwd_kernel<R, D, 2, SM>, fwd_smem_);
+    raise_smem(mpm_fwd_kernel<R, D, 3, SM>, fwd_smem_);
+    raise_smem(mpm_adj_kernel<R, D, 1, SM>, adj_smem_);
+    raise_smem(mpm_adj_kernel<R, D, 2, SM>, adj_smem_);
+    raise_smem(mpm_adj_kernel<R, D, 3, SM>, adj_smem_);
   }
   template <int SM>
   void fwd_t(int mode, const FwdArgs<R>& a) {
