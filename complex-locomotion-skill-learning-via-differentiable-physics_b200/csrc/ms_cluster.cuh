@@ -22,7 +22,8 @@
 // 50-1974 vertices, 90 substeps over four segments, first pass 10.3 -> 2.3 ms,
 // recompute 4.3 -> 0.85, reverse 12.1 -> 3.5; one quadruped, 101 substeps, 0.91
 // -> 0.64 ms.  What bounds a small robot now is the instruction count of each
-// phase (about 1 k per warp and substep) and 3-5 cluster barriers of ~0.5 us.
+// phase (about 1 k per warp and substep) and, with L layers, L + 1 cluster barriers
+// forward and L + 2 in reverse of ~0.5 us each.
 #pragma once
 #include <type_traits>
 

@@ -160,7 +160,7 @@ __global__ void na_advance(cls_noalloc_advance a, float drag_s, float* __restric
 // substep.  The springs' impulses are evaluated spring-parallel into a table and
 // summed per vertex in spring order (a row list built at the start), without
 // atomics.  Bound by the latency of its three barriers per substep and of the
-// impulse's arithmetic: 64 quadrupeds (93 vertices, 608 springs) 10.3 -> 2.2 us per
+// impulse's arithmetic: 64 quadrupeds (93 vertices, 608 springs) 10.3 -> 1.9 us per
 // substep (two launches and six global atomics per spring before).
 struct FusedShared {
   cls::V4<float>* x;
