@@ -38,7 +38,7 @@ def _batch(robots, envs, precision, steps=13, path="per_env"):
 
 
 @pytest.mark.parametrize("precision", [32, 64])
-@pytest.mark.parametrize("threads", [64, 256])
+@pytest.mark.parametrize("threads", [64, 256, 512, 1024])
 @pytest.mark.parametrize("n_v, hubs, rest, parallel", [
     (60, (48,), 60, 1),                        # the longest list of one thread
     (60, (49, 48, 50), 60, 1),
@@ -117,3 +117,25 @@ def test_one_robot_keeps_its_tables():
         b.set_spring_tables(0)
         assert b.clusters[0] > 1         # both forms evaluate the hub's springs by a half-warp
         b.close()
+
+
+def test_policy_steps():
+    """Steps with outputs from outside: the same observations with tables and without."""
+    from cls_b200._capi import ptr
+    out = []
+    for mode in (-1, 0):
+        b = _batch([_robot(120, (92, 60), 300), _robot(20, (), 40)], [0, 1], 32)
+        try:
+            b.set_spring_tables(mode)
+            rng = np.random.default_rng(3)
+            obs, aux, act = np.zeros(4096), np.zeros(8), rng.uniform(-1, 1, 4096)
+            seen = []
+            for t in range(6):
+                b._c(b.lib.cls_env_step(b.h, t, ptr(act) if t else None, ptr(obs), ptr(aux)))
+                seen += [obs.copy(), aux.copy()]
+            out.append(seen)
+        finally:
+            b.close()
+    assert not np.array_equal(out[0][0], out[0][-2])
+    for u, w in zip(*out):
+        assert np.isfinite(u).all() and np.array_equal(u, w)
