@@ -15,8 +15,11 @@ namespace {
 // Each kernel of the chain releases its dependent at once and waits, before it
 // reads what an earlier launch wrote, until all of them have finished; the tables
 // read ahead of that wait are laid out when the batch is prepared.  4096 spiders, a
-// training step of 80 substeps: 35.5 -> 33.8 ms; 300: 14.6 -> 14.3.
-template <typename... P, typename... A>
+// training step of 80 substeps: 35.5 -> 33.8 ms; 300: 14.6 -> 14.3.  Not in FP64, where
+// CTAs are larger and those that wait take the running launches' room (21 substeps and
+// their adjoint of 100 / 256 / 400 / 1000 spiders with and without: 7.2 / 7.8 / 8.9 / 13.8 and
+// 7.5 / 7.9 / 9.0 / 12.1 ms, of 150-vertex robots 3.7 / 4.7 / 5.1 / 6.2 and 3.9 / 4.1 / 4.2 / 5.8).
+template <typename R, typename... P, typename... A>
 cudaError_t chain(void (*fn)(P...), int grid, int threads, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchConfig_t c{};
   cudaLaunchAttribute at{};
@@ -27,7 +30,7 @@ cudaError_t chain(void (*fn)(P...), int grid, int threads, size_t smem, cudaStre
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   c.attrs = &at;
-  c.numAttrs = 1;
+  c.numAttrs = std::is_same<R, float>::value ? 1 : 0;
   return cudaLaunchKernelEx(&c, fn, P(args)...);
 }
 }  // namespace
@@ -78,7 +81,7 @@ cudaError_t DenseLaunch<R>::step_fwd(const MsArgs<R>& a, bool hubs, int grid, in
                               int t_first, int t_end, int mode, int src_slot, int k_prev, int k_cur) {
   auto fn = !a.imp_cap ? ms_step_fwd_kernel<R, kStepThreads, TAB_NONE>
                        : (hubs ? HubKernels<R>::step_fwd() : ms_step_fwd_kernel<R, kStepThreads, TAB_ROWS>);
-  return chain(fn, grid, threads, smem, s, a, t, t_first, t_end, mode, src_slot, k_prev, k_cur);
+  return chain<R>(fn, grid, threads, smem, s, a, t, t_first, t_end, mode, src_slot, k_prev, k_cur);
 }
 
 template <typename R>
@@ -86,7 +89,7 @@ cudaError_t DenseLaunch<R>::step_rev(const MsArgs<R>& a, bool hubs, int grid, in
                               int t_pre, int t_begin, int t_end, int last_seg) {
   auto fn = !a.adj_cap ? ms_step_rev_kernel<R, kStepThreads, TAB_NONE>
                        : (hubs ? HubKernels<R>::step_rev() : ms_step_rev_kernel<R, kStepThreads, TAB_ROWS>);
-  return chain(fn, grid, threads, smem, s, a, t_post, t_pre, t_begin, t_end, last_seg);
+  return chain<R>(fn, grid, threads, smem, s, a, t_post, t_pre, t_begin, t_end, last_seg);
 }
 
 template <typename R>
@@ -94,12 +97,12 @@ cudaError_t DenseLaunch<R>::gemm(const MsArgs<R>& a, bool adjoint, int n_jobs, i
                                  const TcJob* tc, int kslot, cudaStream_t s) {
   if constexpr (std::is_same<R, float>::value) {
     if (job_cols == kDenseTNSmall)
-      return chain(adjoint ? ms_ctrl_gemm_tc_kernel<1, kDenseTNSmall> : ms_ctrl_gemm_tc_kernel<0, kDenseTNSmall>, n_jobs,
+      return chain<R>(adjoint ? ms_ctrl_gemm_tc_kernel<1, kDenseTNSmall> : ms_ctrl_gemm_tc_kernel<0, kDenseTNSmall>, n_jobs,
                    umma::kBulkThreads, umma::BulkShape<kDenseTNSmall, kBulkStages>::kSmemBytes, s, a, tc, kslot);
-    return chain(adjoint ? ms_ctrl_gemm_tc_kernel<1, kDenseTN> : ms_ctrl_gemm_tc_kernel<0, kDenseTN>, n_jobs,
+    return chain<R>(adjoint ? ms_ctrl_gemm_tc_kernel<1, kDenseTN> : ms_ctrl_gemm_tc_kernel<0, kDenseTN>, n_jobs,
                  umma::kBulkThreads, umma::BulkShape<kDenseTN, kBulkStages>::kSmemBytes, s, a, tc, kslot);
   } else {
-    return chain(adjoint ? ms_ctrl_gemm_simt_kernel<R, 1> : ms_ctrl_gemm_simt_kernel<R, 0>, n_jobs, 256, 0, s, a, jobs,
+    return chain<R>(adjoint ? ms_ctrl_gemm_simt_kernel<R, 1> : ms_ctrl_gemm_simt_kernel<R, 0>, n_jobs, 256, 0, s, a, jobs,
                  kslot);
   }
 }

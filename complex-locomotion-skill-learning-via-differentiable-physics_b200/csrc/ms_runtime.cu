@@ -767,8 +767,7 @@ class SimImpl final : public SimBase {
   size_t adj_entries(int threads) const { return 8 * nmax_ > threads ? imp_cap_ : 0; }
   // Shared memory of the batched step kernels: tables as the fused kernels have them,
   // where they fit beside the rest (a caller's small blocks leave the fused kernels
-  // more room), and in FP64 only on demand (300 FP64 robots of 44 vertices: forward +
-  // reverse 3.8 ms with tables, 2.7 without).
+  // more room).
   void size_dense() {
     int dev = 0, optin = 0;
     CLS_CUDA(cudaGetDevice(&dev));
@@ -781,9 +780,7 @@ class SimImpl final : public SimBase {
       drev_smem_ = rev_smem_bytes<R>(nmax_, smem_amax_, smem_omax_, smem_omax_, dense_threads_, entries);
       return dfwd_smem_ + fwd_static <= (size_t)optin && drev_smem_ + rev_static <= (size_t)optin;
     };
-    const bool wanted = std::is_same<R, float>::value || tables_forced_;
-    CLS_REQUIRE((wanted && fits(imp_cap_)) || fits(0),
-                "robot too large for the batched controller's step kernels");
+    CLS_REQUIRE(fits(imp_cap_) || fits(0), "robot too large for the batched controller's step kernels");
   }
 
   // Launch shape of the fused kernels: threads per CTA select the kernel
@@ -1100,13 +1097,10 @@ class SimImpl final : public SimBase {
       use_shape(threads_, wsh_on_ ? 1 : 0);
       if (d_wt_.p) size_dense();
     };
-    const bool keep_forced = tables_forced_;
     try {
-      tables_forced_ = mode == 1;
       apply(mode == 0 ? 0 : fit);
     } catch (...) {
       try {
-        tables_forced_ = keep_forced;
         apply(keep);
       } catch (...) {
       }
@@ -1464,8 +1458,7 @@ class SimImpl final : public SimBase {
   void enable_dense() {
     constexpr bool f32 = std::is_same<R, float>::value;
     // step kernels: one CTA per env, a thread per vertex up to kStepThreads (FP64:
-    // 128, its 180 registers leave no second CTA of 256); per
-    // CTA the fused kernels' shared-memory carve with the controller buffers
+    // 128); per CTA the fused kernels' shared-memory carve with the controller buffers
     // sized for the output layer only (step_args)
     dense_threads_ = std::min(f32 ? kStepThreads : 128, std::max(128, (nmax_ + 31) / 32 * 32));
     size_dense();
@@ -2634,7 +2627,6 @@ class SimImpl final : public SimBase {
   int smax_ = 0;
   static constexpr size_t kImpSmemMax = 48 * 1024 + 32;  // 3072 springs in FP32 and the zero entry
   int table_max_ = 1;  // entries of the largest robot's table
-  bool tables_forced_ = false;  // set_spring_tables(1)
   size_t dense_entries_ = 0;    // of the batched step kernels' tables
   bool hubs_ = false;  // a robot has vertices of more than kEllRows springs
   DevBuf<unsigned short> d_inc_ell_;

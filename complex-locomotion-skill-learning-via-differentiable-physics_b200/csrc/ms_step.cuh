@@ -15,6 +15,9 @@ __host__ __device__ __forceinline__ int pad4(int x) { return (x + 3) & ~3; }
 // / reverse step kernels: 128 threads 15.3 / 19.5 ms, 128 x 8 CTAs 11.1 / 15.9, 256 x
 // 3 12.6 / 14.8, 256 x 4 10.8 / 12.8; 300 spiders differ by 10 %.
 constexpr int kStepCtas = 4;
+// FP64: 128 registers, four CTAs of the 128 threads it runs with (181 registers without
+// the bound: 400 robots of 150 vertices, 21 substeps and their adjoint, 4.9 -> 4.2 ms).
+constexpr int kStepCtas64 = 2;
 // One CTA per env; the substep halves with the env's state in the CTA's
 // shared memory (the fused kernels' carve with the controller buffers sized
 // for the output layer only).  One warp per env
@@ -30,7 +33,7 @@ constexpr int kStepCtas = 4;
 // The state comes from checkpoint slot src_slot at t == t_first, else from
 // live_x/v.
 template <typename R, int MAXT, int TAB>
-__global__ void __launch_bounds__(MAXT, sizeof(R) == 4 ? kStepCtas : 1)
+__global__ void __launch_bounds__(MAXT, sizeof(R) == 4 ? kStepCtas : kStepCtas64)
 ms_step_fwd_kernel(MsArgs<R> a, int t, int t_first, int t_end, int mode, int src_slot, int k_prev,
                    int k_cur) {
   extern __shared__ __align__(256) char smem_raw[];
@@ -95,7 +98,7 @@ ms_step_fwd_kernel(MsArgs<R> a, int t, int t_first, int t_end, int mode, int src
 // launch of the segment (t_pre = t_end - 1) seeds it (last segment) or takes
 // the carry of the later segment.
 template <typename R, int MAXT, int TAB>
-__global__ void __launch_bounds__(MAXT, sizeof(R) == 4 ? kStepCtas : 1)
+__global__ void __launch_bounds__(MAXT, sizeof(R) == 4 ? kStepCtas : kStepCtas64)
 ms_step_rev_kernel(MsArgs<R> a, int t_post, int t_pre, int t_begin, int t_end, int last_seg) {
   extern __shared__ __align__(256) char smem_raw[];
   __shared__ RobotDesc rb;

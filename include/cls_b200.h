@@ -308,8 +308,8 @@ int cls_get_launch_shape(const cls_sim* sim, int32_t* threads_per_block, int32_t
 int cls_set_clusters(cls_sim* sim, int32_t size, int32_t heavy);
 int cls_get_clusters(const cls_sim* sim, int32_t* size, int32_t* heavy);
 
-/* Per-spring tables of the fused single-CTA kernels and the batched step kernels
- * (in FP64 there only with mode 1): each spring's impulse (forward) and adjoint terms (reverse)
+/* Per-spring tables of the fused single-CTA kernels and the batched step kernels:
+ * each spring's impulse (forward) and adjoint terms (reverse)
  * evaluated once into shared memory and summed by a thread per vertex (a vertex of
  * more than 48 springs: by a half-warp), instead of evaluated from both of its
  * endpoints.  mode -1 (the default at creation): on when the largest robot's table

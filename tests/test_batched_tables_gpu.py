@@ -1,5 +1,5 @@
-"""Spring tables of the batched controller's step kernels: reported as they are, on
-demand in FP64, and never the reason that a robot is refused."""
+"""Spring tables of the batched controller's step kernels: reported as they are, and
+never the reason that a robot is refused."""
 import numpy as np
 import pytest
 
@@ -19,19 +19,18 @@ def _batch(robot, envs, precision, threads=0, steps=9):
 
 @pytest.mark.parametrize("precision", [32, 64])
 def test_report_and_choice(precision):
-    """Automatic: FP32 with tables, FP64 without; mode 1 has them in both, with the bits
-    of the direct gathers."""
+    """On by default, with the bits of the direct gathers."""
     from cls_b200 import robot_design
     from cls_b200.batch import Robot
     b = _batch(Robot.actuated_outputs(*robot_design.quadruped_lattice(), hidden=[16]), 5, precision)
     try:
         assert b.spring_tables
         b.set_controller_path("batched")
-        assert b.spring_tables == (precision == 32)
+        assert b.spring_tables
         out = []
         for mode in (-1, 0, 1):
             b.set_spring_tables(mode)
-            assert b.spring_tables == {-1: precision == 32, 0: False, 1: True}[mode]
+            assert b.spring_tables == (mode != 0)
             b.simulate(9)
             out.append([*b.final_state(), *b.state_grads()])
         for other in out[1:]:
@@ -70,3 +69,30 @@ def test_largest_robot_of_small_blocks():
         assert all(np.isfinite(a).all() for a in (*b.final_state(), *b.state_grads()))
     finally:
         b.close()
+
+
+def test_fp64_robots_beyond_two_per_sm():
+    """400 FP64 robots take 1.03 times as long as 256: four step CTAs fit an SM (1.35 when
+    two did and launches that waited took their room)."""
+    import torch
+    from cls_b200 import robot_design
+    from cls_b200.batch import Robot
+    robot = Robot.actuated_outputs(*robot_design.random_lattice(np.random.default_rng(150), 150), hidden=[64])
+    times = []
+    for envs in (256, 400):
+        b = _batch(robot, envs, 64, steps=22)
+        try:
+            b.set_controller_path("batched")
+            b.set_stream(torch.cuda.current_stream().cuda_stream)
+            t = []
+            for _ in range(9):
+                ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+                ev[0].record()
+                b.simulate(21)
+                ev[1].record()
+                torch.cuda.synchronize()
+                t.append(ev[0].elapsed_time(ev[1]))
+            times.append(np.median(t[2:]))
+        finally:
+            b.close()
+    assert times[1] < 1.2 * times[0]
