@@ -17,7 +17,7 @@
 //     n_envs * n_vertices * 3 <= kScratchFloats and are rejected otherwise;
 //   * every GPU that loads the library holds that 8 MiB until the process ends;
 //   * robots whose springs fit in one CTA's shared memory (about 5000) need no
-//     scratch: one launch runs all substeps (na_fused).  Larger ones use the
+//     scratch: one launch runs all substeps (na_fused, na_slices).  Larger ones use the
 //     array, and calls that overlap on the GPU race with each other there and
 //     give wrong results; serialise them;
 //   * each call clears the part it uses before the first substep, so nothing
@@ -207,6 +207,53 @@ __device__ __forceinline__ void na_hubs(const FusedShared& s, int N, Work work) 
   }
 }
 
+// The thread's springs tid, tid + blockDim, ..: their ends, all loads in flight at once
+// (-1, -1 beyond the last and where an end is outside the robot).
+constexpr int kSpringMax = kFillMax / 2;   // per thread
+__device__ __forceinline__ void na_ends(const cls_noalloc_advance& a, int2 (&ab)[kSpringMax]) {
+  const int S = a.n_springs, N = a.n_vertices;
+#pragma unroll
+  for (int k = 0; k < kSpringMax; ++k) {
+    const int q = threadIdx.x + k * blockDim.x;
+    ab[k] = q < S ? make_int2(a.spring_a[q], a.spring_b[q]) : make_int2(-1, -1);
+  }
+#pragma unroll
+  for (int k = 0; k < kSpringMax; ++k)
+    if (ab[k].x < 0 || ab[k].x >= N || ab[k].y < 0 || ab[k].y >= N) ab[k] = make_int2(-1, -1);
+}
+
+// counts ptr[1 .. n] to row starts ptr[0 .. n] (ptr[0] = 0), by all threads; part: n / 32 + 1
+// ints.  Ends with a barrier.
+__device__ __forceinline__ void na_row_starts(int* ptr, int n, int* part) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  auto scan = [&](int c) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, c, o);
+      if (lane >= o) c += up;
+    }
+    return c;
+  };
+  __syncthreads();
+  for (int g = wid; 32 * g <= n; g += nw) {
+    const int i = 32 * g + lane, c = scan(i <= n ? ptr[i] : 0);
+    if (i <= n) ptr[i] = c;
+    if (lane == 31) part[g] = c;
+  }
+  __syncthreads();
+  if (wid == 0) {
+    int carry = 0;
+    for (int g0 = 0; 32 * g0 <= n; g0 += 32) {
+      const int g = g0 + lane, c = carry + scan(32 * g <= n ? part[g] : 0);
+      if (32 * g <= n) part[g] = c;
+      carry = __shfl_sync(0xffffffffu, c, 31);
+    }
+  }
+  __syncthreads();
+  for (int i = 32 + threadIdx.x; i <= n; i += blockDim.x) ptr[i] += part[(i >> 5) - 1];
+  __syncthreads();
+}
+
 __global__ void __launch_bounds__(1024) na_fused(cls_noalloc_advance a, float drag_s) {
   extern __shared__ __align__(16) char na_smem[];
   FusedShared s;
@@ -222,48 +269,39 @@ __global__ void __launch_bounds__(1024) na_fused(cls_noalloc_advance a, float dr
     s.v[i] = v;
   }
   for (int i = tid; i <= N; i += nt) s.ptr[i] = 0;
+  int2 ab[kSpringMax];
+  na_ends(a, ab);
   __syncthreads();
-  for (int q = tid; q < S; q += nt) {
-    const int ia = a.spring_a[q], ib = a.spring_b[q];
-    const bool ok = ia >= 0 && ia < N && ib >= 0 && ib < N;
-    s.ab[q] = ok ? make_ushort2((unsigned short)ia, (unsigned short)ib) : make_ushort2(kNone, kNone);
-    s.par[q] = make_float4(a.rest_length[q], a.stiffness[q], a.actuation_coef[q], a.actuation[(size_t)blockIdx.x * S + q]);
-    if (ok) {
-      atomicAdd(s.ptr + ia + 1, 1);
-      atomicAdd(s.ptr + ib + 1, 1);
-    }
-  }
-  __syncthreads();
-  // row starts: inclusive scan of the counts by the first warp
-  if (tid < 32) {
-    int carry = 0;
-    for (int i0 = 0; i0 <= N; i0 += 32) {
-      int c = i0 + tid <= N ? s.ptr[i0 + tid] : 0;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int up = __shfl_up_sync(0xffffffffu, c, o);
-        if (tid >= o) c += up;
-      }
-      c += carry;
-      if (i0 + tid <= N) s.ptr[i0 + tid] = c;
-      carry = __shfl_sync(0xffffffffu, c, 31);
-    }
+  for (int k = 0; k < kSpringMax; ++k) {
+    const int q = tid + k * nt;
+    if (q < S) s.ab[q] = make_ushort2((unsigned short)ab[k].x, (unsigned short)ab[k].y);  // -1: kNone
+    if (ab[k].x < 0) continue;
+    atomicAdd(s.ptr + ab[k].x + 1, 1);
+    atomicAdd(s.ptr + ab[k].y + 1, 1);
   }
-  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kSpringMax; ++k) {
+    const int q = tid + k * nt;
+    if (q < S)
+      s.par[q] = make_float4(a.rest_length[q], a.stiffness[q], a.actuation_coef[q], a.actuation[(size_t)blockIdx.x * S + q]);
+  }
+  int* fill = reinterpret_cast<int*>(s.v);   // the velocities come back below
+  na_row_starts(s.ptr, N, fill);
   // rows in any order, then sorted; the long rows of hub vertices are written in
   // order by a warp each (na_hubs)
   bool long_row = false;
   for (int i = tid; i < N; i += nt) long_row |= s.ptr[i + 1] - s.ptr[i] > kThreadRow;
   const bool hubs = __syncthreads_or(long_row);
-  int* fill = reinterpret_cast<int*>(s.v);   // the velocities come back below
   for (int i = tid; i < N; i += nt) fill[i] = s.ptr[i];
   __syncthreads();
   auto by_thread = [&](int i) { return !hubs || s.ptr[i + 1] - s.ptr[i] <= kThreadRow; };
-  for (int q = tid; q < S; q += nt) {
-    const ushort2 ab = s.ab[q];
-    if (ab.x == kNone) continue;
-    if (by_thread(ab.x)) s.inc[atomicAdd(fill + ab.x, 1)] = (unsigned short)(2 * q);
-    if (by_thread(ab.y)) s.inc[atomicAdd(fill + ab.y, 1)] = (unsigned short)(2 * q + 1);
+#pragma unroll
+  for (int k = 0; k < kSpringMax; ++k) {
+    if (ab[k].x < 0) continue;
+    const int q = tid + k * nt;
+    if (by_thread(ab[k].x)) s.inc[atomicAdd(fill + ab[k].x, 1)] = (unsigned short)(2 * q);
+    if (by_thread(ab[k].y)) s.inc[atomicAdd(fill + ab[k].y, 1)] = (unsigned short)(2 * q + 1);
   }
   const int lane = tid & 31;
   const unsigned below = (1u << lane) - 1u;
@@ -382,18 +420,225 @@ __global__ void __launch_bounds__(1024) na_fused(cls_noalloc_advance a, float dr
   }
 }
 
-// largest dynamic shared memory of na_fused on the current device (0: unknown)
-size_t fused_capacity() {
+// The same with a cluster of C CTAs per env, for calls of few envs: each CTA holds the
+// positions and velocities of the whole env, and the lists, impulses and sums of its own
+// vertices -- an incidence's impulse is evaluated for its own vertex, a thread per
+// incidence, and summed in na_fused's order.  Every substep ends with the new state
+// stored into all CTAs of the cluster.  What one CTA of na_fused takes one after another
+// for thousands of springs (900 vertices, 4600 springs: 23 us for a call of one substep, 244
+// of 32) is C times less here (13.4 and 128 with C = 8).  Bound by the latency of a call's
+// dozen short phases.
+constexpr int kSliceHeld = 2;      // incidences of a thread whose springs stay in registers
+
+struct SliceShared {
+  cls::V4<float>* x;
+  cls::V4<float>* v;
+  cls::V4<float>* imp;     // per own incidence, the first slice_table(..) of them
+  cls::V4<float>* sum;     // per own vertex
+  unsigned short* inc;     // per own vertex in spring order: 2 spring + side (room for all)
+  int* ptr;                // row starts of the own vertices, + 1
+  int* fill;
+};
+// Twice the balanced share: with room for every incidence, which one CTA could own,
+// little L1 is left (4600 springs, one substep, C = 8: 16.7 us).  Those beyond the table
+// are evaluated as their row is summed.
+__host__ __device__ inline int slice_table(int ns, int C) { return 4 * ns / C + 32; }
+
+__host__ __device__ inline size_t carve_slices(char* base, int nv, int ns, int C, SliceShared* s) {
+  size_t off = 0;
+  auto take = [&](size_t bytes) { char* p = base + off; off += (bytes + 15) & ~size_t(15); return p; };
+  SliceShared z;
+  z.x = (cls::V4<float>*)take(sizeof(cls::V4<float>) * nv);
+  z.v = (cls::V4<float>*)take(sizeof(cls::V4<float>) * nv);
+  z.imp = (cls::V4<float>*)take(sizeof(cls::V4<float>) * slice_table(ns, C));
+  z.sum = (cls::V4<float>*)take(sizeof(cls::V4<float>) * (nv / C + 1));
+  z.inc = (unsigned short*)take(sizeof(unsigned short) * 2 * ns);
+  z.ptr = (int*)take(sizeof(int) * (nv + 1));
+  z.fill = (int*)take(sizeof(int) * nv);
+  if (s) *s = z;
+  return off;
+}
+
+__global__ void __launch_bounds__(1024) na_slices(cls_noalloc_advance a, float drag_s) {
+  extern __shared__ __align__(16) char na_smem[];
+  const int C = (int)cls::cl::size();
+  SliceShared s;
+  carve_slices(na_smem, a.n_vertices, a.n_springs, C, &s);
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, N = a.n_vertices, S = a.n_springs;
+  const int cap = slice_table(S, C), rank = (int)cls::cl::rank(), env = (int)blockIdx.x / C;
+  const int v0 = (int)((long long)N * rank / C), M = (int)((long long)N * (rank + 1) / C) - v0;
+  float* xe = a.x + (size_t)env * N * 3;
+  float* ve = a.v + (size_t)env * N * 3;
+  const float* act = a.actuation + (size_t)env * S;
+  for (int i = tid; i < N; i += nt) {
+    cls::V4<float> x, v;
+    x.x = xe[3 * i]; x.y = xe[3 * i + 1]; x.z = xe[3 * i + 2]; x.w = 0;
+    v.x = ve[3 * i]; v.y = ve[3 * i + 1]; v.z = ve[3 * i + 2]; v.w = 0;
+    s.x[i] = x;
+    s.v[i] = v;
+  }
+  for (int i = tid; i <= M; i += nt) s.ptr[i] = 0;
+  int2 ab[kSpringMax];
+  na_ends(a, ab);
+  // own(f): f(own vertex, 2 spring + side) for the own ends of the thread's springs
+  auto own = [&](auto f) {
+#pragma unroll
+    for (int k = 0; k < kSpringMax; ++k) {
+      const int q = tid + k * nt;
+      if (ab[k].x < 0) continue;
+      if (ab[k].x >= v0 && ab[k].x < v0 + M) f(ab[k].x - v0, 2 * q);
+      if (ab[k].y >= v0 && ab[k].y < v0 + M) f(ab[k].y - v0, 2 * q + 1);
+    }
+  };
+  __syncthreads();
+  own([&](int i, int) { atomicAdd(s.ptr + i + 1, 1); });
+  na_row_starts(s.ptr, M, s.fill);
+  bool long_row = false;
+  for (int i = tid; i < M; i += nt) {
+    s.fill[i] = s.ptr[i];
+    long_row |= s.ptr[i + 1] - s.ptr[i] > kThreadRow;
+  }
+  const bool hubs = __syncthreads_or(long_row);
+  own([&](int i, int code) { s.inc[atomicAdd(s.fill + i, 1)] = (unsigned short)code; });
+  __syncthreads();
+  const int n_inc = s.ptr[M];
+  {  // a thread per incidence: its place in its row is the number of smaller ones
+    unsigned short code[kFillMax];
+    int to[kFillMax];
+#pragma unroll
+    for (int k = 0; k < kFillMax; ++k) {
+      const int at = tid + k * nt;
+      to[k] = -1;
+      if (at >= n_inc) continue;
+      code[k] = s.inc[at];
+      const int i = ((code[k] & 1) ? a.spring_b : a.spring_a)[code[k] >> 1] - v0;
+      int r = s.ptr[i];
+      for (int p = s.ptr[i], e = s.ptr[i + 1]; p < e; ++p) r += s.inc[p] < code[k];
+      to[k] = r;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kFillMax; ++k)
+      if (to[k] >= 0) s.inc[to[k]] = code[k];
+  }
+  cls::MsArgs<float> p;
+  p.dt = a.dt;
+  p.gravity = a.gravity;
+  p.ground = a.ground_height;
+  p.drag_s = drag_s;
+  p.friction = a.friction;
+  __syncthreads();
+  // the springs of the thread's incidences; the first ones stay in registers
+  struct Spring {
+    int a, b;
+    float4 c;
+  };
+  auto spring = [&](int k) {
+    const int q = s.inc[k] >> 1;
+    Spring g;
+    g.a = a.spring_a[q];
+    g.b = a.spring_b[q];
+    g.c = make_float4(a.rest_length[q], a.stiffness[q], a.actuation_coef[q], act[q]);
+    return g;
+  };
+  auto impulse = [&](const Spring& g) {
+    float imp[3];
+    cls::spring_impulse<float>(s.x[g.a], s.x[g.b], s.v[g.a], s.v[g.b], g.c.x, g.c.y, g.c.z, g.c.w, a.dt,
+                               a.dashpot_damping, imp);
+    cls::V4<float> r;
+    r.x = imp[0]; r.y = imp[1]; r.z = imp[2]; r.w = 0;
+    return r;
+  };
+  const int n_tab = n_inc < cap ? n_inc : cap;
+  Spring held[kSliceHeld];
+#pragma unroll
+  for (int k = 0; k < kSliceHeld; ++k)
+    if (tid + k * nt < n_tab) held[k] = spring(tid + k * nt);
+  for (int step = 0; step < a.n_substeps; ++step) {
+#pragma unroll
+    for (int k = 0; k < kSliceHeld; ++k)
+      if (tid + k * nt < n_tab) s.imp[tid + k * nt] = impulse(held[k]);
+    for (int k = tid + kSliceHeld * nt; k < n_tab; k += nt) s.imp[k] = impulse(spring(k));
+    __syncthreads();
+    auto add = [&](int k, cls::V4<float>& vi) {
+      const cls::V4<float> r = k < cap ? s.imp[k] : impulse(spring(k));
+      if (s.inc[k] & 1) { vi.x += r.x; vi.y += r.y; vi.z += r.z; }
+      else { vi.x -= r.x; vi.y -= r.y; vi.z -= r.z; }
+    };
+    for (int i = tid; i < M; i += nt) {
+      cls::V4<float> vi;
+      vi.x = vi.y = vi.z = vi.w = 0;
+      const int e = s.ptr[i + 1];
+      if (e - s.ptr[i] > kThreadRow) continue;
+#pragma unroll 4
+      for (int k = s.ptr[i]; k < e; ++k) add(k, vi);
+      s.sum[i] = vi;
+    }
+    if (hubs) {
+      FusedShared rows;
+      rows.ptr = s.ptr;
+      na_hubs(rows, M, [&](int h) {
+        cls::V4<float> vi;
+        vi.x = vi.y = vi.z = vi.w = 0;
+        for (int k = s.ptr[h] + lane; k < s.ptr[h + 1]; k += 32) add(k, vi);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          vi.x += __shfl_xor_sync(0xffffffffu, vi.x, o);
+          vi.y += __shfl_xor_sync(0xffffffffu, vi.y, o);
+          vi.z += __shfl_xor_sync(0xffffffffu, vi.z, o);
+        }
+        if (lane == 0) s.sum[h] = vi;
+      });
+    }
+    // all CTAs have read the state (before the first substep: the caller's arrays too)
+    cls::cl::sync();
+    for (int i = tid; i < M; i += nt) {
+      cls::V4<float> x = s.x[v0 + i], v = s.v[v0 + i];
+      cls::advance_vertex<float>(p, x, v, s.sum[i]);
+      if (step + 1 < a.n_substeps) {
+        for (int r = 0; r < C; ++r) {
+          *cls::cl::peer(s.x + v0 + i, r) = x;
+          *cls::cl::peer(s.v + v0 + i, r) = v;
+        }
+      } else {
+        const int g = 3 * (v0 + i);
+        xe[g] = x.x; xe[g + 1] = x.y; xe[g + 2] = x.z;
+        ve[g] = v.x; ve[g + 1] = v.y; ve[g + 2] = v.z;
+      }
+    }
+    if (step + 1 < a.n_substeps) cls::cl::sync();
+  }
+}
+
+// largest dynamic shared memory of na_fused on the current device (0: unknown) and
+// its SMs
+size_t fused_capacity(int* n_sm) {
   int dev = 0, optin = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return 0;
   return (size_t)optin;
 }
 
-int fused_threads(const cls_noalloc_advance& a) {
+// Threads of na_fused.  With more envs than SMs, 512 where two CTAs' shared memory fits
+// an SM, whose threads two of 1024 would fill (600 spiders, one / 32 substeps: 49 / 474 ->
+// 35 / 372 us).
+int fused_threads(const cls_noalloc_advance& a, int n_sm, size_t smem, size_t most) {
   const int work = a.n_springs > a.n_vertices ? a.n_springs : a.n_vertices;
-  return work <= 256 ? 256 : (work <= 1024 ? 512 : 1024);
+  const bool pairs = a.n_envs > n_sm && work <= kSpringMax * 512 && 2 * smem <= most;
+  return work <= 256 ? 256 : (work <= 1024 || pairs ? 512 : 1024);
+}
+
+// CTAs per env of na_slices, 1 for na_fused: clusters that can all run at once (8 up to
+// 12 envs, 4 up to 29 on 148 SMs), from where they are the faster form for calls of any
+// length (na_fused / na_slices, us, one env, 1 and 32 substeps: 1000 springs 10.5 / 10.5 and
+// 80 / 85, 1378 12.5 / 10.5 and 98 / 94, 3000 16.8 / 12.5 and 164 / 107, 4600 22.8 / 13.4 and
+// 242 / 128; 29 envs of 1378 12.5 / 11.3 and 99 / 99).
+constexpr int kSliceSprings = 1300, kSliceThreads = 1024;
+int slice_count(const cls_noalloc_advance& a, int n_sm) {
+  if (a.n_springs < kSliceSprings || 2 * a.n_springs > kFillMax * kSliceThreads) return 1;
+  return 12LL * a.n_envs <= n_sm ? 8 : (5LL * a.n_envs <= n_sm ? 4 : 1);
 }
 
 int grid_for(long long n) {
@@ -441,20 +686,41 @@ extern "C" int cls_ms_advance_noalloc(const cls_noalloc_advance* a, void* stream
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const float drag_s = (float)exp(-(double)a->dt * (double)a->drag_damping);
-  // one CTA per env when an env's springs fit in its shared memory (up to about
-  // 5000 springs); larger ones keep a launch per phase over the scratch array
+  // one CTA (or cluster) per env when an env's springs fit in a CTA's shared memory (up to
+  // about 5000 springs); larger ones keep a launch per phase over the scratch array
   const size_t smem = carve_fused(nullptr, a->n_vertices, a->n_springs, nullptr);
-  const size_t fused_max = fused_capacity();
-  if (a->n_substeps > 0 && a->n_vertices <= kFusedMax && 2 * a->n_springs <= kFillMax * fused_threads(*a) &&
+  int n_sm = 0;
+  const size_t fused_max = fused_capacity(&n_sm);
+  const int threads = fused_threads(*a, n_sm, smem, fused_max);
+  if (a->n_substeps > 0 && a->n_vertices <= kFusedMax && 2 * a->n_springs <= kFillMax * threads &&
       smem <= fused_max) {
     // the limit belongs to the kernel in the whole process: always the device's
     // maximum, so that a call with a smaller robot on another host thread never
     // lowers it between this call's raise and its launch
+    const int slices = slice_count(*a, n_sm);
+    const size_t bytes = carve_slices(nullptr, a->n_vertices, a->n_springs, slices, nullptr);
+    if (slices > 1 && bytes <= fused_max) {
+      cudaError_t e = cudaFuncSetAttribute(na_slices, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_max);
+      cudaLaunchConfig_t c{};
+      cudaLaunchAttribute at{};
+      c.gridDim = dim3((unsigned)(a->n_envs * slices));
+      c.blockDim = dim3(kSliceThreads);
+      c.dynamicSmemBytes = bytes;
+      c.stream = s;
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = (unsigned)slices;
+      at.val.clusterDim.y = at.val.clusterDim.z = 1;
+      c.attrs = &at;
+      c.numAttrs = 1;
+      if (e == cudaSuccess) e = cudaLaunchKernelEx(&c, na_slices, *a, drag_s);
+      if (e == cudaSuccess) return CLS_OK;
+      cudaGetLastError();  // a device that cannot hold such a cluster: one CTA
+    }
     cudaError_t e = smem > 48 * 1024
                         ? cudaFuncSetAttribute(na_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_max)
                         : cudaSuccess;
     if (e == cudaSuccess) {
-      na_fused<<<a->n_envs, fused_threads(*a), smem, s>>>(*a, drag_s);
+      na_fused<<<a->n_envs, threads, smem, s>>>(*a, drag_s);
       e = cudaGetLastError();
     }
     if (e != cudaSuccess) {
