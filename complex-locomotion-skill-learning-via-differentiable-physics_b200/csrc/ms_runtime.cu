@@ -576,7 +576,6 @@ class SimImpl final : public SimBase {
     // largest robot's table is small (the forward gathers then read them)
     smax_ = smax;
     imp_cap_ = table_fits() ? table_max_ : 0;
-    fwd_base_ = fwd_smem_bytes<R>(nmax_, dmax, p0max, imp_cap_);
     int dev = 0;
     CLS_CUDA(cudaGetDevice(&dev));
     CLS_CUDA(cudaDeviceGetAttribute(&n_sm_, cudaDevAttrMultiProcessorCount, dev));
@@ -753,18 +752,27 @@ class SimImpl final : public SimBase {
                            : (threads_ <= 512 ? ms_reverse_kernel<R, 512, TAB> : ms_reverse_kernel<R, 1024, TAB>);
   }
   FwdFn fwd_fn() const {
-    if (imp_cap_ && hubs_) return HubKernels<R>::forward(threads_);
-    return imp_cap_ ? fwd_of<TAB_ROWS>() : fwd_of<TAB_NONE>();
+    const bool table = fwd_entries(threads_) > 0;
+    if (table && hubs_) return HubKernels<R>::forward(threads_);
+    return table ? fwd_of<TAB_ROWS>() : fwd_of<TAB_NONE>();
   }
   RevFn rev_fn() const {
     const bool table = adj_entries(threads_) > 0;
     if (table && hubs_) return HubKernels<R>::reverse(threads_);
     return table ? rev_of<TAB_ROWS>() : rev_of<TAB_NONE>();
   }
-  // entries of the fused reverse kernel's adjoint table: none for robots so small
-  // that the direct gather's half-warps take their vertices in two rounds (160
-  // robots of 44 vertices, 512 threads: reverse 1.29 ms with the table, 1.22 without)
-  size_t adj_entries(int threads) const { return 8 * nmax_ > threads ? imp_cap_ : 0; }
+  // Entries of the fused kernels' tables: none for robots so small that the direct
+  // gather's half-warps take their vertices in two rounds, where a thread per vertex
+  // leaves most of the block idle (forward of 101 substeps of one robot of 30 / 44 / 60
+  // vertices with tables 0.70 / 0.83 / 0.85 ms, without 0.59 / 0.79 / 0.80; 160 robots of 44, 512
+  // threads: reverse 1.29 and 1.22).  The FP64 forward only up to 32 vertices (30 / 44 with
+  // 0.91 / 1.15, without 0.86 / 1.21).
+  bool few_vertices(int threads) const { return 8 * nmax_ <= threads; }
+  size_t fwd_entries(int threads) const {
+    const bool direct = few_vertices(threads) && !tables_forced_ && (std::is_same<R, float>::value || nmax_ <= 32);
+    return direct ? 0 : imp_cap_;
+  }
+  size_t adj_entries(int threads) const { return few_vertices(threads) ? 0 : imp_cap_; }
   // Shared memory of the batched step kernels: tables as the fused kernels have them,
   // where they fit beside the rest (a caller's small blocks leave the fused kernels
   // more room).
@@ -799,6 +807,7 @@ class SimImpl final : public SimBase {
     const int keep = threads_;
     threads_ = threads;
     try {
+      const size_t fwd0 = fwd_smem_bytes<R>(nmax_, smem_dmax_, smem_p0max_, fwd_entries(threads));
       const size_t rev0 = rev_smem_bytes<R>(nmax_, smem_amax_, smem_omax_, smem_dmax_, threads, adj_entries(threads));
       const size_t ctrl = ctrl_smem_bytes<R>(wspan_max_, bspan_max_);
       int dev = 0, optin = 0;
@@ -809,7 +818,7 @@ class SimImpl final : public SimBase {
       CLS_CUDA(cudaFuncGetAttributes(&ra, rev_fn()));
       const size_t fwd_cap = (size_t)optin - fa.sharedSizeBytes;
       const size_t rev_cap = (size_t)optin - ra.sharedSizeBytes;
-      CLS_REQUIRE(fwd_base_ <= fwd_cap && rev0 <= rev_cap,
+      CLS_REQUIRE(fwd0 <= fwd_cap && rev0 <= rev_cap,
                   "robot too large for one CTA's shared memory (" + std::to_string(rev0) +
                       " bytes needed, " + std::to_string(rev_cap) + " available)");
       CLS_CUDA(cudaFuncSetAttribute(fwd_fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_cap));
@@ -822,17 +831,17 @@ class SimImpl final : public SimBase {
         CLS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rev_fn(), threads, r));
         return std::min(nf, nb);
       };
-      const int r_off = resident(fwd_base_, rev0);
+      const int r_off = resident(fwd0, rev0);
       CLS_REQUIRE(r_off >= 1,
                   "no CTA of " + std::to_string(threads) + " threads can be resident on an SM");
-      const int r_on = resident(fwd_base_ + ctrl, rev0 + ctrl);
+      const int r_on = resident(fwd0 + ctrl, rev0 + ctrl);
       CLS_REQUIRE(wsh != 1 || r_on >= 1,
                   "the controller (" + std::to_string(ctrl) + " bytes) does not fit in shared memory "
                   "beside the kernels' own");
       const bool on = wsh == 1 || (wsh == -1 && r_on >= 1 && r_on >= r_off);
       std::vector<ClusterPlan> plans = plan_clusters(optin);
       check_forced(plans, force_size_);
-      fwd_smem_ = fwd_base_ + (on ? ctrl : 0);
+      fwd_smem_ = fwd0 + (on ? ctrl : 0);
       rev_smem_ = rev0 + (on ? ctrl : 0);
       resident_ = on ? r_on : r_off;
       wsh_on_ = on;
@@ -1093,14 +1102,16 @@ class SimImpl final : public SimBase {
     const size_t keep = imp_cap_;
     auto apply = [&](size_t cap) {
       imp_cap_ = cap;
-      fwd_base_ = fwd_smem_bytes<R>(nmax_, smem_dmax_, smem_p0max_, imp_cap_);
       use_shape(threads_, wsh_on_ ? 1 : 0);
       if (d_wt_.p) size_dense();
     };
+    const bool keep_forced = tables_forced_;
     try {
+      tables_forced_ = mode == 1;
       apply(mode == 0 ? 0 : fit);
     } catch (...) {
       try {
+        tables_forced_ = keep_forced;
         apply(keep);
       } catch (...) {
       }
@@ -1274,7 +1285,7 @@ class SimImpl final : public SimBase {
     a.inc_ell = reinterpret_cast<const uint4*>(d_inc_ell_.p);
     a.spr_ab = d_spr_ab_.p;
     a.spr_p = d_spr_p_.p;
-    a.imp_cap = (int)imp_cap_;
+    a.imp_cap = (int)fwd_entries(threads_);
     a.adj_cap = (int)adj_entries(threads_);
     a.w = d_w_.p;
     a.bias = d_bias_.p;
@@ -2576,7 +2587,6 @@ class SimImpl final : public SimBase {
   // kernels keep it in shared memory; forward shared memory without it
   long long wspan_max_ = 0, bspan_max_ = 0;
   bool wsh_on_ = false;
-  size_t fwd_base_ = 0;
   size_t fwd_smem_ = 0, rev_smem_ = 0, n_queue_ = 0;
   HostMapped mapped_;
   std::vector<double> cost_;       // per env: cost of a substep (processing order, cluster sizes)
@@ -2627,6 +2637,7 @@ class SimImpl final : public SimBase {
   int smax_ = 0;
   static constexpr size_t kImpSmemMax = 48 * 1024 + 32;  // 3072 springs in FP32 and the zero entry
   int table_max_ = 1;  // entries of the largest robot's table
+  bool tables_forced_ = false;  // set_spring_tables(1)
   size_t dense_entries_ = 0;    // of the batched step kernels' tables
   bool hubs_ = false;  // a robot has vertices of more than kEllRows springs
   DevBuf<unsigned short> d_inc_ell_;

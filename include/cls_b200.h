@@ -315,8 +315,10 @@ int cls_get_clusters(const cls_sim* sim, int32_t* size, int32_t* heavy);
  * endpoints.  mode -1 (the default at creation): on when the largest robot's table
  * fits (<= 3072 springs in FP32); 0 off; 1 on (CLS_ERR_INVALID when it does not
  * fit).  The same results (each spring is evaluated in the same argument order
- * either way and gathered in the same order).  cls_spring_tables: whether the kernels
- * of the controller path in use have them.  No reference counterpart. */
+ * either way and gathered in the same order).  cls_spring_tables: whether the controller
+ * path in use has tables; with mode -1 fused kernels whose robots have no more than an
+ * eighth as many vertices as a block has threads gather directly all the same, which
+ * is faster there.  No reference counterpart. */
 int cls_set_spring_tables(cls_sim* sim, int32_t mode);
 int cls_spring_tables(const cls_sim* sim, int32_t* on);
 
